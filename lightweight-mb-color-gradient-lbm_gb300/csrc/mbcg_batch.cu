@@ -1,61 +1,11 @@
-// mbcg_batch.cu -- persistent batch step: one launch advances every live lattice of the server
-// by one time step.
-//
-// The work is a flat queue of tiles (BatchTile) over all live lattices, sorted by the host
-// (largest tiles first, grouped by body).  Each CTA of a grid of at most one CTA per SM takes
-// the next tile with an atomic counter and runs the same step_tile() as the plain kernel,
-// instantiated for the lattice's (Q, storage, feature set), on that lattice's step parameters in
-// a constant-memory table indexed by slot.  The stage mbarriers are initialised once per CTA; their phase
-// carries from tile to tile.
+// mbcg_batch.cu -- the batch step's dispatch (kernels in mbcg_batch_q{19,27}.cu) and the state hash.
+#include <algorithm>
+
 #include "mbcg_batch.h"
-#include "mbcg_step.cuh"
 
 namespace mbcg {
 
 namespace {
-
-__constant__ StepParams c_batch_params[kBatchParamSlots * 2]; // [slot][parity]
-
-template <int W>
-__global__ void __launch_bounds__(32 * W, 1)
-    batch_kernel(const BatchCase* __restrict__ cases, const BatchTile* __restrict__ tiles, int ntiles,
-                 const ChunkState* __restrict__ chunk, int* __restrict__ counters, int j) {
-    __shared__ int s_tile;
-    unsigned char* smem = aligned_smem_base();
-    init_stage_barriers(smem);
-    uint32_t phase = 0;
-    const int tid = threadIdx.y * 32 + threadIdx.x;
-    for (;;) {
-        __syncthreads(); // everyone is done with the previous tile's s_tile
-        if (tid == 0) s_tile = atomicAdd(&counters[j], 1);
-        __syncthreads();
-        const int t = s_tile;
-        if (t >= ntiles) return;
-        const BatchTile bt = tiles[t];
-        const ChunkState cs = chunk[bt.slot];
-        if (j >= cs.nsteps) continue;
-        const int par = cs.parity0 ^ (j & 1);
-        const BatchCase& C = cases[bt.slot];
-        const StepParams& sP = c_batch_params[bt.slot * 2 + par]; // this lattice, this parity
-        const CUtensorMap* maps = C.maps[par];
-        const long long step = cs.step0 + j + 1;
-        bool ok = true;
-        switch (C.kind) {
-        case BK_Q19_F32: ok = step_tile<19, float, W, true, F_ALL, false>(sP, maps, bt.bx, bt.by, bt.bz, step, smem, phase); break;
-        case BK_Q19_F16: ok = step_tile<19, __half, W, true, F_ALL, false>(sP, maps, bt.bx, bt.by, bt.bz, step, smem, phase); break;
-        case BK_Q19_BF16: ok = step_tile<19, __nv_bfloat16, W, true, F_ALL, false>(sP, maps, bt.bx, bt.by, bt.bz, step, smem, phase); break;
-        case BK_Q27_F32: ok = step_tile<27, float, W, true, F_ALL, false>(sP, maps, bt.bx, bt.by, bt.bz, step, smem, phase); break;
-        case BK_Q27_F16: ok = step_tile<27, __half, W, true, F_ALL, false>(sP, maps, bt.bx, bt.by, bt.bz, step, smem, phase); break;
-        case BK_Q27_BF16: ok = step_tile<27, __nv_bfloat16, W, true, F_ALL, false>(sP, maps, bt.bx, bt.by, bt.bz, step, smem, phase); break;
-        case BK_Q19_F32_P: ok = step_tile<19, float, W, true, 0>(sP, maps, bt.bx, bt.by, bt.bz, step, smem, phase); break;
-        case BK_Q19_F16_P: ok = step_tile<19, __half, W, true, 0>(sP, maps, bt.bx, bt.by, bt.bz, step, smem, phase); break;
-        case BK_Q27_F32_P: ok = step_tile<27, float, W, true, 0>(sP, maps, bt.bx, bt.by, bt.bz, step, smem, phase); break;
-        case BK_Q27_F16_P: ok = step_tile<27, __half, W, true, 0>(sP, maps, bt.bx, bt.by, bt.bz, step, smem, phase); break;
-        default: ok = false; break;
-        }
-        if (!ok) return; // step_tile has set the lattice's status word
-    }
-}
 
 // order-independent: sum over nodes of mix64(field, index, bits), wrapping
 template <typename S>
@@ -81,21 +31,17 @@ __global__ void state_hash_kernel(const StepParams P, unsigned long long* out) {
 
 } // namespace
 
-int batch_smem_bytes() { return Geo<float, kBatchW>::smem; }
-
 cudaError_t upload_batch_params(const StepParams* params, int n, cudaStream_t s) {
     if (n < 0 || n > kBatchParamSlots) return cudaErrorInvalidValue;
-    return cudaMemcpyToSymbolAsync(c_batch_params, params, sizeof(StepParams) * 2 * n, 0, cudaMemcpyHostToDevice, s);
+    if (cudaError_t e = upload_batch_params_q19(params, n, s)) return e;
+    return upload_batch_params_q27(params, n, s);
 }
 
-cudaError_t launch_batch(const BatchCase* cases, const BatchTile* tiles, int ntiles, const ChunkState* chunk,
-                         int* counters, int j, int grid, cudaStream_t s) {
-    auto kern = batch_kernel<kBatchW>;
-    static std::atomic<unsigned long long> configured{0};
-    if (cudaError_t e = configure_once(kern, batch_smem_bytes(), configured)) return e;
-    if (grid < 1 || ntiles < 1) return cudaSuccess;
-    kern<<<grid, dim3(32, kBatchW, 1), batch_smem_bytes(), s>>>(cases, tiles, ntiles, chunk, counters, j);
-    return cudaGetLastError();
+cudaError_t launch_batch(int kind, const BatchCase* cases, const BatchTile* tiles, int ntiles, const ChunkState* chunk,
+                         int* counter, int j, int grid, cudaStream_t s) {
+    if (kind < 0 || kind >= BK_COUNT) return cudaErrorInvalidValue;
+    return batch_q(kind) == 27 ? launch_batch_q27(kind, cases, tiles, ntiles, chunk, counter, j, grid, s)
+                               : launch_batch_q19(kind, cases, tiles, ntiles, chunk, counter, j, grid, s);
 }
 
 cudaError_t launch_state_hash(int precision, const StepParams& P, unsigned long long* out, cudaStream_t s) {

@@ -20,6 +20,10 @@ inline int batch_kind(int q, int precision, int features) {
     return (q == 27 ? BK_Q27_F32 : BK_Q19_F32) + precision;
 }
 
+inline int batch_q(int kind) {
+    return (kind >= BK_Q27_F32 && kind <= BK_Q27_BF16) || kind >= BK_Q27_F32_P ? 27 : 19;
+}
+
 // One resident lattice: TMA descriptors and step parameters for both directions
 // (parity s reads state s and writes state s^1).
 struct BatchCase {
@@ -42,7 +46,7 @@ struct ChunkState {
     int nsteps;
 };
 
-constexpr int kBatchW = kStepW; // rows of the batch kernel's CTAs
+constexpr int kBatchW = kStepW; // shape of the batch kernel's CTAs (step_rows)
 // Lattices resident at once: the batch kernel reads each one's step parameters (both parities)
 // from a constant-memory table of this many slots (2 x 64 x 392 bytes), as uniform loads the
 // instructions take as operands, where a copy in shared memory costs a load into a register per use.
@@ -51,9 +55,17 @@ constexpr int kBatchParamSlots = 64;
 // into that table, in stream order.
 cudaError_t upload_batch_params(const StepParams* params, int n, cudaStream_t s);
 
-cudaError_t launch_batch(const BatchCase* cases, const BatchTile* tiles, int ntiles, const ChunkState* chunk,
-                         int* counters, int j, int grid, cudaStream_t s);
-int batch_smem_bytes();
+cudaError_t upload_batch_params_q19(const StepParams* params, int n, cudaStream_t s);
+cudaError_t upload_batch_params_q27(const StepParams* params, int n, cudaStream_t s);
+
+// One time step of the tiles of one kind (launch j of a replay).  grid 0: only opt the kernel into its
+// shared memory (outside any capture).
+cudaError_t launch_batch(int kind, const BatchCase* cases, const BatchTile* tiles, int ntiles, const ChunkState* chunk,
+                         int* counter, int j, int grid, cudaStream_t s);
+cudaError_t launch_batch_q19(int kind, const BatchCase* cases, const BatchTile* tiles, int ntiles, const ChunkState* chunk,
+                             int* counter, int j, int grid, cudaStream_t s);
+cudaError_t launch_batch_q27(int kind, const BatchCase* cases, const BatchTile* tiles, int ntiles, const ChunkState* chunk,
+                             int* counter, int j, int grid, cudaStream_t s);
 
 // 64-bit order-independent hash of the fluid nodes (1..n-2 on every axis) of a state, added
 // into *out (mbcg_batch.cu)

@@ -114,6 +114,12 @@ void fill_physics(const mbcg_params& p, StepParams& P) {
     P.inv_pi_scale = p.pi_scale > 0 ? static_cast<float>(1.0 / p.pi_scale) : 0.0f;
     P.rho_mean = static_cast<float>(0.5 * (p.rho_r0 + p.rho_b0));
     P.rho_half_diff = static_cast<float>(0.5 * (p.rho_r0 - p.rho_b0));
+    {
+        // the mean density cut to 9 bits, so that rho - rho_ref of a density near it is exact
+        int e = 0;
+        const double m = std::frexp(static_cast<double>(P.rho_mean), &e);
+        P.rho_ref = static_cast<float>(std::ldexp(std::floor(m * 512.0 + 0.5), e - 9));
+    }
     P.do_bc = 1;
     P.ghost_images = 1;
 }
@@ -124,28 +130,35 @@ int choose_zchunk(const mbcg_params& p, int W) {
         if (v > 0) return v;
     }
     const long long gx = (p.nx - 2 + kStepTileX - 1) / kStepTileX;
-    const long long gy = (p.ny - 2 + W - 3) / (W - 2);
-    const int nzf = p.nz - 2;
+    const int rows = step_tile_rows(W);
+    const long long g = gx * ((p.ny - 2 + rows - 1) / rows); // tiles side by side
     int sms = 152;
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // W = 16: one CTA per SM (W = 8: two).  Pick the number of z chunks that best fills whole
-    // waves, charging each chunk the three extra planes it stages before its first destination
-    // plane.
-    sms *= W == kStepWSmall ? 2 : 1;
-    double best = -1.0;
-    int best_chunk = nzf;
-    for (long long gz = 1; gz <= std::max(1, nzf / 8); ++gz) {
-        const long long chunk = (nzf + gz - 1) / gz;
-        const long long gzr = (nzf + chunk - 1) / chunk;
-        const long long ctas = gx * gy * gzr;
-        const long long waves = (ctas + sms - 1) / sms;
-        const double fill = static_cast<double>(ctas) / static_cast<double>(waves * sms);
-        const double eff = fill * static_cast<double>(chunk) / static_cast<double>(chunk + 3);
-        if (eff > best + 1e-9) {
-            best = eff;
-            best_chunk = static_cast<int>(chunk);
+    const long long units = static_cast<long long>(sms) * (W == kStepWSmall ? 2 : 1); // CTAs at a time
+    // The depth with the shortest launch: tiles of a chunk take its planes and about three more (the two
+    // source planes outside it, and the start: 18.5 us at depth 1, 43 at 8, 127 at 32 on one tile per
+    // SM, 3.5 us a plane), run in waves, and the two-plane tiles at the ends of a non-periodic z axis
+    // fill what the last wave leaves idle.  Small lattices get thin tiles this way (32^3: depth 1, 18.5 us
+    // a step against 43 at depth 8).
+    constexpr long long kExtra = 3;
+    const int nzf = p.nz - 2, cap = z_cap(p.nz, p.bc[2]), inner = nzf - 2 * cap;
+    const long long thin = cap ? 2 * g : 0, thin_cost = cap + kExtra;
+    long long best = -1;
+    int best_chunk = inner;
+    for (int chunks = 1; chunks <= inner; ++chunks) {
+        const int chunk = (inner + chunks - 1) / chunks;
+        const int depth_chunks = (inner + chunk - 1) / chunk;
+        const long long tiles = g * depth_chunks, cost = chunk + kExtra;
+        const long long waves = (tiles + units - 1) / units, idle = waves * units - tiles;
+        long long t = waves * cost;
+        const long long room = idle * (cost / thin_cost);
+        if (thin > room) t += (thin - room + units - 1) / units * thin_cost;
+        if (best < 0 || t < best) {
+            best = t;
+            best_chunk = chunk;
         }
+        if (chunk > 1) chunks = std::max(chunks, (inner + chunk - 2) / (chunk - 1) - 1); // next smaller depth
     }
     return best_chunk;
 }
@@ -178,19 +191,19 @@ bool tma_capable(const mbcg_params& p, const void* const* f, long long pitch, in
     return get_encode() != nullptr;
 }
 
-// TMA descriptors of one state for step CTAs of W rows: rhor / rhob boxes kStepRBX x (W+2),
-// the other fields kStepMX x W, one plane deep
+// TMA descriptors of one state for step CTAs of shape W: rhor / rhob boxes kStepRBX x (rows+2),
+// the other fields kStepMX x rows, one plane deep
 int encode_maps(const mbcg_params& p, const void* const* f, long long pitch, int precision, int W, TensorMaps& T) {
     EncodeFn enc = get_encode();
     if (!enc) return fail(MBCG_E_CUDA, "cuTensorMapEncodeTiled unavailable");
-    const int es = elem_bytes(precision);
+    const int es = elem_bytes(precision), rows = step_rows(W);
     for (int i = 0; i < NF; ++i) {
         const cuuint64_t dims[3] = {static_cast<cuuint64_t>(p.nx), static_cast<cuuint64_t>(p.ny),
                                     static_cast<cuuint64_t>(p.nz)};
         const cuuint64_t strides[2] = {static_cast<cuuint64_t>(pitch * es),
                                        static_cast<cuuint64_t>(pitch * p.ny * es)};
         const cuuint32_t box[3] = {static_cast<cuuint32_t>(i < 2 ? kStepRBX : kStepMX),
-                                   static_cast<cuuint32_t>(i < 2 ? W + 2 : W), 1u};
+                                   static_cast<cuuint32_t>(i < 2 ? rows + 2 : rows), 1u};
         const cuuint32_t estr[3] = {1u, 1u, 1u};
         const CUresult r = enc(&T.m[i], es == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 3,
                                const_cast<void*>(f[i]), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -4,6 +4,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 
 #include "mbcg.h"
@@ -11,10 +12,14 @@
 
 namespace mbcg {
 
-// Step CTA shapes: W warps = W source rows (W-2 destination rows plus a halo row on each
-// side) by 32 lanes (30 destination columns plus halo).  The plain step is built for both.
-constexpr int kStepW = 16;     // default
-constexpr int kStepWSmall = 8; // two CTAs per SM
+// Step CTA shapes.  A warp is 32 lanes (30 destination columns plus halo) and two source rows, one in
+// each half of packed registers; a CTA of R source rows (R / 2 warps) owns R - 2 destination rows.
+// The plain step is built for two shapes, named by the block_rows of the C ABI:
+//   16 (default): 24 source rows, 12 warps, one CTA per SM (168 registers a thread)
+//    8:            8 source rows,  4 warps, two CTAs per SM
+constexpr int kStepW = 16;
+constexpr int kStepWSmall = 8;
+constexpr int step_rows(int w) { return w == kStepWSmall ? 8 : 24; }
 constexpr int kStepTileX = 30; // destination columns per tile
 constexpr int kStepRBX = 48;   // staged width of the rhor / rhob boxes
 constexpr int kStepMX = 40;    // staged width of the other nine boxes
@@ -33,7 +38,12 @@ cudaError_t launch_step_q27_f32(bool tma, int w, const StepParams& P, const Tens
 cudaError_t launch_step_q27_f16(bool tma, int w, const StepParams& P, const TensorMaps& T, cudaStream_t s);
 cudaError_t launch_step_q27_bf16(bool tma, int w, const StepParams& P, const TensorMaps& T, cudaStream_t s);
 int step_smem_bytes(int precision, int w);
-inline int step_tile_rows(int w) { return w - 2; }
+inline int step_tile_rows(int w) { return step_rows(w) - 2; }
+// The step addresses the planes of a tile by 32-bit byte offsets: the deepest tile it may be given.
+inline int max_zchunk(long long plane, int elem_bytes) {
+    const long long bytes = plane * elem_bytes;
+    return static_cast<int>(std::min<long long>(1 << 20, std::max<long long>(1, ((1LL << 32) - 1) / bytes - 1)));
+}
 
 // boundary functors, initial conditions, diagnostics, layout conversion (mbcg_aux.cu)
 cudaError_t launch_bc(int precision, const StepParams& P, cudaStream_t s);

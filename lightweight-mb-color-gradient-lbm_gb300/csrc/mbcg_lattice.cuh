@@ -163,6 +163,7 @@ struct StepParams {
     // scaled-deviation storage
     float rho_scale, inv_rho_scale, u_ref, inv_u_ref, pi_scale, inv_pi_scale;
     float rho_mean, rho_half_diff; // rho_nominal = rho_mean + phi * rho_half_diff
+    float rho_ref;      // density that the step's sums leave out (few bits, so that differences with it are exact)
     // launch geometry
     int zchunk;         // destination planes per CTA
     int do_bc;          // fuse the inlet/outlet functors into the step
@@ -173,6 +174,7 @@ struct StepParams {
                           // barrier nothing completes, with this limit (exercises the bail path)
     const void* a[NF];  // current state
     void* b[NF];        // next state
+    long long b_stride; // bytes between its fields, where they are equally spaced (batch kernel only)
 };
 
 // Optional parts of the step a lattice needs: bounce-back walls, a body force, density-ratio rest
@@ -215,6 +217,24 @@ MBCG_HD float noise_xi(unsigned long long seed, long long step, unsigned long lo
     unsigned long long h = mix64(seed + 0x9E3779B97F4A7C15ULL * static_cast<unsigned long long>(step + 1));
     h = mix64(h ^ (node * 4ULL + static_cast<unsigned long long>(comp)));
     return static_cast<float>(static_cast<double>(h >> 40) * (1.0 / 8388608.0) - 1.0);
+}
+
+// Tiles along z.  A periodic axis is cut into chunks of zchunk planes.  On a non-periodic one the first
+// and the last two fluid planes are tiles of their own (listed last: they fill the tail of a launch), so
+// that the chunks between them stay clear of the boundary and run without its parts (tile_is_interior).
+MBCG_HD int z_cap(int nz, int bcz) { return bcz != MBCG_BC_PERIODIC && nz >= 10 ? 2 : 0; }
+MBCG_HD int z_chunks(int nz, int bcz, int zchunk) { return (nz - 2 - 2 * z_cap(nz, bcz) + zchunk - 1) / zchunk; }
+MBCG_HD int z_tiles(int nz, int bcz, int zchunk) { return z_chunks(nz, bcz, zchunk) + (z_cap(nz, bcz) ? 2 : 0); }
+// destination planes zd0 .. zd1-1 of tile bz
+MBCG_HD void z_range(int nz, int bcz, int zchunk, int bz, int& zd0, int& zd1) {
+    const int cap = z_cap(nz, bcz), n = z_chunks(nz, bcz, zchunk);
+    if (bz < n) {
+        zd0 = 1 + cap + bz * zchunk;
+        zd1 = zd0 + zchunk < nz - 1 - cap ? zd0 + zchunk : nz - 1 - cap;
+    } else {
+        zd0 = bz == n ? 1 : nz - 1 - cap;
+        zd1 = zd0 + cap;
+    }
 }
 
 // Periodic image of a coordinate p in [-1, n] on an axis with fluid nodes 1..n-2

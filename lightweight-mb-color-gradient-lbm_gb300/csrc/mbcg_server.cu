@@ -1,5 +1,5 @@
 // mbcg_server.cu -- continuous-batching server: many lattices resident in one device arena,
-// advanced together by the persistent batch kernel (mbcg_batch.cu), one CUDA graph per batch
+// advanced together by the persistent batch kernels (mbcg_batch_kernel.cuh), one CUDA graph per batch
 // composition.  The C ABI is declared in include/mbcg.h (mbcg_server_*).
 //
 // Threads.  Client threads submit, poll, wait, fetch and release under the server mutex.  One
@@ -148,6 +148,9 @@ struct mbcg_server {
     mbcg_server_config cfg{};
     int device = 0, nsm = 152;
     cudaStream_t st = nullptr, st_io = nullptr;
+    // the graph's branches, one per kind of body (capture only)
+    cudaStream_t branch_st[BK_COUNT] = {};
+    cudaEvent_t fork_ev = nullptr, join_ev[BK_COUNT] = {};
     void* arena_base = nullptr;
     Arena arena;
     BatchCase* d_cases = nullptr;
@@ -219,6 +222,7 @@ StepParams step_params(const Request& r, int from, int* status_word) {
         P.a[i] = r.fields[from][i];
         P.b[i] = r.fields[from ^ 1][i];
     }
+    P.b_stride = static_cast<long long>(r.fstride) * r.es;
     return P;
 }
 
@@ -423,14 +427,17 @@ void make_tiles(const mbcg_server* s, int z, std::vector<TileItem>& items, std::
         const Request& r = *s->reqs.at(id);
         const int gx = (r.p.nx - 2 + kStepTileX - 1) / kStepTileX;
         const int gy = (r.p.ny - 2 + step_tile_rows(kBatchW) - 1) / step_tile_rows(kBatchW);
-        const int nzf = r.p.nz - 2;
-        const int nch = std::max(1, (nzf + z - 1) / z);
+        const int nzf = r.p.nz - 2 - 2 * z_cap(r.p.nz, r.p.bc[2]);
+        const int zmax = std::min(z, max_zchunk(r.plane, r.es));
+        const int nch = std::max(1, (nzf + zmax - 1) / zmax);
         const int depth = (nzf + nch - 1) / nch;
-        const int gz = (nzf + depth - 1) / depth;
+        const int gz = z_tiles(r.p.nz, r.p.bc[2], depth);
         zc[slot] = depth;
         const int kind = batch_kind(r.p.q, r.p.precision, r.features);
         for (int bz = 0; bz < gz; ++bz) {
-            const double planes = std::min(depth, nzf - bz * depth) + 2 + s->tile_ovh;
+            int zd0, zd1;
+            z_range(r.p.nz, r.p.bc[2], depth, bz, zd0, zd1);
+            const double planes = zd1 - zd0 + 2 + s->tile_ovh;
             for (int by = 0; by < gy; ++by)
                 for (int bx = 0; bx < gx; ++bx)
                     items.push_back({BatchTile{static_cast<uint16_t>(slot), static_cast<uint16_t>(bx),
@@ -438,7 +445,7 @@ void make_tiles(const mbcg_server* s, int z, std::vector<TileItem>& items, std::
                                      kind, planes * s->plane_ns[kind]});
         }
     }
-    // longest tiles first: the atomic queue then runs a greedy longest-processing-time schedule
+    // longest tiles first: the atomic queues then run a greedy longest-processing-time schedule
     std::stable_sort(items.begin(), items.end(), [](const TileItem& a, const TileItem& b) {
         if (a.cost != b.cost) return a.cost > b.cost;
         return a.kind < b.kind;
@@ -466,7 +473,7 @@ cudaError_t rebuild(mbcg_server* s) {
         make_tiles(s, best_z, best_items, best_zc);
     } else {
         double best = 1e300;
-        for (int z : {8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256, 512}) {
+        for (int z : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256, 512}) {
             make_tiles(s, z, items, zc);
             const double t = predict_ns(items, s->nsm);
             if (t < best * 0.999) {
@@ -477,7 +484,7 @@ cudaError_t rebuild(mbcg_server* s) {
             }
         }
     }
-    s->last_z = best_z;
+    s->last_z = s->cfg.zchunk > 0 ? best_z : std::max(best_z, 8); // 8 stands for every thinner depth
     // lattice table with this composition's depths
     for (int slot = 0; slot < s->cfg.max_live; ++slot) {
         if (!s->slot_req[slot]) continue;
@@ -490,8 +497,16 @@ cudaError_t rebuild(mbcg_server* s) {
                            sizeof(BatchCase) * s->cfg.max_live);
     if (e == cudaSuccess) e = upload_params(s);
     if (e != cudaSuccess) return e;
+    // one queue per kind, in one array
+    std::stable_sort(best_items.begin(), best_items.end(),
+                     [](const TileItem& a, const TileItem& b) { return a.kind < b.kind; });
     std::vector<BatchTile> tiles(best_items.size());
-    for (size_t i = 0; i < best_items.size(); ++i) tiles[i] = best_items[i].t;
+    int kind_tiles[BK_COUNT] = {}, kind_first[BK_COUNT] = {};
+    for (size_t i = 0; i < best_items.size(); ++i) {
+        tiles[i] = best_items[i].t;
+        kind_tiles[best_items[i].kind] += 1;
+    }
+    for (int kind = 1; kind < BK_COUNT; ++kind) kind_first[kind] = kind_first[kind - 1] + kind_tiles[kind - 1];
     const int ntiles = static_cast<int>(tiles.size());
     if (static_cast<size_t>(ntiles) > s->tiles_cap) {
         // the old queue may still be read by a replay in flight
@@ -507,14 +522,29 @@ cudaError_t rebuild(mbcg_server* s) {
         e = upload(s, s->tile_stage, &s->tile_ring, s->d_tiles, tiles.data(), tiles.size() * sizeof(BatchTile));
         if (e != cudaSuccess) return e;
     }
-    // capture: reset the per-launch counters, then chunk_steps launches
-    const int grid = std::max(1, std::min(ntiles, s->nsm));
+    // capture: reset the per-launch counters, then chunk_steps launches of each kind, the kinds on
+    // parallel branches (a lattice's next step waits for the tiles of its own kind only)
+    const int K = s->cfg.chunk_steps;
     cudaGraph_t g = nullptr;
     e = cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return e;
-    cudaError_t ec = cudaMemsetAsync(s->d_counters, 0, sizeof(int) * s->cfg.chunk_steps, s->st);
-    for (int j = 0; j < s->cfg.chunk_steps && ec == cudaSuccess; ++j)
-        ec = launch_batch(s->d_cases, s->d_tiles, ntiles, s->d_chunk, s->d_counters, j, grid, s->st);
+    cudaError_t ec = cudaMemsetAsync(s->d_counters, 0, sizeof(int) * K * BK_COUNT, s->st);
+    if (ec == cudaSuccess) ec = cudaEventRecord(s->fork_ev, s->st);
+    bool first = true;
+    for (int kind = 0; kind < BK_COUNT && ec == cudaSuccess; ++kind) {
+        if (!kind_tiles[kind]) continue;
+        cudaStream_t st = first ? s->st : s->branch_st[kind];
+        if (!first) ec = cudaStreamWaitEvent(st, s->fork_ev, 0);
+        const int grid = std::min(kind_tiles[kind], s->nsm);
+        for (int j = 0; j < K && ec == cudaSuccess; ++j)
+            ec = launch_batch(kind, s->d_cases, s->d_tiles + kind_first[kind], kind_tiles[kind], s->d_chunk,
+                              s->d_counters + kind * K + j, j, grid, st);
+        if (!first) {
+            if (ec == cudaSuccess) ec = cudaEventRecord(s->join_ev[kind], st);
+            if (ec == cudaSuccess) ec = cudaStreamWaitEvent(s->st, s->join_ev[kind], 0);
+        }
+        first = false;
+    }
     e = cudaStreamEndCapture(s->st, &g);
     if (ec != cudaSuccess) e = ec;
     if (e != cudaSuccess) {
@@ -723,9 +753,9 @@ void worker_main(mbcg_server* s) {
 
 // Calibration of the planner's cost model.  For each kernel body, one synthetic lattice whose
 // tile grid per z chunk is exactly one CTA per SM (8 x nsm/8 tiles) is stepped with deep
-// (128-plane) and shallow (16-plane) tiles: t_deep = (130 + o) c and t_shallow = 8 (18 + o) c
+// (64-plane) and shallow (16-plane) tiles: t_deep = (66 + o) c and t_shallow = 4 (18 + o) c
 // give the time c of one tile plane and the fixed cost o of a tile in planes.
-cudaError_t time_launches(mbcg_server* s, int ntiles, int reps, float* ms) {
+cudaError_t time_launches(mbcg_server* s, int kind, int ntiles, int reps, float* ms) {
     ChunkState cs{0, 0, 1 << 20};
     cudaError_t e = cudaMemcpyAsync(s->d_chunk, &cs, sizeof(cs), cudaMemcpyHostToDevice, s->st);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->d_counters, 0, sizeof(int) * (reps + 1), s->st);
@@ -733,10 +763,10 @@ cudaError_t time_launches(mbcg_server* s, int ntiles, int reps, float* ms) {
     if (e == cudaSuccess) e = cudaEventCreate(&a);
     if (e == cudaSuccess) e = cudaEventCreate(&b);
     const int grid = std::min(ntiles, s->nsm);
-    if (e == cudaSuccess) e = launch_batch(s->d_cases, s->d_tiles, ntiles, s->d_chunk, s->d_counters, 0, grid, s->st);
+    if (e == cudaSuccess) e = launch_batch(kind, s->d_cases, s->d_tiles, ntiles, s->d_chunk, s->d_counters, 0, grid, s->st);
     if (e == cudaSuccess) e = cudaEventRecord(a, s->st);
     for (int j = 1; j <= reps && e == cudaSuccess; ++j)
-        e = launch_batch(s->d_cases, s->d_tiles, ntiles, s->d_chunk, s->d_counters, j, grid, s->st);
+        e = launch_batch(kind, s->d_cases, s->d_tiles, ntiles, s->d_chunk, s->d_counters + j, j, grid, s->st);
     if (e == cudaSuccess) e = cudaEventRecord(b, s->st);
     if (e == cudaSuccess) e = cudaEventSynchronize(b);
     if (e == cudaSuccess) e = cudaEventElapsedTime(ms, a, b);
@@ -748,6 +778,7 @@ cudaError_t time_launches(mbcg_server* s, int ntiles, int reps, float* ms) {
 int calibrate(mbcg_server* s) {
     if (s->nsm % 8 != 0) return MBCG_OK; // keep the default model
     const int gx = 8, gy = s->nsm / 8;
+    constexpr int kDeep = 64, kShallow = 16, kTiles = kDeep / kShallow;
     const int reps = 4;
     double ovh_sum = 0.0;
     int ovh_n = 0;
@@ -767,7 +798,7 @@ int calibrate(mbcg_server* s) {
         p.precision = prec;
         p.nx = 2 + gx * kStepTileX;
         p.ny = 2 + gy * step_tile_rows(kBatchW);
-        p.nz = 2 + 128;
+        p.nz = 2 + kDeep;
         p.bc[0] = p.bc[1] = p.bc[2] = MBCG_BC_PERIODIC;
         p.ic = MBCG_IC_BUBBLE;
         p.bubble_radius = 40;
@@ -793,13 +824,13 @@ int calibrate(mbcg_server* s) {
         if (e == cudaSuccess && batch_kind(q, prec, r.features) != kind) e = cudaErrorInvalidValue;
         float t[2] = {0, 0};
         for (int d = 0; d < 2 && e == cudaSuccess; ++d) {
-            const int depth = d == 0 ? 128 : 16;
+            const int depth = d == 0 ? kDeep : kShallow;
             BatchCase& C = s->h_cases[0];
             C.P[0].zchunk = C.P[1].zchunk = depth;
             e = cudaMemcpyAsync(s->d_cases, &C, sizeof(C), cudaMemcpyHostToDevice, s->st);
             if (e == cudaSuccess) e = upload_batch_params(C.P, 1, s->st); // pageable: staged before return
             std::vector<BatchTile> tiles;
-            for (int bz = 0; bz < 128 / depth; ++bz)
+            for (int bz = 0; bz < kDeep / depth; ++bz)
                 for (int by = 0; by < gy; ++by)
                     for (int bx = 0; bx < gx; ++bx)
                         tiles.push_back(BatchTile{0, static_cast<uint16_t>(bx), static_cast<uint16_t>(by),
@@ -815,18 +846,19 @@ int calibrate(mbcg_server* s) {
                 e = cudaMemcpyAsync(s->d_tiles, tiles.data(), tiles.size() * sizeof(BatchTile), cudaMemcpyHostToDevice,
                                     s->st);
             float ms = 0.0f;
-            if (e == cudaSuccess) e = time_launches(s, static_cast<int>(tiles.size()), reps, &ms);
+            if (e == cudaSuccess) e = time_launches(s, kind, static_cast<int>(tiles.size()), reps, &ms);
             t[d] = ms * 1e6f / reps; // ns per launch
         }
         cudaError_t es2 = cudaStreamSynchronize(s->st);
         if (e == cudaSuccess) e = es2;
         s->arena.release(r.off, r.bytes);
         if (e != cudaSuccess) return cuda_fail(e, "calibration");
-        // t0 = (130 + o) c, t1 = 8 (18 + o) c  =>  o = (130 t1 - 144 t0) / (8 t0 - t1)
+        // t0 = (deep + 2 + o) c, t1 = tiles (shallow + 2 + o) c
         const double t0 = t[0], t1 = t[1];
-        double o = (8.0 * t0 - t1) != 0.0 ? (130.0 * t1 - 144.0 * t0) / (8.0 * t0 - t1) : 3.0;
+        const double num = (kDeep + 2) * t1 - kTiles * (kShallow + 2) * t0, den = kTiles * t0 - t1;
+        double o = den != 0.0 ? num / den : 3.0;
         o = std::min(std::max(o, 0.0), 32.0);
-        s->plane_ns[kind] = t0 / (130.0 + o);
+        s->plane_ns[kind] = t0 / (kDeep + 2 + o);
         ovh_sum += o;
         ovh_n += 1;
     }
@@ -861,6 +893,11 @@ void destroy_server(mbcg_server* s) {
     for (cudaEvent_t e : s->event_pool) cudaEventDestroy(e);
     for (cudaEvent_t e : s->inflight) cudaEventDestroy(e);
     if (s->t0_ev) cudaEventDestroy(s->t0_ev);
+    if (s->fork_ev) cudaEventDestroy(s->fork_ev);
+    for (int kind = 0; kind < BK_COUNT; ++kind) {
+        if (s->join_ev[kind]) cudaEventDestroy(s->join_ev[kind]);
+        if (s->branch_st[kind]) cudaStreamDestroy(s->branch_st[kind]);
+    }
     if (s->d_tiles) cudaFree(s->d_tiles);
     if (s->d_chunk) cudaFree(s->d_chunk);
     if (s->d_counters) cudaFree(s->d_counters);
@@ -943,14 +980,20 @@ int mbcg_server_create(const mbcg_server_config* cfg_in, mbcg_server** out) {
         if (!s->h_cases) e = cudaErrorMemoryAllocation;
     }
     if (e == cudaSuccess) e = cudaMalloc(&s->d_chunk, sizeof(ChunkState) * cfg.max_live);
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_counters, sizeof(int) * std::max(cfg.chunk_steps, 8));
+    if (e == cudaSuccess) e = cudaMalloc(&s->d_counters, sizeof(int) * std::max(cfg.chunk_steps, 8) * BK_COUNT);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->fork_ev, cudaEventDisableTiming);
+    for (int kind = 0; kind < BK_COUNT && e == cudaSuccess; ++kind) {
+        e = cudaStreamCreateWithFlags(&s->branch_st[kind], cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->join_ev[kind], cudaEventDisableTiming);
+    }
     if (e == cudaSuccess) {
         s->tiles_cap = 65536;
         e = cudaMalloc(&s->d_tiles, s->tiles_cap * sizeof(BatchTile));
     }
     if (e == cudaSuccess) e = cudaMemsetAsync(s->d_chunk, 0, sizeof(ChunkState) * cfg.max_live, s->st);
-    // opt the batch kernel into its shared memory outside any capture
-    if (e == cudaSuccess) e = launch_batch(s->d_cases, nullptr, 0, s->d_chunk, s->d_counters, 0, 0, s->st);
+    // opt the batch kernels into their shared memory outside any capture
+    for (int kind = 0; kind < BK_COUNT && e == cudaSuccess; ++kind)
+        e = launch_batch(kind, s->d_cases, nullptr, 0, s->d_chunk, s->d_counters, 0, 0, s->st);
     if (e == cudaSuccess) e = cudaEventCreate(&s->t0_ev);
     if (e == cudaSuccess) e = cudaEventRecord(s->t0_ev, s->st);
     if (e == cudaSuccess) e = cudaEventSynchronize(s->t0_ev);

@@ -21,8 +21,8 @@ cudaError_t launch_step(int q, int precision, bool tma, int w, const StepParams&
 }
 
 int step_smem_bytes(int precision, int w) {
-    if (precision == MBCG_FP32) return w == kStepWSmall ? Geo<float, kStepWSmall>::smem : Geo<float, kStepW>::smem;
-    return w == kStepWSmall ? Geo<__half, kStepWSmall>::smem : Geo<__half, kStepW>::smem;
+    if (precision == MBCG_FP32) return w == kStepWSmall ? Geo<float, step_rows(kStepWSmall)>::smem : Geo<float, step_rows(kStepW)>::smem;
+    return w == kStepWSmall ? Geo<__half, step_rows(kStepWSmall)>::smem : Geo<__half, step_rows(kStepW)>::smem;
 }
 
 } // namespace mbcg

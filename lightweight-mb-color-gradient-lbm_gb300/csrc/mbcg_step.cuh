@@ -1,47 +1,58 @@
 // mbcg_step.cuh -- fused moment-based colour-gradient time step for sm_103a (GB300).
 //
-// step_tile() advances one tile (30 columns x (W-2) rows x zchunk planes) of one lattice by one
+// step_tile() advances one tile (30 columns x (W-2) rows x a chunk of planes) of one lattice by one
 // time step of the reference's main loop (main.cu:41-45):
 //   RCS (lbm.cuh:20-262)  +  jet inlet/outlet functors (kernels.cu:102-114)  [+ swap by the host]
 // The plain step kernel runs one tile per CTA over a grid covering the lattice; the batch
-// kernel (mbcg_batch.cu) runs tiles of many lattices from a queue in persistent CTAs.  The
+// kernels (mbcg_batch_kernel.cuh) run tiles of many lattices from a queue in persistent CTAs.  The
 // translation units mbcg_step_q{19,27}_{f32,f16,bf16}.cu instantiate the plain kernel.
 //
 // Formulation.  The reference pulls, for every destination node and direction i, the post-
 // collision population of the source node x - c_i and rebuilds it from the source's 11
 // moments (feq + oms*fneqr, Omega2 and recolouring at interfaces).  Every one of those
-// populations is a polynomial in c_i whose coefficients depend only on the source node, so
-// here each source node is visited once:
-//   1. its coefficient tensor p_abc (monomials cx^a cy^b cz^c, a,b,c <= 2; 17 non-zero) is
-//      built from the moments (equilibrium, regularised non-equilibrium, Guo force,
-//      density-ratio rest term, Omega2), plus the rest-population correction r0;
-//   2. a separable inverse transform over x, y, z evaluates all Q populations g_i = w_i V(c_i)
-//      (+ r0 at i = 0); red populations are fr_i = aR g_i + Delta_i (recolouring);
-//   3. populations are streamed and projected onto the destination's moments by the
-//      separable forward transform, one axis at a time:
-//        z: the CTA marches along z; class cz of source plane k feeds destination plane k+cz,
-//        x: warp lanes are consecutive x nodes; neighbours exchange by __shfl_up/down_sync,
-//        y: warps are consecutive y rows; neighbours exchange through shared memory.
-// The colour gradient F (forces.cuh:20-60) is evaluated once per interface source node from a
-// ring of psi = (rhor - rhob)/rho planes kept in shared memory.
+// populations is w_i times a polynomial in c_i (powers a, b, c <= 2 of cx, cy, cz; 17 coefficients)
+// that depends only on the source node, and a destination needs only the moments of order <= 2 of what
+// it receives.  So each source is visited once and populations are never formed: one axis at a time,
+// the polynomial is evaluated at c_a = -1, 0, +1, the outer two values stream to the neighbours along
+// that axis, and the receiver sums its moments along it:
+//   x: the 8 coefficients (in cy^b cz^c) at cx = -1 and +1 cross to the neighbouring lanes (8 shuffles
+//      each way); the column keeps order 0, 1, 2 in x of each,
+//   y: those at cy = -1 and +1 go to the neighbouring warps' rows through shared memory (12 values each
+//      way for D3Q27, 8 for D3Q19),
+//   z: the CTA marches along z; what plane k sends with cz = -1, 0, +1 joins the sums of the destination
+//      planes k-1, k, k+1.
+// Red populations are the total's times the source's colour fraction plus the recolouring term, itself
+// a polynomial whose coefficients are multiples of one vector: an interface source sends three more
+// values along x.  The colour gradient F (forces.cuh:20-60) is evaluated once per interface source
+// from a ring of psi = (rhor - rhob)/rho planes kept in shared memory.
 //
-// Tiling.  A CTA is 32 lanes (x) x W warps (y).  Lanes 0 and 31 and warps 0 and W-1 are
+// Two nodes a thread.  A warp holds two rows of the tile, w from below and w from above, one in each
+// half of f32x2 registers, the upper one in a frame with y mirrored: both halves take the same
+// operations throughout, and every arithmetic instruction does two nodes' work.  The kernel is bound by
+// instruction issue and latency, not by HBM (D3Q27 jet 256x256x1024, FP32, measured in ncu): 560 warp
+// instructions per 32 node updates and 12 warps per SM, against 971 and 16 for one node a thread with all
+// 27 populations formed and crossing lanes; 2.72 ms -> 2.02 ms a step (24.7 -> 33.2 GLUPS).
+//
+// Tiling.  A CTA is 32 lanes (x) x W rows (y), W/2 warps.  Lanes 0 and 31 and rows 0 and W-1 are
 // halo sources; the CTA writes the 30 x (W-2) destination columns in between, for a chunk of
-// zchunk planes.  Each source plane arrives in shared memory through TMA
-// (cp.async.bulk.tensor.3d, one box per field, 4-slot ring tracked by mbarriers).  The ghost
-// frame of a periodic x / y axis holds the periodic image of the opposite fluid layer (every
-// store writes it through), so every source a tile needs is inside its staged box
+// planes.  W = 24 (12 warps, one CTA per SM) is the tallest that leaves a thread the 168 registers the
+// body needs: W = 16 with 8 warps and 220 registers took 2.69 ms on that jet.  Each source plane arrives
+// in shared memory through TMA (cp.async.bulk.tensor.3d, one box per field, 3- or 4-slot ring tracked by
+// mbarriers).  The ghost frame of a periodic x / y axis holds the periodic image of the opposite fluid
+// layer (every store writes it through), so every source a tile needs is inside its staged box
 // (bounds.cuh:34-77 wraps on read instead); the periodic images two layers out that the colour
-// gradient needs come from global memory one plane ahead.
+// gradient needs come from global memory by cp.async.  Warp 0 holds the two halo rows, so it has no
+// sums to finish: it issues the copies and prepares the psi elements around the tile meanwhile.
 //
 // Boundary kinds: periodic; inlet/outlet (the reference's ghost-source branch,
 // lbm.cuh:79-151, plus the inlet and outlet functors fused into the store of the first and
 // last fluid layer); wall (halfway bounce-back).
 //
-// Feature sets.  kFeat selects at compile time which optional parts a kernel carries:
+// Feature sets.  kFeat selects at compile time which optional parts a tile carries:
 // F_WALL (bounce-back walls), F_FORCE (body force and density-ratio rest term), F_INOUT (an
 // inlet/outlet axis).  A lattice runs on any instantiation whose set covers its parameters;
-// the smaller sets leave out code, registers and branches the lattice never uses.
+// the smaller sets leave out code, registers and branches the lattice never uses, and tiles clear of
+// the non-periodic axis leave out its parts.
 #pragma once
 
 #include <cuda.h>
@@ -63,7 +74,7 @@ constexpr int kTX = kStepTileX; // destination columns per CTA (30)
 constexpr int kRBX = kStepRBX;   // staged width of rhor/rhob rows (34 needed + 16-byte alignment slack)
 constexpr int kMX = kStepMX;     // staged width of the other 9 fields (32 needed + slack)
 constexpr int kPSX = 34;   // psi ring width (32 sources + 1 on each side)
-constexpr int kNSTAGE = 4; // planes staged: k, k+1, and k+2, k+3 in flight
+constexpr int kMaxStages = 4; // planes staged at most: k, k+1, and k+2, k+3 in flight
 constexpr unsigned kFull = 0xffffffffu;
 
 constexpr int align128(int b) { return (b + 127) / 128 * 128; }
@@ -73,6 +84,8 @@ constexpr int align128(int b) { return (b + 127) / 128 * 128; }
 // includes 128 bytes of slack for aligning the base).
 template <typename S, int W>
 struct Geo {
+    // planes staged: k, k+1, and two more in flight, or one where the tile leaves no room for two
+    static constexpr int NST = W > 16 && sizeof(S) == 4 ? 3 : kMaxStages;
     static constexpr int RBY = W + 2;
     static constexpr int MY = W;
     static constexpr int rb_field = align128(RBY * kRBX * (int)sizeof(S));
@@ -80,14 +93,21 @@ struct Geo {
     static constexpr int stage = 2 * rb_field + 9 * m_field;
     static constexpr int tx = 2 * RBY * kRBX * (int)sizeof(S) + 9 * MY * kMX * (int)sizeof(S);
     static constexpr int psi_plane = RBY * kPSX;           // floats
-    static constexpr int psi = kNSTAGE * psi_plane * 4;    // bytes (ring slot = stage slot)
-    static constexpr int xbuf_floats = 3 * 2 * 4 * W * 32; // float4 [class][slot][row][lane]
-    static constexpr int xbuf = xbuf_floats * 4;
+    static constexpr int psi = NST * psi_plane * 4;    // bytes (ring slot = stage slot)
+    static constexpr int H = W / 2;                        // warps: two rows each
+    static constexpr int xbuf = 25 * (H + 1) * 32 * 8;     // float2 [quantity][warp, one more][lane]
+    // psi elements beside the source nodes inside the lattice: the frame around the tile, and the
+    // column nx and row ny where the lattice ends inside it
+    static constexpr int frame = 2 * kPSX + 2 * W + (W + 2) + kPSX;
+    static constexpr int ftab = align128(frame * 8 + 8);   // int2 [element], then the two list lengths
+    static constexpr int fbuf = align128(frame * 8);       // uint2 [far element]: words of fields 0 and 1
     static constexpr int off_bar = 0;
     static constexpr int off_stage = 128;
-    static constexpr int off_psi = off_stage + kNSTAGE * stage;
+    static constexpr int off_psi = off_stage + NST * stage;
     static constexpr int off_xbuf = off_psi + psi;
-    static constexpr int smem = off_xbuf + xbuf + 128;
+    static constexpr int off_ftab = off_xbuf + xbuf;
+    static constexpr int off_fbuf = off_ftab + ftab;
+    static constexpr int smem = off_fbuf + fbuf + 128;
 };
 
 // ------------------------------------------------------------------ PTX helpers
@@ -128,6 +148,10 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
 }
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(__cvta_generic_to_global(src)) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ int floor8(int v) { return v & ~7; }
@@ -157,6 +181,15 @@ __device__ __forceinline__ int psi_coord(const StepParams& P, int a, int p, int 
 }
 
 // ------------------------------------------------------------------ state access
+// Fast reciprocal (<= 1 ulp, one MUFU instruction).  The flushing form: for the densities and
+// gradients it is used on (far from the subnormal range) it gives the same value as
+// __fdividef(1, v), which spends four more instructions on scaling subnormal operands.
+__device__ __forceinline__ float fast_rcp(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 template <typename S>
 struct Node {
     float rr, rb, ux, uy, uz, pxx, pxy, pyy, pyz, pzz, pxz;
@@ -166,7 +199,7 @@ template <typename S>
 __device__ __forceinline__ float psi_of(const StepParams& P, S s0, S s1) {
     if constexpr (std::is_same<S, float>::value) {
         const float r = Codec<S>::to_f(s0), b = Codec<S>::to_f(s1);
-        return __fdividef(r - b, r + b);
+        return (r - b) * fast_rcp(r + b);
     } else {
         (void)P;
         (void)s0;
@@ -177,7 +210,7 @@ __device__ __forceinline__ float psi_of(const StepParams& P, S s0, S s1) {
 // psi from the two stored slots already widened to float
 template <typename S>
 __device__ __forceinline__ float psi_of_slots(float v0, float v1) {
-    if constexpr (std::is_same<S, float>::value) return __fdividef(v0 - v1, v0 + v1);
+    if constexpr (std::is_same<S, float>::value) return (v0 - v1) * fast_rcp(v0 + v1);
     else return phi_of_slot(v1);
 }
 
@@ -195,6 +228,26 @@ __device__ __forceinline__ void decode(const StepParams& P, const float (&v)[NF]
         n.pxx = P.pi_scale * v[5]; n.pxy = P.pi_scale * v[6]; n.pyy = P.pi_scale * v[7];
         n.pyz = P.pi_scale * v[8]; n.pzz = P.pi_scale * v[9]; n.pxz = P.pi_scale * v[10];
     }
+}
+
+// decode the stored slots of this thread's two nodes; the second node's y axis is mirrored
+// (see step_tile), so its y-odd moments change sign
+template <typename S, typename N2>
+__device__ __forceinline__ void decode2(const StepParams& P, const float (&va)[NF], const float (&vb)[NF], N2& n) {
+    Node<S> a, b;
+    decode<S>(P, va, a);
+    decode<S>(P, vb, b);
+    n.rr = make_float2(a.rr, b.rr);
+    n.rb = make_float2(a.rb, b.rb);
+    n.ux = make_float2(a.ux, b.ux);
+    n.uy = make_float2(a.uy, -b.uy);
+    n.uz = make_float2(a.uz, b.uz);
+    n.pxx = make_float2(a.pxx, b.pxx);
+    n.pxy = make_float2(a.pxy, -b.pxy);
+    n.pyy = make_float2(a.pyy, b.pyy);
+    n.pyz = make_float2(a.pyz, -b.pyz);
+    n.pzz = make_float2(a.pzz, b.pzz);
+    n.pxz = make_float2(a.pxz, b.pxz);
 }
 
 // The 16-bit forms round every stored slot stochastically (`key`: the node's random stream).
@@ -231,10 +284,14 @@ __device__ __forceinline__ unsigned node_round_key(const StepParams& P, unsigned
     return base + 6U * node;
 }
 
+// Store a node at byte offset `off` from `tile` (bytes) in every field.  The offset within a tile's
+// planes fits 32 bits (the launch caps zchunk for it), so each store is a uniform base and one
+// 32-bit register instead of a 64-bit sum per field.
 template <typename S>
-__device__ __forceinline__ void store_node(const StepParams& P, long long o, const S (&v)[NF]) {
+__device__ __forceinline__ void store_node(const StepParams& P, long long tile, unsigned off, const S (&v)[NF]) {
 #pragma unroll
-    for (int f = 0; f < NF; ++f) static_cast<S*>(P.b[f])[o] = v[f];
+    for (int f = 0; f < NF; ++f)
+        *reinterpret_cast<S*>(static_cast<unsigned char*>(P.b[f]) + tile + off) = v[f];
 }
 
 template <typename S>
@@ -243,176 +300,197 @@ __device__ __forceinline__ void load_global(const StepParams& P, long long o, fl
     for (int f = 0; f < NF; ++f) v[f] = Codec<S>::to_f(static_cast<const S*>(P.a[f])[o]);
 }
 
-// ------------------------------------------------------------------ coefficient tensor
-struct Coef {
-    float p000, p100, p010, p001, p200, p020, p002, p110, p101, p011;
-    float p210, p201, p120, p102, p021, p012, p111, r0;
-};
-
-// Equilibrium (pdf.cuh:16-36) at (rho, u) + oms * regularised non-equilibrium (pdf.cuh:38-79)
-// from (Pi, v) + 1/2 Guo force (pdf.cuh:94-136) + density-ratio rest term, as the
-// coefficients of a polynomial in c (w_i factored out).
-// Phase-dependent relaxation (forces.cuh:101-108): tau_eff = (1 + psi)/2 tau_r + (1 - psi)/2 tau_b
-__device__ __forceinline__ float tau_eff_of(const StepParams& P, float rr, float rb) {
-    const float psix = (rr - rb) / (rr + rb);
-    return 0.5f * (1.0f + psix) * P.tau_r + 0.5f * (1.0f - psix) * P.tau_b;
-}
-
-template <int kFeat>
-__device__ __forceinline__ void build_coef(const StepParams& P, Coef& c, float rho, float rr, float rb, float ux,
-                                           float uy, float uz, float vx, float vy, float vz, float pxx, float pxy,
-                                           float pyy, float pyz, float pzz, float pxz) {
-    float oms = P.oms;
-    if constexpr ((kFeat & F_FORCE) != 0)
-        if (P.tau_var) oms = 1.0f - 1.0f / tau_eff_of(P, rr, rb);
-    const float usq = ux * ux + uy * uy + uz * uz;
-    const float rux = rho * ux, ruy = rho * uy, ruz = rho * uz;
-    const float t1 = 3.0f - 4.5f * usq;
-    const float a3xxy = pxx * vy + 2.0f * pxy * vx;
-    const float a3xxz = pxx * vz + 2.0f * pxz * vx;
-    const float a3xyy = pyy * vx + 2.0f * pxy * vy;
-    const float a3xzz = pzz * vx + 2.0f * pxz * vz;
-    const float a3yyz = pyy * vz + 2.0f * pyz * vy;
-    const float a3yzz = pzz * vy + 2.0f * pyz * vz;
-    const float a3xyz = pxy * vz + pxz * vy + pyz * vx;
-    const float o45 = 4.5f * oms, o9 = 9.0f * oms, o135 = 13.5f * oms;
-    // p000 holds only the small isotropic part; rho itself is added to every direction last
-    // (see emit), so the rounding of rho + small treats rest and moving populations alike
-    c.p000 = -1.5f * (rho * usq + oms * (pxx + pyy + pzz));
-    c.p100 = rux * t1 + 4.5f * rux * ux * ux - o45 * (a3xyy + a3xzz);
-    c.p010 = ruy * t1 + 4.5f * ruy * uy * uy - o45 * (a3xxy + a3yzz);
-    c.p001 = ruz * t1 + 4.5f * ruz * uz * uz - o45 * (a3xxz + a3yyz);
-    c.p200 = 4.5f * rux * ux + o45 * pxx;
-    c.p020 = 4.5f * ruy * uy + o45 * pyy;
-    c.p002 = 4.5f * ruz * uz + o45 * pzz;
-    c.p110 = 9.0f * rux * uy + o9 * pxy;
-    c.p101 = 9.0f * rux * uz + o9 * pxz;
-    c.p011 = 9.0f * ruy * uz + o9 * pyz;
-    c.p210 = 13.5f * rux * ux * uy + o135 * a3xxy;
-    c.p201 = 13.5f * rux * ux * uz + o135 * a3xxz;
-    c.p120 = 13.5f * rux * uy * uy + o135 * a3xyy;
-    c.p102 = 13.5f * rux * uz * uz + o135 * a3xzz;
-    c.p021 = 13.5f * ruy * uy * uz + o135 * a3yyz;
-    c.p012 = 13.5f * ruy * uz * uz + o135 * a3yzz;
-    c.p111 = 27.0f * rux * uy * uz + 2.0f * o135 * a3xyz;
-    c.r0 = 0.0f;
-    if constexpr ((kFeat & F_FORCE) == 0) return;
-    if (P.forced) {
-        const float Fx = rho * P.g[0], Fy = rho * P.g[1], Fz = rho * P.g[2];
-        const float Gxxy = Fx * ux * uy + 0.5f * Fy * ux * ux;
-        const float Gxxz = Fx * ux * uz + 0.5f * Fz * ux * ux;
-        const float Gxyy = Fy * ux * uy + 0.5f * Fx * uy * uy;
-        const float Gxzz = Fz * ux * uz + 0.5f * Fx * uz * uz;
-        const float Gyyz = Fy * uy * uz + 0.5f * Fz * uy * uy;
-        const float Gyzz = Fz * uy * uz + 0.5f * Fy * uz * uz;
-        const float Gxyz = Fx * uy * uz + Fy * ux * uz + Fz * ux * uy;
-        c.p000 -= 1.5f * (Fx * ux + Fy * uy + Fz * uz);
-        c.p100 += 1.5f * Fx - 4.5f * (Gxyy + Gxzz);
-        c.p010 += 1.5f * Fy - 4.5f * (Gxxy + Gyzz);
-        c.p001 += 1.5f * Fz - 4.5f * (Gxxz + Gyyz);
-        c.p200 += 4.5f * Fx * ux;
-        c.p020 += 4.5f * Fy * uy;
-        c.p002 += 4.5f * Fz * uz;
-        c.p110 += 4.5f * (Fx * uy + Fy * ux);
-        c.p101 += 4.5f * (Fx * uz + Fz * ux);
-        c.p011 += 4.5f * (Fy * uz + Fz * uy);
-        c.p210 += 13.5f * Gxxy;
-        c.p201 += 13.5f * Gxxz;
-        c.p120 += 13.5f * Gxyy;
-        c.p102 += 13.5f * Gxzz;
-        c.p021 += 13.5f * Gyyz;
-        c.p012 += 13.5f * Gyzz;
-        c.p111 += 13.5f * Gxyz;
-    }
-    if (P.ratio) {
-        const float K = rr * P.kappa_r + rb * P.kappa_b;
-        c.p000 += K;
-        c.r0 -= K;
-    }
-}
-
-// ------------------------------------------------------------------ accumulators
-// (rho, red) and (jx, xx) are packed pairs: they always take the same operations, which then
-// issue as one f32x2 instruction (add/fma.f32x2, sm_100 and later) instead of two.
-struct Acc {
-    float2 rr, jxx;
-    float jy, jz, xy, yy, yz, zz, xz;
-    __device__ __forceinline__ void zero() {
-        rr = jxx = make_float2(0.0f, 0.0f);
-        jy = jz = xy = yy = yz = zz = xz = 0.0f;
-    }
-};
-
-__device__ __forceinline__ float2 pair(float v) { return make_float2(v, v); }
-// a + f b on both halves (f = 1: a plain add, as fmaf(1, b, a) would round)
-template <int F>
-__device__ __forceinline__ float2 acc2(float2 a, float2 b) {
-    if constexpr (F == 1) return __fadd2_rn(a, b);
-    else return __ffma2_rn(pair(static_cast<float>(F)), b, a);
-}
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-    float2 r;
+// ------------------------------------------------------------------ packed pairs
+// Every thread advances two nodes of its column, one in each half of f32x2 registers
+// (add / mul / fma .rn.f32x2, sm_100 and later: two FP32 operations per issued instruction, each
+// rounded exactly like the scalar one).
+using F2 = float2;
+__device__ __forceinline__ F2 pair(float v) { return make_float2(v, v); }
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ F2 operator*(float a, F2 b) { return __fmul2_rn(pair(a), b); }
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
+    F2 r;
     asm("{.reg .b64 pa, pb, pd;\n\tmov.b64 pa, {%2, %3};\n\tmov.b64 pb, {%4, %5};\n\t"
         "sub.rn.f32x2 pd, pa, pb;\n\tmov.b64 {%0, %1}, pd;}"
         : "=f"(r.x), "=f"(r.y)
         : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
     return r;
 }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ F2 fma2(float a, F2 b, F2 c) { return __ffma2_rn(pair(a), b, c); }
+__device__ __forceinline__ F2 neg2(F2 a) { return make_float2(-a.x, -a.y); } // a free operand modifier
+__device__ __forceinline__ F2 swap2(F2 a) { return make_float2(a.y, a.x); }
+__device__ __forceinline__ F2 shfl_up2(F2 v) {
+    return make_float2(__shfl_up_sync(kFull, v.x, 1), __shfl_up_sync(kFull, v.y, 1));
+}
+__device__ __forceinline__ F2 shfl_down2(F2 v) {
+    return make_float2(__shfl_down_sync(kFull, v.x, 1), __shfl_down_sync(kFull, v.y, 1));
+}
 
-// A quantity over the three x velocities of one (cy, cz): `o` = (cx = -1, cx = +1) as an f32x2
-// pair, `c` = cx = 0.  The two outer values always take the same operations.
-struct Tri {
-    float2 o;
-    float c;
+// ------------------------------------------------------------------ source coefficients
+// Phase-dependent relaxation (forces.cuh:101-108): tau_eff = (1 + psi)/2 tau_r + (1 - psi)/2 tau_b
+__device__ __forceinline__ float tau_eff_of(const StepParams& P, float rr, float rb) {
+    const float psix = (rr - rb) / (rr + rb);
+    return 0.5f * (1.0f + psix) * P.tau_r + 0.5f * (1.0f - psix) * P.tau_b;
+}
+
+// Moments of a source pair.
+struct Node2 {
+    F2 rr, rb, ux, uy, uz, pxx, pxy, pyy, pyz, pzz, pxz;
 };
-__device__ __forceinline__ Tri tri(float base, float odd, float centre) {
-    return Tri{make_float2(base - odd, base + odd), centre};
-}
-__device__ __forceinline__ Tri operator+(Tri a, Tri b) { return Tri{__fadd2_rn(a.o, b.o), a.c + b.c}; }
-__device__ __forceinline__ Tri operator-(Tri a, Tri b) { return Tri{sub2(a.o, b.o), a.c - b.c}; }
-__device__ __forceinline__ Tri operator+(Tri a, float s) { return Tri{__fadd2_rn(a.o, pair(s)), a.c + s}; }
 
-// add one population of velocity (ex, ey, ez) to a destination's moment sums
-__device__ __forceinline__ void add_pop(Acc& a, float g, float r, int ex, int ey, int ez) {
-    a.rr.x += g;
-    a.rr.y += r;
-    if (ex) { a.jxx.x += ex * g; a.jxx.y += g; }
-    if (ey) { a.jy += ey * g; a.yy += g; }
-    if (ez) { a.jz += ez * g; a.zz += g; }
-    if (ex && ey) a.xy += ex * ey * g;
-    if (ey && ez) a.yz += ey * ez * g;
-    if (ex && ez) a.xz += ex * ez * g;
+// The post-collision population of direction c, divided by its weight and less the reference
+// density, is a polynomial in c:
+//   rhod + p000 + p100 cx + p010 cy + p001 cz + 3/2 (exx cx^2 + eyy cy^2 + ezz cz^2)
+//   + 3 (exy cx cy + exz cx cz + eyz cy cz)
+//   + 9/2 (kxxy cx^2 cy + kxxz cx^2 cz + kxyy cx cy^2 + kxzz cx cz^2 + kyyz cy^2 cz + kyzz cy cz^2)
+//   + 9 kxyz cx cy cz
+// with the numeric factors left out of the coefficients: they fold into the multiply-adds of the
+// transform.  Equilibrium (pdf.cuh:16-36) at (rho, u) + oms * regularised non-equilibrium
+// (pdf.cuh:38-79) from (Pi, v) + 1/2 Guo force (pdf.cuh:94-136); v = u except at ghost sources
+// (kGhost), whose non-equilibrium part comes from the fluid node behind them.
+struct Coef {
+    F2 p000, p100, p010, p001, exx, eyy, ezz, exy, exz, eyz;
+    F2 kxxy, kxxz, kxyy, kxzz, kyyz, kyzz, kxyz;
+};
+
+template <int kFeat>
+__device__ __forceinline__ void build_coef(const StepParams& P, Coef& c, const Node2& n, F2 rho, F2 vx, F2 vy, F2 vz,
+                                           F2 o3, F2 fgx, F2 fgy, F2 fgz) {
+    constexpr bool kGhost = (kFeat & F_INOUT) != 0, kF = (kFeat & F_FORCE) != 0;
+    const F2 r3 = 3.0f * rho;
+    const F2 nx = r3 * n.ux, ny = r3 * n.uy, nz = r3 * n.uz;
+    const F2 fxx = o3 * n.pxx, fyy = o3 * n.pyy, fzz = o3 * n.pzz;
+    const F2 fxy = o3 * n.pxy, fxz = o3 * n.pxz, fyz = o3 * n.pyz;
+    c.exx = fma2(nx, n.ux, fxx);
+    c.eyy = fma2(ny, n.uy, fyy);
+    c.ezz = fma2(nz, n.uz, fzz);
+    c.exy = fma2(nx, n.uy, fxy);
+    c.exz = fma2(nx, n.uz, fxz);
+    c.eyz = fma2(ny, n.uz, fyz);
+    F2 dxy = fxy + fxy, dxz = fxz + fxz, dyz = fyz + fyz;
+    if constexpr (!kGhost) {
+        F2 gxy = dxy, gyx = dxy, gxz = dxz, gzx = dxz, gyz = dyz, gzy = dyz, hxz = fxz;
+        F2 exx = c.exx, eyy = c.eyy, ezz = c.ezz, exy = c.exy;
+        if constexpr (kF) {
+            if (P.forced) {
+                // s_ab = 3/2 F_b u_a; the force adds s_ab + s_ba to e_ab
+                const F2 h = 1.5f * rho;
+                const F2 Fx = h * fgx, Fy = h * fgy, Fz = h * fgz;
+                const F2 sxy = Fy * n.ux, syx = Fx * n.uy, sxz = Fz * n.ux, szx = Fx * n.uz, syz = Fz * n.uy, szy = Fy * n.uz;
+                exx = c.exx = fma2(2.0f, Fx * n.ux, c.exx);
+                eyy = c.eyy = fma2(2.0f, Fy * n.uy, c.eyy);
+                ezz = c.ezz = fma2(2.0f, Fz * n.uz, c.ezz);
+                exy = c.exy = c.exy + (sxy + syx);
+                c.exz = c.exz + (sxz + szx);
+                c.eyz = c.eyz + (syz + szy);
+                gxy = gxy + sxy;
+                gyx = gyx + syx;
+                gxz = gxz + sxz;
+                gzx = gzx + szx;
+                gyz = gyz + syz;
+                gzy = gzy + szy;
+                hxz = hxz + sxz;
+            }
+        }
+        c.kxxy = fma2(gxy, n.ux, exx * n.uy);
+        c.kxxz = fma2(gxz, n.ux, exx * n.uz);
+        c.kxyy = fma2(gyx, n.uy, eyy * n.ux);
+        c.kyyz = fma2(gyz, n.uy, eyy * n.uz);
+        c.kxzz = fma2(gzx, n.uz, ezz * n.ux);
+        c.kyzz = fma2(gzy, n.uz, ezz * n.uy);
+        c.kxyz = fma2(fyz, n.ux, fma2(hxz, n.uy, exy * n.uz));
+    } else {
+        F2 qxx = nx * n.ux, qyy = ny * n.uy, qzz = nz * n.uz, qxy = nx * n.uy;
+        c.kxxy = fma2(dxy, vx, fma2(fxx, vy, qxx * n.uy));
+        c.kxxz = fma2(dxz, vx, fma2(fxx, vz, qxx * n.uz));
+        c.kxyy = fma2(dxy, vy, fma2(fyy, vx, qyy * n.ux));
+        c.kyyz = fma2(dyz, vy, fma2(fyy, vz, qyy * n.uz));
+        c.kxzz = fma2(dxz, vz, fma2(fzz, vx, qzz * n.ux));
+        c.kyzz = fma2(dyz, vz, fma2(fzz, vy, qzz * n.uy));
+        c.kxyz = fma2(fyz, vx, fma2(fxz, vy, fma2(fxy, vz, qxy * n.uz)));
+        if constexpr (kF) {
+            if (P.forced) {
+                const F2 h = 1.5f * rho;
+                const F2 Fx = h * fgx, Fy = h * fgy, Fz = h * fgz;
+                const F2 sxx = Fx * n.ux, syy = Fy * n.uy, szz = Fz * n.uz;
+                const F2 sxy = Fy * n.ux, syx = Fx * n.uy, sxz = Fz * n.ux, szx = Fx * n.uz, syz = Fz * n.uy, szy = Fy * n.uz;
+                c.exx = fma2(2.0f, sxx, c.exx);
+                c.eyy = fma2(2.0f, syy, c.eyy);
+                c.ezz = fma2(2.0f, szz, c.ezz);
+                c.exy = c.exy + (sxy + syx);
+                c.exz = c.exz + (sxz + szx);
+                c.eyz = c.eyz + (syz + szy);
+                c.kxxy = c.kxxy + fma2(sxy, n.ux, 2.0f * (sxx * n.uy));
+                c.kxxz = c.kxxz + fma2(sxz, n.ux, 2.0f * (sxx * n.uz));
+                c.kxyy = c.kxyy + fma2(syx, n.uy, 2.0f * (syy * n.ux));
+                c.kyyz = c.kyyz + fma2(syz, n.uy, 2.0f * (syy * n.uz));
+                c.kxzz = c.kxzz + fma2(szx, n.uz, 2.0f * (szz * n.ux));
+                c.kyzz = c.kyzz + fma2(szy, n.uz, 2.0f * (szz * n.uy));
+                c.kxyz = c.kxyz + fma2(sxz, n.uy, (sxy + syx) * n.uz);
+            }
+        }
+    }
+    c.p100 = fma2(-1.5f, c.kxyy + c.kxzz, nx);
+    c.p010 = fma2(-1.5f, c.kxxy + c.kyzz, ny);
+    c.p001 = fma2(-1.5f, c.kxxz + c.kyyz, nz);
+    if constexpr (kF) {
+        if (P.forced) {
+            const F2 h = 1.5f * rho;
+            c.p100 = fma2(h, fgx, c.p100);
+            c.p010 = fma2(h, fgy, c.p010);
+            c.p001 = fma2(h, fgz, c.p001);
+        }
+    }
+    // the isotropic part from the same rounded e as the anisotropic one, so that the second-order
+    // terms sum to zero over the directions
+    c.p000 = -0.5f * (c.exx + c.eyy + c.ezz);
 }
+
+// Sums of one destination pair over the directions received so far (weights scaled to integers):
+// tot (less the reference density), red (likewise less part E), the momentum and the second moments.
+struct Acc2 {
+    F2 tot, red, E, jx, jy, jz, xx, xy, yy, yz, zz, xz;
+    __device__ __forceinline__ void zero() {
+        tot = red = E = jx = jy = jz = xx = xy = yy = yz = zz = xz = make_float2(0.0f, 0.0f);
+    }
+};
 
 // ------------------------------------------------------------------ the kernel
-// fast reciprocal (MUFU-based, <= 2 ulp); the colour fraction of a pure node stays exact
-__device__ __forceinline__ float fast_rcp(float v) { return __fdividef(1.0f, v); }
 
-// Store one node at (x, y, z); on periodic x / y axes the first and last fluid layers are also
-// written to their image in the opposite ghost layer, so the next step reads every source
-// (including wrapped ones) from the staged box (bounds.cuh:34-77 wraps on read instead).
+// On periodic x / y axes the first and last fluid layers are also written to their image in the
+// opposite ghost layer, so the next step reads every source (including wrapped ones) from the staged
+// box (bounds.cuh:34-77 wraps on read instead).  tile / off: the node's address, as in store_node;
 // ix / iy: the column's periodic image in x / y (-1: none).
 template <typename S>
-__device__ __forceinline__ void finalize_store(const StepParams& P, int x, int y, int z, float rr, float rb,
-                                               float ux, float uy, float uz, const float (&pi)[6], int ix, int iy,
-                                               unsigned key_base) {
+__device__ __forceinline__ void store_images(const StepParams& P, long long tile, unsigned off, int x, int y,
+                                             const S (&out)[NF], int ix, int iy) {
+    const long long dx = static_cast<long long>(ix - x) * static_cast<int>(sizeof(S));
+    const long long dy = static_cast<long long>(iy - y) * P.pitch * static_cast<int>(sizeof(S));
+    if (ix >= 0) store_node<S>(P, tile + dx, off, out);
+    if (iy >= 0) store_node<S>(P, tile + dy, off, out);
+    if (ix >= 0 && iy >= 0) store_node<S>(P, tile + dx + dy, off, out);
+}
+// Store one node at (x, y, z) and its images.
+template <typename S>
+__device__ __forceinline__ void finalize_store(const StepParams& P, long long tile, unsigned off, int x, int y, int z,
+                                               float rr, float rb, float ux, float uy, float uz, const float (&pi)[6],
+                                               int ix, int iy, unsigned key_base) {
     const float u[3] = {ux, uy, uz};
     S out[NF];
     encode<S>(P, rr, rb, u, pi, out, sizeof(S) == 4 ? 0U : node_round_key(P, key_base, x, y, z));
-    const long long zo = static_cast<long long>(z) * P.plane;
-    store_node<S>(P, zo + static_cast<long long>(y) * P.pitch + x, out);
-    if ((ix & iy) != -1) { // either is >= 0: the faces of a periodic x / y axis only
-        if (ix >= 0) store_node<S>(P, zo + static_cast<long long>(y) * P.pitch + ix, out);
-        if (iy >= 0) store_node<S>(P, zo + static_cast<long long>(iy) * P.pitch + x, out);
-        if (ix >= 0 && iy >= 0) store_node<S>(P, zo + static_cast<long long>(iy) * P.pitch + ix, out);
-    }
+    store_node<S>(P, tile, off, out);
+    if ((ix & iy) != -1) store_images<S>(P, tile, off, x, y, out, ix, iy); // either is >= 0
 }
 
 // 128-byte aligned base of the dynamic shared memory (TMA destinations need it; every Geo
-// size carries the slack)
+// size carries the slack).  Plain pointer arithmetic on the shared array, so that the compiler
+// knows every access through it for a shared-memory one (LDS / STS with 32-bit addresses; through
+// an integer cast they become generic accesses with 64-bit address arithmetic).
 __device__ __forceinline__ unsigned char* aligned_smem_base() {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    return reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+    return smem_raw + ((128U - (smem_u32(smem_raw) & 127U)) & 127U);
 }
 
 // Initialise the stage mbarriers (one elected thread) before the first tile of a CTA.  One more
@@ -420,7 +498,7 @@ __device__ __forceinline__ unsigned char* aligned_smem_base() {
 __device__ __forceinline__ void init_stage_barriers(unsigned char* smem) {
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
     if (threadIdx.x == 0 && threadIdx.y == 0) {
-        for (int s = 0; s <= kNSTAGE; ++s) mbar_init(&bars[s], 1);
+        for (int s = 0; s <= kMaxStages; ++s) mbar_init(&bars[s], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -430,99 +508,80 @@ __device__ __forceinline__ void init_stage_barriers(unsigned char* smem) {
 // is the index of the state being written (keys the inlet noise); `phase` carries the parity
 // of the stage mbarriers from one tile of a CTA to the next (0 before the first tile).
 // Returns false if a staged plane never arrived (the status word is set and the CTA must stop).
-// kLeanZ: compile the steady-state body for an inlet/outlet z axis (the batch kernel, whose
-// lattices never have one, leaves it out).
-template <int Q, typename S, int W, bool kTMA, int kFeat, bool kLeanZ = true>
+// kStride: the next state's fields lie P.b_stride bytes apart (states the library owns).  The batch
+// kernel, whose parameters come from a table, then keeps one pointer instead of eleven.
+template <int Q, typename S, int W, bool kTMA, int kFeat, bool kStride = false>
 __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap* maps, int bx, int by, int bz,
                                           long long step, unsigned char* smem, uint32_t& phase) {
     using G = Geo<S, W>;
     float* psi_ring = reinterpret_cast<float*>(smem + G::off_psi);
-    float4* xbuf = reinterpret_cast<float4*>(smem + G::off_xbuf);
+    float2* xbuf = reinterpret_cast<float2*>(smem + G::off_xbuf);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + G::off_bar);
 
     const int lane = threadIdx.x;
     const int w = threadIdx.y;
+    constexpr int H = G::H;       // warps of the CTA
+    constexpr int kThreads = 32 * H;
+    constexpr bool kSepW = (Q == 27);
+    constexpr int kNSTAGE = G::NST;
     const int tid = w * 32 + lane;
     const int nx = P.nx, ny = P.ny, nz = P.nz;
 
     const int xb = kTX * bx;     // source column of lane 0
-    const int yb = (W - 2) * by; // source row of warp 0
-    const int xs = xb + lane, ys = yb + w;
-    const int zd0 = 1 + P.zchunk * bz;
-    const int zd1 = min(zd0 + P.zchunk, nz - 1);
+    const int yb = (W - 2) * by; // source row 0
+    const int xs = xb + lane;
+    // this thread's rows: w from below and w from above.  The second is computed in a frame with y
+    // mirrored, where both rows have warp w-1 behind them (outwards) and warp w+1 before them, so
+    // the two halves take the same operations everywhere.
+    const int wa = w, wb = W - 1 - w;
+    const int ysa = yb + wa, ysb = yb + wb;
+    int zd0, zd1; // destination planes
+    z_range(nz, P.bc[2], P.zchunk, bz, zd0, zd1);
     const int kfirst = zd0 - 2;
 
     const int xr0 = floor8(xb - 1); // first staged column of rhor/rhob
     const int xm0 = floor8(xb);     // first staged column of the other fields
     const int offRB = xb - xr0;
     const int offM = xb - xm0;
-    const int bR = (w + 1) * kRBX + lane + offRB; // this node in the rhor/rhob boxes
-    const int bM = w * kMX + lane + offM;         // this node in the other boxes
+    // these nodes in the rhor/rhob boxes and in the other boxes
+    const int bRa = (wa + 1) * kRBX + lane + offRB, bRb = (wb + 1) * kRBX + lane + offRB;
+    const int bMa = wa * kMX + lane + offM, bMb = wb * kMX + lane + offM;
 
-    const bool dest_thread = lane >= 1 && lane <= kTX && w >= 1 && w <= W - 2 && xs <= nx - 2 && ys <= ny - 2;
+    const bool dest_x = lane >= 1 && lane <= kTX && xs <= nx - 2 && w >= 1; // warp 0: the halo rows
+    const bool dest_a = dest_x && ysa <= ny - 2, dest_b = dest_x && ysb <= ny - 2;
     const int rx = axis_role<kFeat>(P, 0, xs, nx);
-    const int ry = axis_role<kFeat>(P, 1, ys, ny);
-    const bool in_xy = rx != R_OUT && ry != R_OUT;
+    const int rya = axis_role<kFeat>(P, 1, ysa, ny), ryb = axis_role<kFeat>(P, 1, ysb, ny);
+    const bool in_xy_a = rx != R_OUT && rya != R_OUT, in_xy_b = rx != R_OUT && ryb != R_OUT;
     const int ia = P.inout_axis;
-    // the node's role, given the role of its plane
-    auto role_of = [&](int rz) -> int {
+    // a node's role, given the roles of its row and plane
+    auto role_of = [&](int ry, int rz) -> int {
         if (rx == R_OUT || ry == R_OUT || rz == R_OUT) return R_OUT;
         if ((kFeat & F_WALL) && (rx == R_WALL || ry == R_WALL || rz == R_WALL)) return R_WALL;
         if ((kFeat & F_INOUT) && (rx == R_GHOST || ry == R_GHOST || rz == R_GHOST)) return R_GHOST;
         return R_FLUID;
     };
-    const int role_xy = role_of(R_FLUID); // on fluid planes
+    const int role_xy[2] = {role_of(rya, R_FLUID), role_of(ryb, R_FLUID)}; // on fluid planes
     // stochastic rounding of the 16-bit stores: key base of this step
     const unsigned key_base = sizeof(S) == 4 ? 0U : round_key_base(P.seed, step);
-    // the inlet / outlet functors run at this column (x or y axis) or on planes 1 and nz-2 (z)
-    const bool bc_xy = (kFeat & F_INOUT) && P.do_bc && (ia == 0 || ia == 1) &&
-                       ((ia == 0 ? xs : ys) == 1 || (ia == 0 ? xs : ys) == (ia == 0 ? nx : ny) - 2);
-    const bool bc_z = (kFeat & F_INOUT) && P.do_bc && ia == 2;
-    // periodic images of this column's store (x = 1 / nx-2, y = 1 / ny-2 on a periodic axis)
-    const int img_x = P.bc[0] == MBCG_BC_PERIODIC ? (xs == 1 ? nx - 1 : (xs == nx - 2 ? 0 : -1)) : -1;
-    const int img_y = P.bc[1] == MBCG_BC_PERIODIC ? (ys == 1 ? ny - 1 : (ys == ny - 2 ? 0 : -1)) : -1;
+    // periodic images of this column's stores (x = 1 / nx-2, y = 1 / ny-2 on a periodic axis)
+    auto image_of = [&](int a, int p, int n) {
+        return P.bc[a] == MBCG_BC_PERIODIC ? (p == 1 ? n - 1 : (p == n - 2 ? 0 : -1)) : -1;
+    };
+    const bool images = (image_of(0, xs, nx) & image_of(1, ysa, ny) & image_of(1, ysb, ny)) != -1; // any
 
-    // psi fill: each thread owns <= kPsiPer ring elements; their mapping never changes along z.
-    // Each element reads the staged box at the node whose stored value equals psi there (the
-    // periodic ghost frame holds images), or, for the periodic images two layers out that the
-    // box cannot hold, a global load issued one plane ahead into registers.
-    constexpr int kPsiPer = (G::psi_plane + 32 * W - 1) / (32 * W);
-    int psi_box[kPsiPer];      // box index, -1: prefetched global load, -2: no element
-    long long psi_g[kPsiPer];  // mapped (x, y) offset in global memory
-    float pf0[kPsiPer], pf1[kPsiPer];
-#pragma unroll
-    for (int j = 0; j < kPsiPer; ++j) {
-        const int e = tid + j * 32 * W;
-        psi_box[j] = -2;
-        psi_g[j] = 0;
-        pf0[j] = pf1[j] = 0.0f;
-        if (e < G::psi_plane) {
-            const int r = e / kPSX, c = e % kPSX;
-            const int gx = xb - 1 + c, gy = yb - 1 + r;
-            if (gx < -1 || gx > nx || gy < -1 || gy > ny) {
-                // beyond the ghost frame and its one-node halo: read only by the colour gradient of
-                // sources outside the lattice, whose populations reach no destination of the tile,
-                // so any staged element serves (no global load)
-                psi_box[j] = 0;
-                continue;
-            }
-            const int mx = psi_coord(P, 0, gx, nx), my = psi_coord(P, 1, gy, ny);
-            const bool px = P.bc[0] == MBCG_BC_PERIODIC, py = P.bc[1] == MBCG_BC_PERIODIC;
-            const int dx = (px && gx >= 0 && gx <= nx - 1) ? gx : mx;
-            const int dy = (py && gy >= 0 && gy <= ny - 1) ? gy : my;
-            const int bc_ = dx - xr0, br_ = dy - (yb - 1);
-            psi_box[j] = (bc_ >= 0 && bc_ < kRBX && br_ >= 0 && br_ < G::RBY) ? br_ * kRBX + bc_ : -1;
-            psi_g[j] = static_cast<long long>(my) * P.pitch + mx;
-        }
-    }
+    // psi ring: each thread fills its two nodes' elements.  pa / pb: the box element whose psi stands
+    // for the node (itself; on non-periodic x / y axes the colour-gradient rule maps ghost layers).
+    constexpr bool kMapXY = (kFeat & (F_WALL | F_INOUT)) != 0;
+    auto own_coord = [&](int a, int p, int n) {
+        const int kind = P.bc[a];
+        if (kind == MBCG_BC_INOUT) return p >= n - 1 ? n - 2 : p;
+        return kind == MBCG_BC_WALL ? min(max(p, 1), n - 2) : p;
+    };
+    const int pxo = kMapXY ? own_coord(0, xs, nx) : xs;
+    const int pya = kMapXY ? own_coord(1, ysa, ny) : ysa, pyb = kMapXY ? own_coord(1, ysb, ny) : ysb;
+    const int bPa = (pya - (yb - 1)) * kRBX + pxo - xr0, bPb = (pyb - (yb - 1)) * kRBX + pxo - xr0;
 
-    // periodic images two layers out are read from global memory; most tiles have none
-    bool far_any = false;
-#pragma unroll
-    for (int j = 0; j < kPsiPer; ++j) far_any = far_any || psi_box[j] == -1;
-    far_any = __syncthreads_or(far_any) != 0;
-
-    // Plane k lives in stage slot (k - kfirst) mod 3, and its psi in the ring slot of the same
+    // Plane k lives in stage slot (k - kfirst) mod kNSTAGE, and its psi in the ring slot of the same
     // index; the z loop advances the slot incrementally.
     auto nxt = [](int sl) -> int { return sl == kNSTAGE - 1 ? 0 : sl + 1; };
     auto prv = [](int sl) -> int { return sl == 0 ? kNSTAGE - 1 : sl - 1; };
@@ -550,7 +609,7 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
         } else {
             // plain-load path for layouts TMA cannot describe (row pitch not 16-byte aligned)
             const long long zo = static_cast<long long>(kz) * P.plane;
-            for (int e = tid; e < 2 * G::RBY * kRBX; e += 32 * W) {
+            for (int e = tid; e < 2 * G::RBY * kRBX; e += kThreads) {
                 const int f = e / (G::RBY * kRBX), r = (e / kRBX) % G::RBY, c = e % kRBX;
                 const int gx = xr0 + c, gy = yb - 1 + r;
                 S v = Codec<S>::from_f(0.0f);
@@ -558,7 +617,7 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
                     v = static_cast<const S*>(P.a[f])[zo + gy * P.pitch + gx];
                 rb_box(st, f)[r * kRBX + c] = v;
             }
-            for (int e = tid; e < 9 * G::MY * kMX; e += 32 * W) {
+            for (int e = tid; e < 9 * G::MY * kMX; e += kThreads) {
                 const int f = 2 + e / (G::MY * kMX), r = (e / kMX) % G::MY, c = e % kMX;
                 const int gx = xm0 + c, gy = yb + r;
                 S v = Codec<S>::from_f(0.0f);
@@ -586,9 +645,14 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
             return true;
         }
     };
+    // warp 0 looks at a plane before the CTA's own wait for it
+    auto peek_slot = [&](int sl) -> bool {
+        if constexpr (kTMA) return mbar_wait_bounded(&bars[sl], (par >> sl) & 1u, kWaitLimit);
+        else return true;
+    };
     // On a failed wait: flag it, drain the copies still in flight (bounded) and leave.  If the drain
     // gives up too, copies may still land in this block's shared memory after it exits, which the
-    // status cannot tell apart (a flag for it cost the ten-body batch kernel 3-5 %): the host treats
+    // status cannot tell apart (a flag for it once cost the batch kernel 3-5 %): the host treats
     // any non-zero status as a poisoned context.
     auto bail = [&](int k_issued) {
         if (tid == 0 && P.status) atomicOr(P.status, 1);
@@ -601,66 +665,151 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
     };
 
     // ---- psi ring: psi = (rhor - rhob)/rho (mathUtilities.cuh:12-19) of plane k over
-    // columns xb-1..xb+32 and rows yb-1..yb+W, colour-gradient neighbour rule applied
-    auto prefetch_psi = [&](int mz) {
-        const long long zo = static_cast<long long>(mz) * P.plane;
-#pragma unroll
-        for (int j = 0; j < kPsiPer; ++j)
-            if (psi_box[j] == -1) {
-                pf0[j] = Codec<S>::to_f(static_cast<const S*>(P.a[0])[zo + psi_g[j]]);
-                pf1[j] = Codec<S>::to_f(static_cast<const S*>(P.a[1])[zo + psi_g[j]]);
-            }
-    };
-    // mz: the plane the colour-gradient rule maps k to; plane_in_box: it is the staged plane
-    auto fill_psi = [&](int mz, bool plane_in_box, int sl, bool prefetched) {
-        float* ring = psi_ring + sl * G::psi_plane;
-        if (plane_in_box && !far_any) {
-            // every element of this tile is in the staged box (the first one of each thread
-            // always exists: the ring plane has at least 32 W elements)
-            unsigned char* st = stage_at(sl);
-            const S* r0b = rb_box(st, 0);
-            const S* r1b = rb_box(st, 1);
-            ring[tid] = psi_of<S>(P, r0b[psi_box[0]], r1b[psi_box[0]]);
-#pragma unroll
-            for (int j = 1; j < kPsiPer; ++j)
-                if (psi_box[j] >= 0) ring[tid + j * 32 * W] = psi_of<S>(P, r0b[psi_box[j]], r1b[psi_box[j]]);
-            return;
-        }
-        const long long zo = static_cast<long long>(mz) * P.plane;
-        unsigned char* st = stage_at(sl);
-        const S* r0b = rb_box(st, 0);
-        const S* r1b = rb_box(st, 1);
-#pragma unroll
-        for (int j = 0; j < kPsiPer; ++j) {
-            if (psi_box[j] == -2) continue;
-            float v;
-            if (plane_in_box && psi_box[j] >= 0) {
-                v = psi_of<S>(P, r0b[psi_box[j]], r1b[psi_box[j]]);
-            } else if (prefetched && psi_box[j] == -1) {
-                v = psi_of_slots<S>(pf0[j], pf1[j]);
+    // columns xb-1..xb+32 and rows yb-1..yb+W, colour-gradient neighbour rule applied.  mz: the plane
+    // the rule maps k to; plane_in_box: it is the staged plane.
+    // The elements that are no node of the lattice in this tile (the frame: rows yb-1 and yb+W, columns
+    // xb-1 and xb+32, and column nx and row ny where the lattice ends inside the tile) are warp 0's: it
+    // has no destination rows, so it fills them for plane k+2 while the others finish plane k.  Two lists
+    // in one table: from the front the elements whose value the staged box holds (ring position, box
+    // index), from the back those it does not, the periodic images two layers out (ring position), each
+    // with the node's (x, y) offset in global memory.  The far ones are copied to shared memory by
+    // cp.async while the plane is computed.
+    int2* ftab = reinterpret_cast<int2*>(smem + G::off_ftab);
+    int* fcount = reinterpret_cast<int*>(ftab + G::frame);
+    uint2* fbuf = reinterpret_cast<uint2*>(smem + G::off_fbuf);
+    const int col_n = nx - (xb - 1), row_n = ny - (yb - 1); // ring column / row of nx / ny
+    const bool has_col = col_n <= kPSX - 2, has_row = row_n <= W;
+    const int nframe = 2 * kPSX + 2 * W + (has_col ? W + 2 : 0) + (has_row ? kPSX : 0);
+    auto build_frame = [&]() {
+        for (int e = tid; e < nframe; e += kThreads) {
+            int r, c, i = e;
+            if (i < 2 * kPSX) {
+                r = i < kPSX ? 0 : W + 1;
+                c = i < kPSX ? i : i - kPSX;
+            } else if ((i -= 2 * kPSX) < 2 * W) {
+                r = 1 + (i >> 1);
+                c = (i & 1) ? kPSX - 1 : 0;
+            } else if ((i -= 2 * W) < W + 2 && has_col) {
+                r = i;
+                c = col_n;
             } else {
-                const long long o = zo + psi_g[j];
-                v = psi_of<S>(P, static_cast<const S*>(P.a[0])[o], static_cast<const S*>(P.a[1])[o]);
+                r = row_n;
+                c = has_col ? i - (W + 2) : i;
             }
-            ring[tid + j * 32 * W] = v;
+            const int gx = xb - 1 + c, gy = yb - 1 + r;
+            // beyond the ghost frame and its one-node halo: read only by the colour gradient of
+            // sources outside the lattice, whose populations reach no destination of the tile
+            if (gx < -1 || gx > nx || gy < -1 || gy > ny) continue;
+            const int mx = psi_coord(P, 0, gx, nx), my = psi_coord(P, 1, gy, ny);
+            const bool px = P.bc[0] == MBCG_BC_PERIODIC, py = P.bc[1] == MBCG_BC_PERIODIC;
+            const int dx = (px && gx >= 0 && gx <= nx - 1) ? gx : mx;
+            const int dy = (py && gy >= 0 && gy <= ny - 1) ? gy : my;
+            const int bc_ = dx - xr0, br_ = dy - (yb - 1);
+            const bool box = bc_ >= 0 && bc_ < kRBX && br_ >= 0 && br_ < G::RBY;
+            const int off = static_cast<int>(static_cast<long long>(my) * P.pitch + mx); // a plane is below 2^31 elements
+            const int at = atomicAdd(&fcount[box ? 0 : 1], 1);
+            ftab[box ? at : G::frame - 1 - at] = make_int2(((box ? br_ * kRBX + bc_ : 0) << 16) | (r * kPSX + c), off);
         }
+    };
+    // The 4-byte word of global memory that holds element o of field f of plane mz, and the element in it.
+    auto far_word = [&](int f, int mz, int o) -> uintptr_t {
+        return reinterpret_cast<uintptr_t>(static_cast<const S*>(P.a[f]) + static_cast<long long>(mz) * P.plane + o);
+    };
+    auto far_value = [&](unsigned word, uintptr_t at) -> S {
+        if constexpr (sizeof(S) == 4) {
+            return __uint_as_float(word);
+        } else {
+            const unsigned short h = static_cast<unsigned short>((at & 2) ? word >> 16 : word & 0xffffU);
+            return *reinterpret_cast<const S*>(&h);
+        }
+    };
+    auto fetch_far = [&](int mz) { // warp 0
+        for (int e = lane; e < fcount[1]; e += 32) {
+            const int o = ftab[G::frame - 1 - e].y;
+            cp_async4(&fbuf[e].x, reinterpret_cast<const void*>(far_word(0, mz, o) & ~uintptr_t(3)));
+            cp_async4(&fbuf[e].y, reinterpret_cast<const void*>(far_word(1, mz, o) & ~uintptr_t(3)));
+        }
+    };
+    constexpr int kFramePer = (G::frame + 31) / 32;
+    auto fill_frame = [&](int mz, bool plane_in_box, int sl) { // warp 0, after fetch_far(mz)
+        float* ring = psi_ring + sl * G::psi_plane;
+        unsigned char* st = stage_at(sl);
+        const int near = fcount[0], far = fcount[1];
+        if (plane_in_box) {
+#pragma unroll
+            for (int i = 0; i < kFramePer; ++i) {
+                const int e = lane + 32 * i;
+                if (e < near) {
+                    const int t = ftab[e].x;
+                    ring[t & 0xffff] = psi_of<S>(P, rb_box(st, 0)[t >> 16], rb_box(st, 1)[t >> 16]);
+                }
+            }
+        } else { // a few planes at the ends of a non-periodic z axis
+            for (int e = lane; e < near; e += 32) {
+                const int2 t = ftab[e];
+                const long long o = static_cast<long long>(mz) * P.plane + t.y;
+                ring[t.x & 0xffff] = psi_of<S>(P, static_cast<const S*>(P.a[0])[o], static_cast<const S*>(P.a[1])[o]);
+            }
+        }
+        cp_async_wait_all(); // this lane's words
+        for (int e = lane; e < far; e += 32) {
+            const int2 t = ftab[G::frame - 1 - e];
+            const uint2 v = fbuf[e];
+            ring[t.x & 0xffff] = psi_of<S>(P, far_value(v.x, far_word(0, mz, t.y)), far_value(v.y, far_word(1, mz, t.y)));
+        }
+    };
+    // psi of this thread's nodes into the ring; c0, c1: the nodes' own stored slots (fields 0 and 1)
+    const int rPa = (wa + 1) * kPSX + lane + 1, rPb = (wb + 1) * kPSX + lane + 1; // ring elements
+    const bool lat_a = xs < nx && ysa < ny, lat_b = xs < nx && ysb < ny; // nodes of the lattice
+    auto fill_own = [&](auto mapped, int mz, bool plane_in_box, int sl, F2 c0, F2 c1) {
+        float* ring = psi_ring + sl * G::psi_plane;
+        if constexpr (decltype(mapped)::value) {
+            S a0, a1, b0, b1;
+            if (plane_in_box) {
+                unsigned char* st = stage_at(sl);
+                a0 = rb_box(st, 0)[bPa];
+                a1 = rb_box(st, 1)[bPa];
+                b0 = rb_box(st, 0)[bPb];
+                b1 = rb_box(st, 1)[bPb];
+            } else { // (nodes outside the lattice: any node serves, their psi is not stored)
+                const long long x = min(pxo, nx - 1), z = static_cast<long long>(mz) * P.plane;
+                const long long oa = z + min(pya, ny - 1) * P.pitch + x, ob = z + min(pyb, ny - 1) * P.pitch + x;
+                a0 = static_cast<const S*>(P.a[0])[oa];
+                a1 = static_cast<const S*>(P.a[1])[oa];
+                b0 = static_cast<const S*>(P.a[0])[ob];
+                b1 = static_cast<const S*>(P.a[1])[ob];
+            }
+            if (lat_a) ring[rPa] = psi_of<S>(P, a0, a1);
+            if (lat_b) ring[rPb] = psi_of<S>(P, b0, b1);
+        } else {
+            if (lat_a) ring[rPa] = psi_of_slots<S>(c0.x, c1.x);
+            if (lat_b) ring[rPb] = psi_of_slots<S>(c0.y, c1.y);
+        }
+    };
+    // fields 0 and 1 of this thread's nodes on a staged plane
+    auto load_colours = [&](int sl, F2& c0, F2& c1) {
+        unsigned char* st = stage_at(sl);
+        c0 = make_float2(Codec<S>::to_f(rb_box(st, 0)[bRa]), Codec<S>::to_f(rb_box(st, 0)[bRb]));
+        c1 = make_float2(Codec<S>::to_f(rb_box(st, 1)[bRa]), Codec<S>::to_f(rb_box(st, 1)[bRb]));
     };
 
     // ---- set-up ------------------------------------------------------------------
     // every thread is done with the previous tile's shared memory before it is refilled
     __syncthreads();
-    int k_issued = kfirst + kNSTAGE - 1;
-    for (int k = kfirst; k <= k_issued; ++k) issue(k, k - kfirst);
+    for (int k = kfirst; k < kfirst + kNSTAGE; ++k) issue(k, k - kfirst);
+    if (tid < 2) fcount[tid] = 0;
+    __syncthreads();
+    build_frame();
     if constexpr (!kTMA) __syncthreads();
     {
         // The first wait.  Testing only (wait_test_cycles > 0): it waits on the barrier nothing
         // completes, with that limit, so it runs out and the tile takes the bail path with all its
         // planes in flight.  (Folded into the one wait: a second wait-and-bail path at the tile
-        // start cost the ten-body batch kernel ~20 %.)
+        // start once cost the batch kernel ~20 %.)
         bool ok = true;
         if constexpr (kTMA) {
             const bool test = P.wait_test_cycles > 0;
-            ok = mbar_wait_bounded(test ? &bars[kNSTAGE] : &bars[0], test ? 0u : (par & 1u),
+            ok = mbar_wait_bounded(test ? &bars[kMaxStages] : &bars[0], test ? 0u : (par & 1u),
                                    test ? static_cast<long long>(P.wait_test_cycles) : kWaitLimit);
             if (ok) {
                 par ^= 1u;
@@ -669,596 +818,841 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
         }
         ok = ok && wait_slot(kfirst + 1, 1);
         if (__syncthreads_or(!ok)) {
-            bail(k_issued);
+            bail(kfirst + kNSTAGE - 1);
             return false;
         }
     }
+    F2 c0, c1; // stored slots 0 and 1 of this thread's nodes on the next plane to be a source
     {
         const int m0 = psi_coord(P, 2, kfirst, nz), m1 = psi_coord(P, 2, kfirst + 1, nz);
-        fill_psi(m0, m0 == zload(kfirst), 0, false);
-        fill_psi(m1, m1 == zload(kfirst + 1), 1, false);
+        load_colours(0, c0, c1);
+        fill_own(std::bool_constant<kMapXY>{}, m0, m0 == zload(kfirst), 0, c0, c1);
+        load_colours(1, c0, c1);
+        fill_own(std::bool_constant<kMapXY>{}, m1, m1 == zload(kfirst + 1), 1, c0, c1);
+        if (w == 0) {
+            for (int i = 0; i < 3; ++i) {
+                const int m = psi_coord(P, 2, kfirst + i, nz);
+                fetch_far(m);
+                if (i < 2 || peek_slot(i)) fill_frame(m, m == zload(kfirst + i), i);
+            }
+        }
     }
-    if (far_any) prefetch_psi(psi_coord(P, 2, kfirst + 2, nz));
+    if constexpr (kTMA) {
+        __syncthreads(); // plane kfirst is a source of nothing: its slot is free
+        if (kfirst + kNSTAGE <= zd1 + 1) issue(kfirst + kNSTAGE, 0);
+    }
 
-    Acc accP, accC, accN; // destination planes k-1, k, k+1
+    // store addresses: bytes from the tile's first destination plane, advanced plane by plane
+    const long long tile_base = static_cast<long long>(zd0) * P.plane * static_cast<int>(sizeof(S));
+    const unsigned plane_bytes = static_cast<unsigned>(P.plane) * static_cast<unsigned>(sizeof(S));
+    unsigned off_a = (static_cast<unsigned>(ysa) * static_cast<unsigned>(P.pitch) + static_cast<unsigned>(xs)) *
+                           static_cast<unsigned>(sizeof(S));
+    unsigned off_b = (static_cast<unsigned>(ysb) * static_cast<unsigned>(P.pitch) + static_cast<unsigned>(xs)) *
+                           static_cast<unsigned>(sizeof(S));
+
+    Acc2 accP, accC; // destination planes k-1 and k
     accP.zero();
     accC.zero();
-    accN.zero();
 
-    constexpr float cs2 = 1.0f / 3.0f;
-    float4* xb_self = xbuf + w * 32 + lane; // (X0, XR, X1, X2) of one exported row
+    // inlet / outlet functors fused into the store of the first and last fluid layer: the ghost node
+    // behind node (xs, ys, d), whose new moments are given
+    auto boundary = [&](int ys, int bR, int bM, unsigned char* st, int d, float rr, float rb, float ux, float uy,
+                        float uz, const float (&pi)[6]) {
+        if (ia < 0 || !P.do_bc) return;
+        const int pa = ia == 0 ? xs : (ia == 1 ? ys : d);
+        if (pa != 1 && pa != (ia == 0 ? nx : (ia == 1 ? ny : nz)) - 2) return;
+        const bool inlet = pa == 1;
+        const int gx = ia == 0 ? (inlet ? 0 : nx - 1) : xs;
+        const int gy = ia == 1 ? (inlet ? 0 : ny - 1) : ys;
+        const int gz = ia == 2 ? (inlet ? 0 : nz - 1) : d;
+        const long long og = static_cast<long long>(gz) * P.plane + static_cast<long long>(gy) * P.pitch + gx;
+        float orr, orb, oux, ouy, ouz;
+        if (inlet) {
+            // jet/boundary_conditions.cuh:16-39 (+ seeded per-node noise)
+            const int t0 = ia == 0 ? ys : xs;
+            const int t1 = ia == 2 ? ys : d;
+            const float du = static_cast<float>(t0) - P.jet_c0;
+            const float dv = static_cast<float>(t1) - P.jet_c1;
+            const float m = (du * du + dv * dv) <= (P.jet_radius * P.jet_radius) ? 1.0f : 0.0f;
+            orr = P.jet_blue ? (1.0f - m) * P.rho_r0 : m * P.rho_r0;
+            orb = P.jet_blue ? m * P.rho_b0 : (1.0f - m) * P.rho_b0;
+            float gu[3] = {0.0f, 0.0f, 0.0f};
+            if (m != 0.0f) {
+                if (P.noise_amp != 0.0f) {
+                    const unsigned long long node = static_cast<unsigned long long>(gx) +
+                                                    static_cast<unsigned long long>(gy) * nx +
+                                                    static_cast<unsigned long long>(gz) * nx * ny;
+                    gu[0] = m * P.noise_amp * noise_xi(P.seed, step, node, 0);
+                    gu[1] = m * P.noise_amp * noise_xi(P.seed, step, node, 1);
+                    gu[2] = m * P.noise_amp * noise_xi(P.seed, step, node, 2);
+                }
+            }
+            oux = gu[0] + (ia == 0 ? m * P.jet_velocity : 0.0f);
+            ouy = gu[1] + (ia == 1 ? m * P.jet_velocity : 0.0f);
+            ouz = gu[2] + (ia == 2 ? m * P.jet_velocity : 0.0f);
+        } else if (P.outlet == MBCG_OUTLET_ZERO_GRADIENT) {
+            orr = rr; orb = rb; oux = ux; ouy = uy; ouz = uz;
+        } else {
+            // convective outlet (jet/boundary_conditions.cuh:45-109), old ghost from A
+            float ov[NF];
+            if (ia == 2) {
+                ov[0] = Codec<S>::to_f(rb_box(st, 0)[bR]);
+                ov[1] = Codec<S>::to_f(rb_box(st, 1)[bR]);
+#pragma unroll
+                for (int f = 2; f < NF; ++f) ov[f] = Codec<S>::to_f(m_box(st, f)[bM]);
+            } else {
+                load_global<S>(P, og, ov);
+            }
+            Node<S> on{};
+            decode<S>(P, ov, on);
+            const float ua = ia == 0 ? ux : (ia == 1 ? uy : uz);
+            const float uc = fminf(fmaxf(ua, 0.0f), 1.0f);
+            if (on.rr + on.rb <= 1.0e-20f) {
+                orr = rr; orb = rb; oux = ux; ouy = uy; ouz = uz;
+            } else {
+                orr = on.rr - uc * (on.rr - rr);
+                orb = on.rb - uc * (on.rb - rb);
+                oux = on.ux - uc * (on.ux - ux);
+                ouy = on.uy - uc * (on.uy - uy);
+                ouz = on.uz - uc * (on.uz - uz);
+            }
+        }
+        const int gix = P.bc[0] == MBCG_BC_PERIODIC ? (gx == 1 ? nx - 1 : (gx == nx - 2 ? 0 : -1)) : -1;
+        const int giy = P.bc[1] == MBCG_BC_PERIODIC ? (gy == 1 ? ny - 1 : (gy == ny - 2 ? 0 : -1)) : -1;
+        finalize_store<S>(P, og * static_cast<int>(sizeof(S)), 0U, gx, gy, gz, orr, orb, oux, ouy, ouz, pi, gix, giy, key_base);
+    };
 
     int sl = 1; // slot of plane k (k starts at kfirst + 1)
     int k = zd0 - 1;
-    // One plane of the z-march with the feature set kFB: the tile's own, or, on the steady-state
-    // planes of an inlet/outlet z axis, the same set without the inlet/outlet parts.  Returns false
-    // after a bail.
-    auto plane = [&](auto featc) -> bool {
-        constexpr int kFB = decltype(featc)::value;
+    for (; k <= zd1; ++k, sl = nxt(sl)) {
         const int sl_next = nxt(sl), sl_prev = prv(sl);
         // (1) psi of plane k+1; one barrier both publishes the ring and makes the bail decision
-        // uniform (a plane that never arrived leaves garbage in the ring, which nobody reads)
+        // uniform (a plane that never arrived leaves garbage in the ring, which nobody reads).
         // Plane coordinates: every mapping (staging, colour-gradient rule, node role) is the
         // identity while planes k .. k+3 are fluid planes, which is almost every plane.
-        const bool zid = k >= 1 && k + kNSTAGE - 1 <= nz - 2;
+        const bool zid = k >= 1 && k + 3 <= nz - 2;
         int mz1 = k + 1, mz2 = k + 2, rz = R_FLUID;
-        bool inbox1 = true;
+        bool inbox1 = true, inbox2 = true;
         if (!zid) {
             mz1 = psi_coord(P, 2, k + 1, nz);
             inbox1 = mz1 == zload(k + 1);
             mz2 = psi_coord(P, 2, k + 2, nz);
-            rz = axis_role<kFB>(P, 2, k, nz);
+            inbox2 = mz2 == zload(k + 2);
+            rz = axis_role<kFeat>(P, 2, k, nz);
         }
+        const F2 s0 = c0, s1 = c1; // fields 0 and 1 at plane k
         {
             const bool ok = wait_slot(k + 1, sl_next);
-            if (ok) fill_psi(mz1, inbox1, sl_next, true);
+            load_colours(sl_next, c0, c1);
+            if (ok) fill_own(std::bool_constant<kMapXY>{}, mz1, inbox1, sl_next, c0, c1);
             if (__syncthreads_or(!ok)) {
-                bail(k_issued);
+                bail(min(zd1 + 1, k - 1 + kNSTAGE));
                 return false;
             }
         }
-        if (far_any && k + 2 <= zd1 + 1) prefetch_psi(mz2);
-        // (2) prefetch plane k+3 into the slot plane k-1 used
-        if (k + kNSTAGE - 1 <= zd1 + 1 && k + kNSTAGE - 1 > k_issued) {
-            issue(k + kNSTAGE - 1, sl_prev);
-            k_issued = k + kNSTAGE - 1;
-        }
+        if (w == 0 && k + 2 <= zd1 + 1) fetch_far(mz2); // far psi elements of plane k+2, used in (4)
+        // (2) plain loads: plane k+kNSTAGE-1 into the slot plane k-1 used (TMA: at the end of (4))
+        if constexpr (!kTMA)
+            if (k + kNSTAGE - 1 <= zd1 + 1) issue(k + kNSTAGE - 1, sl_prev);
 
-        // (3) this thread's source node at plane k
-        const int role = zid ? role_xy : role_of(rz);
+        // (3) this thread's source nodes at plane k
+        const int role_a = zid ? role_xy[0] : role_of(rya, rz), role_b = zid ? role_xy[1] : role_of(ryb, rz);
         // Sources outside the lattice (lanes / rows past the last ghost layer) only ever stream
         // into nodes that are not destinations of this tile, so without walls every source is
         // processed branch-free; wall ghost layers hold data and must not emit.
-        const bool active = ((kFB & F_WALL) == 0) || (role == R_FLUID || role == R_GHOST);
+        const bool act_a = ((kFeat & F_WALL) == 0) || (role_a == R_FLUID || role_a == R_GHOST);
+        const bool act_b = ((kFeat & F_WALL) == 0) || (role_b == R_FLUID || role_b == R_GHOST);
 
         unsigned char* st = stage_at(sl);
-        Node<S> nd{};
-        Node<S> fn{}; // first-fluid node of a ghost source (lbm.cuh:85-89)
-        if (active) {
-            float v[NF];
-            v[0] = Codec<S>::to_f(rb_box(st, 0)[bR]);
-            v[1] = Codec<S>::to_f(rb_box(st, 1)[bR]);
+        Node2 nd;
+        F2 vx, vy, vz; // velocity of the non-equilibrium part
+        {
+            float va[NF], vb[NF];
 #pragma unroll
-            for (int f = 2; f < NF; ++f) v[f] = Codec<S>::to_f(m_box(st, f)[bM]);
-            decode<S>(P, v, nd);
-            if constexpr ((kFB & F_INOUT) != 0) {
-                if (role == R_GHOST) {
-                    // the first fluid node behind the ghost: plane 1 or nz-2 (still staged: the
-                    // slot of plane nz-2 is not refilled in the chunk that ends at nz-1), or the
-                    // neighbouring column / row of the staged plane
+            for (int f = 2; f < NF; ++f) {
+                va[f] = Codec<S>::to_f(m_box(st, f)[bMa]);
+                vb[f] = Codec<S>::to_f(m_box(st, f)[bMb]);
+            }
+            va[0] = s0.x;
+            vb[0] = s0.y;
+            va[1] = s1.x;
+            vb[1] = s1.y;
+            decode2<S>(P, va, vb, nd);
+            vx = nd.ux;
+            vy = nd.uy;
+            vz = nd.uz;
+            if constexpr ((kFeat & F_INOUT) != 0) {
+                // a ghost source (lbm.cuh:85-89) takes Pi and its velocity from the first fluid node
+                // behind it: plane 1 or nz-2 (still staged: the slot of plane nz-2 is not refilled in
+                // the chunk that ends at nz-1), or the neighbouring column / row of the staged plane
+                auto ghost = [&](int role, int ryh, int ysh, int bMh, float (&v)[NF]) {
+                    if (role != R_GHOST) return;
                     const unsigned char* sf = st;
-                    int b2 = bM;
+                    int b2 = bMh;
                     if (rz == R_GHOST) {
                         sf = stage_at(k == 0 ? sl_next : sl_prev);
                     } else {
                         const int dx = (rx == R_GHOST) ? (xs == 0 ? 1 : -1) : 0;
-                        const int dy = (ry == R_GHOST) ? (ys == 0 ? 1 : -1) : 0;
-                        b2 = bM + dy * kMX + dx;
+                        const int dy = (ryh == R_GHOST) ? (ysh == 0 ? 1 : -1) : 0;
+                        b2 = bMh + dy * kMX + dx;
                     }
-                    float u[NF];
 #pragma unroll
                     for (int f = 2; f < NF; ++f)
-                        u[f] = Codec<S>::to_f(reinterpret_cast<const S*>(sf + 2 * G::rb_field + (f - 2) * G::m_field)[b2]);
-                    u[0] = u[1] = 1.0f;
-                    decode<S>(P, u, fn);
+                        v[f] = Codec<S>::to_f(reinterpret_cast<const S*>(sf + 2 * G::rb_field + (f - 2) * G::m_field)[b2]);
+                };
+                if (role_a == R_GHOST || role_b == R_GHOST) {
+                    ghost(role_a, rya, ysa, bMa, va);
+                    ghost(role_b, ryb, ysb, bMb, vb);
+                    Node2 fn;
+                    decode2<S>(P, va, vb, fn);
+                    vx = fn.ux;
+                    vy = fn.uy;
+                    vz = fn.uz;
+                    nd.pxx = fn.pxx; nd.pxy = fn.pxy; nd.pyy = fn.pyy;
+                    nd.pyz = fn.pyz; nd.pzz = fn.pzz; nd.pxz = fn.pxz;
                 }
             }
         }
+        if constexpr ((kFeat & F_WALL) != 0) {
+            // a wall source emits nothing: the reference density of the second colour at rest
+            auto rest = [&](bool act, float& rr, float& rb, float& a0, float& a1, float& a2, float& a3, float& a4,
+                            float& a5, float& a6, float& a7, float& a8) {
+                if (act) return;
+                rr = 0.0f;
+                rb = P.rho_ref;
+                a0 = a1 = a2 = a3 = a4 = a5 = a6 = a7 = a8 = 0.0f;
+            };
+            rest(act_a, nd.rr.x, nd.rb.x, nd.ux.x, nd.uy.x, nd.uz.x, nd.pxx.x, nd.pxy.x, nd.pyy.x, nd.pyz.x, nd.pzz.x, nd.pxz.x);
+            rest(act_b, nd.rr.y, nd.rb.y, nd.ux.y, nd.uy.y, nd.uz.y, nd.pxx.y, nd.pxy.y, nd.pyy.y, nd.pyz.y, nd.pzz.y, nd.pxz.y);
+        }
 
-        // coefficient tensor and colour split; inactive sources keep all-zero coefficients
-        Coef cf{};
-        float aR = 0.0f, dcoef = 0.0f, Fx = 0.0f, Fy = 0.0f, Fz = 0.0f, omega2_rest = 0.0f;
-        bool iface = false;
-        if (active) {
-            const float rho = nd.rr + nd.rb;
-            const float inv = fast_rcp(rho);
-            // colour fraction as a correctly rounded quotient (one residual correction): a
-            // product with a rounded reciprocal is biased (aR rho - rr averages +2.5e-10 per
-            // mixed node), which would move colour mass the same way every step
-            const float q0 = nd.rr * inv;
-            const float q1 = fmaf(fmaf(-q0, rho, nd.rr), inv, q0);
-            aR = nd.rb == 0.0f ? 1.0f : (nd.rr == 0.0f ? 0.0f : q1);
-            if (!(kFB & F_INOUT) || role == R_FLUID) {
-                iface = (4.0f * nd.rr * nd.rb * inv * inv) > 1.0e-4f; // lbm.cuh:181,187
-                // zero-filled staging outside the lattice decodes to a mixed node in the 16-bit
-                // forms; keep those (never written) sources off the interface path
-                if constexpr (sizeof(S) != 4) iface = iface && in_xy;
-                build_coef<kFB>(P, cf, rho, nd.rr, nd.rb, nd.ux, nd.uy, nd.uz, nd.ux, nd.uy, nd.uz, nd.pxx, nd.pxy,
-                                  nd.pyy, nd.pyz, nd.pzz, nd.pxz);
-            } else {
-                build_coef<kFB>(P, cf, rho, nd.rr, nd.rb, nd.ux, nd.uy, nd.uz, fn.ux, fn.uy, fn.uz, fn.pxx, fn.pxy,
-                                  fn.pyy, fn.pyz, fn.pzz, fn.pxz);
+        const F2 ref = pair(P.rho_ref);
+        const F2 rho = nd.rr + nd.rb;
+        const F2 inv = make_float2(fast_rcp(rho.x), fast_rcp(rho.y));
+        // Colour fraction as a correctly rounded quotient (one residual correction): a product with
+        // a rounded reciprocal is biased (aR rho - rr averages +2.5e-10 per mixed node), which would
+        // move colour mass the same way every step.
+        const F2 q0 = nd.rr * inv;
+        const F2 aR = fma2(fma2(neg2(q0), rho, nd.rr), inv, q0);
+        // Red populations are W (rr + aR sm) + Delta, sm the population's part without the density.
+        // In a near-steady state every rounding repeats from step to step and moves red mass the same
+        // way (1.3e-5 in 10^4 steps on the 64^3 D3Q19 bubble when rr was rounded once more on its
+        // way), so rr travels in two parts: rho_ref times the colour fraction on a 2^-16 grid, whose
+        // weighted sums are exact in FP32, and the small rest rl.  Likewise the density: rhod, what it
+        // has over rho_ref, is the sum of both colours' rests.  In a pure phase the grid part is 0 or 1
+        // and rl is 0 or rhod: the red sums are then 0 or the total's own bits.
+        auto grid = [](F2 a) { return (a + pair(192.0f)) - pair(192.0f); };
+        const F2 ec = grid(aR);
+        const F2 rl = fma2(-P.rho_ref, ec, nd.rr);
+        const F2 rhod = rl + fma2(P.rho_ref, ec, nd.rb - ref);
+        const F2 ind = 4.0f * nd.rr * nd.rb * inv * inv; // lbm.cuh:181,187
+        bool if_a = ind.x > 1.0e-4f, if_b = ind.y > 1.0e-4f;
+        if constexpr ((kFeat & F_INOUT) != 0) {
+            if_a = if_a && role_a == R_FLUID;
+            if_b = if_b && role_b == R_FLUID;
+        }
+        // zero-filled staging outside the lattice: keep those (never written) sources off the
+        // interface path in the 16-bit forms
+        if constexpr (sizeof(S) != 4) {
+            if_a = if_a && in_xy_a;
+            if_b = if_b && in_xy_b;
+        }
+        const F2 o3 = [&]() {
+            if constexpr ((kFeat & F_FORCE) != 0) {
+                if (P.tau_var)
+                    return make_float2(3.0f * (1.0f - 1.0f / tau_eff_of(P, nd.rr.x, nd.rb.x)),
+                                       3.0f * (1.0f - 1.0f / tau_eff_of(P, nd.rr.y, nd.rb.y)));
+            }
+            return pair(3.0f * P.oms);
+        }();
+        F2 fgx = pair(0.0f), fgy = fgx, fgz = fgx; // acceleration at the source, mirrored frame
+        if constexpr ((kFeat & F_FORCE) != 0) {
+            fgx = make_float2(act_a ? P.g[0] : 0.0f, act_b ? P.g[0] : 0.0f);
+            fgy = make_float2(act_a ? P.g[1] : 0.0f, act_b ? -P.g[1] : 0.0f);
+            fgz = make_float2(act_a ? P.g[2] : 0.0f, act_b ? P.g[2] : 0.0f);
+        }
+        Coef cf;
+        build_coef<kFeat & ~F_INOUT>(P, cf, nd, rho, nd.ux, nd.uy, nd.uz, o3, fgx, fgy, fgz);
+        if constexpr ((kFeat & F_INOUT) != 0) {
+            // ghost sources only: the same node as a fluid source keeps the same bits in any tile
+            if (role_a == R_GHOST || role_b == R_GHOST) {
+                Coef cg;
+                build_coef<kFeat>(P, cg, nd, rho, vx, vy, vz, o3, fgx, fgy, fgz);
+                auto sel = [&](F2& c, F2 g) {
+                    if (role_a == R_GHOST) c.x = g.x;
+                    if (role_b == R_GHOST) c.y = g.y;
+                };
+                sel(cf.p000, cg.p000); sel(cf.p100, cg.p100); sel(cf.p010, cg.p010); sel(cf.p001, cg.p001);
+                sel(cf.exx, cg.exx); sel(cf.eyy, cg.eyy); sel(cf.ezz, cg.ezz);
+                sel(cf.exy, cg.exy); sel(cf.exz, cg.exz); sel(cf.eyz, cg.eyz);
+                sel(cf.kxxy, cg.kxxy); sel(cf.kxxz, cg.kxxz); sel(cf.kxyy, cg.kxyy); sel(cf.kxzz, cg.kxzz);
+                sel(cf.kyyz, cg.kyyz); sel(cf.kyzz, cg.kyzz); sel(cf.kxyz, cg.kxyz);
             }
         }
-        const bool any_iface = __any_sync(kFull, iface);
-        if (any_iface && iface) {
-            // colour gradient at the source (forces.cuh:20-60) from the psi ring
+        // rest-population correction in value units before the rest weight (64 of 216, or 12 of 36)
+        F2 rc0 = pair(0.0f);
+        if constexpr ((kFeat & F_FORCE) != 0) {
+            if (P.ratio) {
+                F2 K = fma2(P.kappa_r, nd.rr, P.kappa_b * nd.rb);
+                if (!act_a) K.x = 0.0f;
+                if (!act_b) K.y = 0.0f;
+                cf.p000 = cf.p000 + K;
+                rc0 = (kSepW ? -3.375f : -3.0f) * K;
+            }
+        }
+
+        // Interface sources: Omega2 into the coefficients, and the recolouring vector dF = d F, of
+        // which Delta_c = W d(|c|) (F . c), d(|c|) = d / |c| (collisionOperators.cuh:60-80).  Other
+        // sources have F = 0, which changes none of their sums, so a warp may take either side.
+        const bool any_iface = __any_sync(kFull, if_a || if_b);
+        F2 dFx = pair(0.0f), dFy = dFx, dFz = dFx;
+        if (any_iface) {
             const float* rm = psi_ring + sl_prev * G::psi_plane;
             const float* r0p = psi_ring + sl * G::psi_plane;
             const float* rp = psi_ring + sl_next * G::psi_plane;
-            float sx = 0.0f, sy = 0.0f, sz = 0.0f;
+            // colour gradient (forces.cuh:20-60) from the psi ring, rows in the mirrored frame of
+            // the second node: R[dy][dz] weighted row sums, D[dy][dz] row differences along x
+            F2 R[3][3], D[3][3];
 #pragma unroll
-            for (int dz = -1; dz <= 1; ++dz) {
-                const float* ring = dz < 0 ? rm : (dz == 0 ? r0p : rp);
+            for (int dz = -1; dz <= 1; ++dz)
 #pragma unroll
                 for (int dy = -1; dy <= 1; ++dy) {
-#pragma unroll
-                    for (int dx = -1; dx <= 1; ++dx) {
-                        if (dx == 0 && dy == 0 && dz == 0) continue;
-                        if (!Stencil<Q>::has(dx, dy, dz)) continue;
-                        const float ps = ring[(w + 1 + dy) * kPSX + lane + 1 + dx];
-                        const float wp = weight<Q>(dx, dy, dz) * ps;
-                        if (dx) sx += dx * wp;
-                        if (dy) sy += dy * wp;
-                        if (dz) sz += dz * wp;
-                    }
-                }
-            }
-            Fx = 3.0f * sx;
-            Fy = 3.0f * sy;
-            Fz = 3.0f * sz;
-            const float absF = sqrtf(Fx * Fx + Fy * Fy + Fz * Fz);
-            // Omega2 (collisionOperators.cuh:16-25) folded into the coefficients
-            float Aeff = P.A; // A_calculation (forces.cuh:114-117) at the node's relaxation time
-            if constexpr ((kFB & F_FORCE) != 0)
-                if (P.tau_var) Aeff = P.s4 / tau_eff_of(P, nd.rr, nd.rb);
-            float hA = (P.omega2_conservative && !(absF > 1.0e-4f)) ? 0.0f : 0.5f * Aeff * absF;
-            if (absF > 1.0e-4f) {
-                const float ia_ = fast_rcp(absF);
-                const float qf = 0.5f * Aeff * ia_;
-                // isotropic part from the same q |F|^2 as the anisotropic part, so Omega2 sums
-                // to zero over the directions in floating point too
-                hA = qf * (Fx * Fx + Fy * Fy + Fz * Fz);
-                cf.p200 += qf * Fx * Fx;
-                cf.p020 += qf * Fy * Fy;
-                cf.p002 += qf * Fz * Fz;
-                cf.p110 += 2.0f * qf * Fx * Fy;
-                cf.p101 += 2.0f * qf * Fx * Fz;
-                cf.p011 += 2.0f * qf * Fy * Fz;
-                // recolouring (collisionOperators.cuh:60-80): beta rr rb / (rho^2 |F|) * feq0, where
-                // the rest equilibrium of moving directions is w rho (w (rho + K) with a density ratio)
-                const float rho = nd.rr + nd.rb;
-                const float feq0 = ((kFB & F_FORCE) && P.ratio) ? rho + nd.rr * P.kappa_r + nd.rb * P.kappa_b : rho;
-                const float irho = fast_rcp(rho);
-                dcoef = P.beta * (nd.rr * nd.rb) * irho * irho * ia_ * feq0;
-            }
-            cf.p000 -= hA;
-            omega2_rest = hA; // rest-population part, -hA (B0 - w0) = +2/3 hA, added below in exact units
-        }
-        const float rho_src = active ? nd.rr + nd.rb : 0.0f;
-        const float rr_src = active ? nd.rr : 0.0f;
-        // colour fractions of the x neighbours (lane -1 and lane +1)
-        float2 aRlr;
-        aRlr.x = __shfl_up_sync(kFull, aR, 1);
-        aRlr.y = __shfl_down_sync(kFull, aR, 1);
-
-        // separable inverse transform, x-pass: t_bc(cx) for the monomials cy^b cz^c
-        const Tri t00 = tri(cf.p000 + cf.p200, cf.p100, cf.p000);
-        const Tri t10 = tri(cf.p010 + cf.p210, cf.p110, cf.p010);
-        const Tri t01 = tri(cf.p001 + cf.p201, cf.p101, cf.p001);
-        const Tri t20 = tri(cf.p020, cf.p120, cf.p020);
-        const Tri t02 = tri(cf.p002, cf.p102, cf.p002);
-        const Tri t11 = tri(cf.p011, cf.p111, cf.p011);
-        const float2 rho2 = pair(rho_src);
-        // Populations are carried scaled by S = 216 (D3Q27) or 36 (D3Q19), where the weights
-        // are small integers that sum to S exactly: float-rounded weights do not sum to 1, and
-        // that error would scale every node's mass each step (about 1.5e-8 per step for D3Q19).
-        // D3Q27 weights are also separable, S w(c) = prod over axes of (4 if c_a = 0 else 1):
-        // populations are carried unweighted and the factors 4 are applied inside the forward
-        // passes.  D3Q19 weights 12, 2, 1 are applied per population.  Each destination
-        // divides its sums by S once, the mass sums with a correctly rounded quotient.
-        constexpr bool kSepW = (Q == 27);
-        const float dk1 = kSepW ? dcoef : 2.0f * dcoef;
-        const float dk2 = dcoef * 0.7071067811865475f;
-        const float dk3 = kSepW ? dcoef * 0.5773502691896258f : 0.0f;
-        // rest-population correction (density-ratio K and the Omega2 rest term), with the Omega2
-        // part in exact units so that Omega2 sums to zero over the directions (B0 - w0 = -2/3
-        // for both lattices)
-        // in value units before the rest weight (64 of 216, or 12 of 36): S r0 / W_0 and
-        // S (w0 - B0) hA / W_0 = (2/3) S hA / W_0, i.e. 3.375 r0 + 2.25 hA or 3 r0 + 2 hA
-        const float rc0 = kSepW ? fmaf(cf.r0, 3.375f, 2.25f * omega2_rest) : fmaf(cf.r0, 3.0f, 2.0f * omega2_rest);
-
-        // wall bounce-back of this node's own populations (destination = this node, plane k)
-        const bool wx0 = P.bc[0] == MBCG_BC_WALL && xs == 1, wx1 = P.bc[0] == MBCG_BC_WALL && xs == nx - 2;
-        const bool wy0 = P.bc[1] == MBCG_BC_WALL && ys == 1, wy1 = P.bc[1] == MBCG_BC_WALL && ys == ny - 2;
-        const bool wz0 = P.bc[2] == MBCG_BC_WALL && k == 1, wz1 = P.bc[2] == MBCG_BC_WALL && k == nz - 2;
-        const bool reflect = (kFB & F_WALL) && role == R_FLUID && dest_thread && (wx0 | wx1 | wy0 | wy1 | wz0 | wz1);
-        const bool any_reflect = (kFB & F_WALL) ? __any_sync(kFull, reflect) : false;
-
-        // ---- emit: populations of the rows this warp exports, x streaming, own-row moments,
-        // y exchange.  Halo rows export one population row (cy = +1 for warp 0, -1 for warp W-1).
-        auto emit = [&](auto rowsc) {
-            constexpr int ROWS = decltype(rowsc)::value;
-            // y-pass per exported row j (cy = j - 1): s0 (cz^0), s1 (cz^1), e2 (cz^0 + cz^2)
-            Tri s0[3], s1[3], e2[3];
-            {
-                const Tri e0 = t00 + t20;
-                const Tri e1 = t01 + cf.p021;
-                if (ROWS & 2) {
-                    s0[1] = t00;
-                    s1[1] = t01;
-                    e2[1] = t00 + t02;
-                }
-                if (ROWS & 4) {
-                    s0[2] = e0 + t10;
-                    s1[2] = e1 + t11;
-                    e2[2] = s0[2] + (t02 + cf.p012);
-                }
-                if (ROWS & 1) {
-                    s0[0] = e0 - t10;
-                    s1[0] = e1 - t11;
-                    e2[0] = s0[0] + (t02 + (-cf.p012));
-                }
-            }
-            auto do_class = [&](auto czc, Acc& acc) {
-                constexpr int cz = decltype(czc)::value;
-                // populations of row j: rho + the small part (rho last, see above); sm keeps the
-                // small parts (value units, before the D3Q19 weight) for the red populations
-                Tri g[3], sm[3];
-#pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    const int cy = j - 1;
-                    g[j].o = sm[j].o = make_float2(0.0f, 0.0f);
-                    g[j].c = sm[j].c = 0.0f;
-                    if (!(ROWS & (1 << j))) continue;
-                    Tri small = cz == 0 ? s0[j] : (cz > 0 ? e2[j] + s1[j] : e2[j] - s1[j]);
-                    if (cy == 0 && cz == 0) small.c += rc0;
-                    const int shc = cy * cy + cz * cz; // |c|^2 of the centre; the outer ones have shc + 1
-                    if (Stencil<Q>::has(1, cy, cz)) {
-                        sm[j].o = small.o;
-                        const float2 vv = __fadd2_rn(rho2, small.o);
-                        g[j].o = (kSepW || shc != 0) ? vv : __fadd2_rn(vv, vv);
-                    }
-                    if (Stencil<Q>::has(0, cy, cz)) {
-                        sm[j].c = small.c;
-                        const float vv = rho_src + small.c;
-                        g[j].c = kSepW ? vv : (shc == 0 ? 12.0f * vv : (shc == 1 ? vv + vv : vv));
-                    }
-                }
-                // recolouring part Delta_i of the red populations (interface sources only; the
-                // red population is aR g_i + Delta_i, collisionOperators.cuh:60-80)
-                auto delta = [&](int i, int j) -> float {
-                    const int cx = i - 1, cy = j - 1, sh = cx * cx + cy * cy + cz * cz;
-                    if (!(ROWS & (1 << j)) || !Stencil<Q>::has(cx, cy, cz) || sh == 0) return 0.0f;
-                    const float dks = sh == 1 ? dk1 : (sh == 2 ? dk2 : dk3);
-                    const float fc = (cx ? cx * Fx : 0.0f) + (cy ? cy * Fy : 0.0f) + (cz ? cz * Fz : 0.0f);
-                    return dks * fc;
-                };
-                // Red population of direction (cx, cy, cz) = (i - 1, j - 1, cz) of a source with
-                // density rho, red density rr, colour fraction aR = rr / rho, population
-                // g = W (rho + sm) and recolouring part Delta.  On interface warps it is formed
-                // as W (rr + aR sm) + Delta, which is aR g + Delta in exact arithmetic, but the
-                // red populations of a source then sum to S rr + aR sum(W sm) (sm sums to zero)
-                // whatever the rounding of aR, where aR g emits S aR rho: in a near-steady state
-                // the quotient's rounding error repeats step after step and its sum over the
-                // interface moved the 64^3 D3Q19 bubble's red mass by 7e-6 in 10^4 steps
-                // (3.5e-7 with this form).  Elsewhere aR is within 2.5e-5 of 0 or 1 and the
-                // populations are aR g.
-                auto red_pop = [&](float rr_, float smv, float gv, float dl, int i, int j, bool withd) -> float {
-                    if (!withd) return aR * gv;
-                    const int cy = j - 1, shc = cy * cy + cz * cz + (i != 1 ? 1 : 0);
-                    const float b = fmaf(aR, smv, rr_);
-                    // D3Q19 weight of the population: 12 (rest), 2 (|c|^2 = 1), 1 (|c|^2 = 2)
-                    if (kSepW || shc == 2) return b + dl;
-                    if (shc == 1) return fmaf(2.0f, b, dl);
-                    return fmaf(12.0f, b, dl);
-                };
-                if constexpr (ROWS == 7 && (kFB & F_WALL) != 0) {
-                    if (any_reflect && reflect) {
-#pragma unroll
-                        for (int i = 0; i < 3; ++i)
-#pragma unroll
-                            for (int j = 0; j < 3; ++j) {
-                                const int cx = i - 1, cy = j - 1;
-                                if (!Stencil<Q>::has(cx, cy, cz)) continue;
-                                const bool into = (wx0 && cx < 0) || (wx1 && cx > 0) || (wy0 && cy < 0) ||
-                                                  (wy1 && cy > 0) || (wz0 && cz < 0) || (wz1 && cz > 0);
-                                if (!into) continue;
-                                const float f = kSepW ? static_cast<float>((cx == 0 ? 4 : 1) * (cy == 0 ? 4 : 1) *
-                                                                           (cz == 0 ? 4 : 1))
-                                                      : 1.0f;
-                                const float gv = i == 0 ? g[j].o.x : (i == 2 ? g[j].o.y : g[j].c);
-                                const float smv = i == 0 ? sm[j].o.x : (i == 2 ? sm[j].o.y : sm[j].c);
-                                const float rr_ = red_pop(rr_src, smv, gv, any_iface ? delta(i, j) : 0.0f, i, j, any_iface);
-                                add_pop(accC, f * gv, f * rr_, -cx, -cy, -cz);
-                            }
-                    }
-                }
-                // x streaming: destination x receives cx=+1 from lane-1 and cx=-1 from lane+1.
-                // The populations cross lanes; on interface warps the source forms its red
-                // populations (red_pop) and they cross too, elsewhere the destination forms them
-                // as aR g from the source's colour fraction (shuffled once per plane).
-                float X0[3], X1[3], X2[3], XR[3];
-                auto xstream = [&](auto ifc) {
-                    constexpr bool kIf = decltype(ifc)::value;
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) {
-                        const int cy = j - 1;
-                        X0[j] = X1[j] = X2[j] = XR[j] = 0.0f;
-                        if (!(ROWS & (1 << j))) continue;
-                        const float r1 = red_pop(rr_src, sm[j].c, g[j].c, kIf ? delta(1, j) : 0.0f, 1, j, kIf);
-                        if (Stencil<Q>::has(1, cy, cz)) {
-                            float2 glr; // (from lane - 1, from lane + 1)
-                            glr.x = __shfl_up_sync(kFull, g[j].o.y, 1);
-                            glr.y = __shfl_down_sync(kFull, g[j].o.x, 1);
-                            X2[j] = glr.x + glr.y;
-                            X0[j] = kSepW ? fmaf(4.0f, g[j].c, X2[j]) : X2[j] + g[j].c;
-                            X1[j] = glr.x - glr.y;
-                            float2 rlr;
-                            if constexpr (kIf) {
-                                // red_pop of this lane's cx = -1 / +1 populations, paired
-                                const bool w2 = !kSepW && cy == 0 && cz == 0; // D3Q19 weight 2
-                                float2 ro = __ffma2_rn(pair(aR), sm[j].o, pair(rr_src));
-                                const float2 dl = make_float2(delta(0, j), delta(2, j));
-                                ro = w2 ? __ffma2_rn(pair(2.0f), ro, dl) : __fadd2_rn(ro, dl);
-                                rlr.x = __shfl_up_sync(kFull, ro.y, 1);
-                                rlr.y = __shfl_down_sync(kFull, ro.x, 1);
-                            } else {
-                                rlr = __fmul2_rn(aRlr, glr);
-                            }
-                            XR[j] = kSepW ? fmaf(4.0f, r1, rlr.x + rlr.y) : (rlr.x + rlr.y) + r1;
-                        } else {
-                            X0[j] = g[j].c;
-                            XR[j] = r1;
-                        }
-                    }
-                };
-                if (any_iface) xstream(std::true_type{});
-                else xstream(std::false_type{});
-                if constexpr ((ROWS & 2) != 0) {
-                    // cy = 0 row stays in this column: add to the destination's sums now.  Plane
-                    // k+1 (cz = +1) receives its first contributions here: they are assigned, so
-                    // its sums need no clearing.
-                    constexpr int fi = kSepW ? (cz == 0 ? 16 : 4) : 1;
-                    constexpr float f = static_cast<float>(fi);
-                    if constexpr (cz == 1) {
-                        acc.rr = fi == 1 ? make_float2(X0[1], XR[1]) : __fmul2_rn(pair(f), make_float2(X0[1], XR[1]));
-                        acc.jxx = fi == 1 ? make_float2(X1[1], X2[1]) : __fmul2_rn(pair(f), make_float2(X1[1], X2[1]));
-                        acc.jz = f * X0[1];
-                        acc.xz = f * X1[1];
-                        acc.zz = f * X0[1];
+                    const float* ring = dz < 0 ? rm : (dz == 0 ? r0p : rp);
+                    const float* pa = ring + (wa + 1 + dy) * kPSX + lane + 1;
+                    const float* pb = ring + (wb + 1 - dy) * kPSX + lane + 1;
+                    const int n = dy * dy + dz * dz;
+                    F2& r = R[dy + 1][dz + 1];
+                    F2& d = D[dy + 1][dz + 1];
+                    if (Q == 27 || n < 2) {
+                        const F2 l = make_float2(pa[-1], pb[-1]), h = make_float2(pa[1], pb[1]);
+                        d = h - l;
+                        if (n != 0) r = fma2(Q == 27 ? 4.0f : 2.0f, make_float2(pa[0], pb[0]), h + l);
                     } else {
-                        acc.rr = acc2<fi>(acc.rr, make_float2(X0[1], XR[1]));
-                        acc.jxx = acc2<fi>(acc.jxx, make_float2(X1[1], X2[1]));
-                        if (cz != 0) {
-                            acc.jz = fmaf(cz * f, X0[1], acc.jz);
-                            acc.xz = fmaf(cz * f, X1[1], acc.xz);
-                            acc.zz = fmaf(f, X0[1], acc.zz);
-                        }
+                        r = make_float2(pa[0], pb[0]);
                     }
                 }
-                // cy = +1 goes to row w+1 (slot 0), cy = -1 to row w-1 (slot 1)
-                constexpr int cls = cz + 1;
-                if constexpr ((ROWS & 4) != 0) {
-                    xb_self[(cls * 2 + 0) * (W * 32)] = make_float4(X0[2], XR[2], X1[2], X2[2]);
-                }
-                if constexpr ((ROWS & 1) != 0) {
-                    xb_self[(cls * 2 + 1) * (W * 32)] = make_float4(X0[0], XR[0], X1[0], X2[0]);
+            F2 Fx, Fy, Fz;
+            const F2 de = (D[0][1] + D[2][1]) + (D[1][0] + D[1][2]);
+            const F2 ry = R[2][1] - R[0][1], rz_ = R[1][2] - R[1][0];
+            const F2 py = R[2][2] - R[0][0], pz = R[2][0] - R[0][2];
+            if constexpr (Q == 27) {
+                const F2 dc = (D[0][0] + D[2][2]) + (D[0][2] + D[2][0]);
+                constexpr float s = 3.0f / 216.0f;
+                Fx = s * fma2(16.0f, D[1][1], fma2(4.0f, de, dc));
+                Fy = s * fma2(4.0f, ry, py + pz);
+                Fz = s * fma2(4.0f, rz_, py - pz);
+            } else {
+                constexpr float s = 3.0f / 36.0f;
+                Fx = s * fma2(2.0f, D[1][1], de);
+                Fy = s * (ry + (py + pz));
+                Fz = s * (rz_ + (py - pz));
+            }
+            if (!if_a) Fx.x = Fy.x = Fz.x = 0.0f;
+            if (!if_b) Fx.y = Fy.y = Fz.y = 0.0f;
+            const F2 F2s = fma2(Fz, Fz, fma2(Fy, Fy, Fx * Fx));
+            F2 qf = pair(0.0f), hA = pair(0.0f), dco = pair(0.0f);
+            const F2 mix = P.beta * (nd.rr * nd.rb) * inv * inv;
+            auto amp = [&](float f2, float rr, float rb, float rho_, float mx, float& q, float& h, float& dc) {
+                const float absF = sqrtf(f2);
+                float Aeff = P.A; // A_calculation (forces.cuh:114-117) at the node's relaxation time
+                if constexpr ((kFeat & F_FORCE) != 0)
+                    if (P.tau_var) Aeff = P.s4 / tau_eff_of(P, rr, rb);
+                // Omega2 (collisionOperators.cuh:16-25); below the cut-off only its isotropic part
+                h = P.omega2_conservative ? 0.0f : 0.5f * Aeff * absF;
+                if (absF > 1.0e-4f) {
+                    const float ia_ = fast_rcp(absF);
+                    q = 0.5f * Aeff * ia_;
+                    h = q * f2; // so Omega2 sums to zero over the directions in floating point too
+                    // recolouring: beta rr rb / (rho^2 |F|) * feq0, where the rest equilibrium of moving
+                    // directions is w rho (w (rho + K) with a density ratio)
+                    const float feq0 = ((kFeat & F_FORCE) && P.ratio) ? rho_ + rr * P.kappa_r + rb * P.kappa_b : rho_;
+                    dc = mx * ia_ * feq0;
                 }
             };
-            do_class(std::integral_constant<int, -1>{}, accP);
-            do_class(std::integral_constant<int, 0>{}, accC);
-            do_class(std::integral_constant<int, 1>{}, accN);
+            if (if_a) amp(F2s.x, nd.rr.x, nd.rb.x, rho.x, mix.x, qf.x, hA.x, dco.x);
+            if (if_b) amp(F2s.y, nd.rr.y, nd.rb.y, rho.y, mix.y, qf.y, hA.y, dco.y);
+            const F2 qx = (2.0f / 3.0f) * qf * Fx, qy = (2.0f / 3.0f) * qf * Fy, qz = (2.0f / 3.0f) * qf * Fz;
+            const F2 oxx = qx * Fx, oyy = qy * Fy, ozz = qz * Fz;
+            cf.exx = cf.exx + oxx;
+            cf.eyy = cf.eyy + oyy;
+            cf.ezz = cf.ezz + ozz;
+            cf.exy = fma2(qx, Fy, cf.exy);
+            cf.exz = fma2(qx, Fz, cf.exz);
+            cf.eyz = fma2(qy, Fz, cf.eyz);
+            cf.p000 = cf.p000 - hA;
+            // rest part -hA (B0 - w0) = +2/3 hA, in value units of the rest weight
+            rc0 = fma2(kSepW ? 2.25f : 2.0f, hA, rc0);
+            dFx = dco * Fx;
+            dFy = dco * Fy;
+            dFz = dco * Fz;
+        }
+
+        // wall bounce-back of this thread's own populations (destination = source, plane k)
+        if constexpr ((kFeat & F_WALL) != 0) {
+            auto reflect = [&](int half, int role, bool dest, int ysh) {
+                const bool wx0 = P.bc[0] == MBCG_BC_WALL && xs == 1, wx1 = P.bc[0] == MBCG_BC_WALL && xs == nx - 2;
+                const bool wy0 = P.bc[1] == MBCG_BC_WALL && ysh == 1, wy1 = P.bc[1] == MBCG_BC_WALL && ysh == ny - 2;
+                const bool wz0 = P.bc[2] == MBCG_BC_WALL && k == 1, wz1 = P.bc[2] == MBCG_BC_WALL && k == nz - 2;
+                if (!(role == R_FLUID && dest && (wx0 | wx1 | wy0 | wy1 | wz0 | wz1))) return;
+                auto h = [&](F2 v) { return half ? v.y : v.x; };
+                const float mir = half ? -1.0f : 1.0f; // y of the mirrored frame
+                float sums[12];
+#pragma unroll
+                for (int i = 0; i < 12; ++i) sums[i] = 0.0f;
+                for (int i = 0; i < 27; ++i) {
+                    const int cxi = i % 3 - 1, cyi = (i / 3) % 3 - 1, czi = i / 9 - 1;
+                    const int n = cxi * cxi + cyi * cyi + czi * czi;
+                    if (n == 0 || (Q == 19 && n == 3)) continue;
+                    const bool into = (wx0 && cxi < 0) || (wx1 && cxi > 0) || (wy0 && cyi < 0) || (wy1 && cyi > 0) ||
+                                      (wz0 && czi < 0) || (wz1 && czi > 0);
+                    if (!into) continue;
+                    const float cx = static_cast<float>(cxi), cy = mir * static_cast<float>(cyi), cz = static_cast<float>(czi);
+                    const float wt = kSepW ? (n == 1 ? 16.0f : (n == 2 ? 4.0f : 1.0f)) : (n == 1 ? 2.0f : 1.0f);
+                    float sm = h(cf.p000) + cx * h(cf.p100) + cy * h(cf.p010) + cz * h(cf.p001);
+                    sm += 1.5f * (cx * cx * h(cf.exx) + cy * cy * h(cf.eyy) + cz * cz * h(cf.ezz));
+                    sm += 3.0f * (cx * cy * h(cf.exy) + cx * cz * h(cf.exz) + cy * cz * h(cf.eyz));
+                    sm += 4.5f * (cx * cx * (cy * h(cf.kxxy) + cz * h(cf.kxxz)) + cy * cy * (cx * h(cf.kxyy) + cz * h(cf.kyyz)) +
+                                  cz * cz * (cx * h(cf.kxzz) + cy * h(cf.kyzz)));
+                    sm += 9.0f * (cx * cy * cz * h(cf.kxyz));
+                    const float g = wt * (h(rhod) + sm);
+                    const float dn = n == 1 ? 1.0f : (n == 2 ? 0.7071067811865475f : 0.5773502691896258f);
+                    const float dl = wt * dn * (cx * h(dFx) + cy * h(dFy) + cz * h(dFz));
+                    // it returns with the opposite velocity
+                    sums[0] += g;
+                    sums[1] += fmaf(wt, fmaf(h(aR), sm, h(rl)), dl);
+                    sums[2] += wt * h(ec);
+                    sums[3] -= cx * g;
+                    sums[4] -= cy * g;
+                    sums[5] -= cz * g;
+                    sums[6] += cx * cx * g;
+                    sums[7] += cx * cy * g;
+                    sums[8] += cy * cy * g;
+                    sums[9] += cy * cz * g;
+                    sums[10] += cz * cz * g;
+                    sums[11] += cx * cz * g;
+                }
+                F2* a[12] = {&accC.tot, &accC.red, &accC.E, &accC.jx, &accC.jy, &accC.jz,
+                             &accC.xx, &accC.xy, &accC.yy, &accC.yz, &accC.zz, &accC.xz};
+#pragma unroll
+                for (int i = 0; i < 12; ++i) {
+                    if (half) a[i]->y += sums[i];
+                    else a[i]->x += sums[i];
+                }
+            };
+            reflect(0, role_a, dest_a, ysa);
+            reflect(1, role_b, dest_b, ysb);
+        }
+
+        // ---- x streaming.  For each power (b, c) of (cy, cz) the source evaluates its polynomial at
+        // cx = -1, 0, +1; the outer two cross to the neighbouring lanes and the destination column
+        // forms the moments of order 0, 1, 2 in x (and the red sum) of that coefficient.
+        const F2 aRl = shfl_up2(aR), aRr = shfl_down2(aR);
+        const F2 s00 = fma2(1.5f, cf.exx, cf.p000);
+        // P: sum over cx = +-1, D: difference; X and rP: order 0 (weights 4 and 1) of the total and of
+        // red for D3Q27; for D3Q19 X = cx = 0 alone and rP, rC red like P and X.
+        struct XM {
+            F2 P, D, X, rP, rC;
         };
-        if (w == 0) emit(std::integral_constant<int, 4>{});
-        else if (w == W - 1) emit(std::integral_constant<int, 1>{});
-        else emit(std::integral_constant<int, 7>{});
+        const F2 aR4 = 4.0f * aR;
+        auto moments_x = [&](F2 l, F2 r, F2 centre) -> XM {
+            XM m;
+            m.P = l + r;
+            m.D = l - r;
+            m.X = kSepW ? fma2(4.0f, centre, m.P) : centre;
+            return m;
+        };
+        auto stream_x = [&](F2 plus, F2 centre, F2 minus) -> XM {
+            const F2 l = shfl_up2(plus), r = shfl_down2(minus);
+            XM m = moments_x(l, r, centre);
+            m.rP = fma2(aRr, r, aRl * l);
+            if constexpr (kSepW) m.rP = fma2(aR4, centre, m.rP);
+            else m.rC = aR * centre;
+            return m;
+        };
+        XM m00;
+        {
+            const F2 sp = s00 + cf.p100, sm = s00 - cf.p100;
+            const F2 l = shfl_up2(rhod + sp), r = shfl_down2(rhod + sm);
+            m00 = moments_x(l, r, rhod + cf.p000);
+            const F2 lr = shfl_up2(fma2(aR, sp, rl)), rr = shfl_down2(fma2(aR, sm, rl));
+            const F2 cr = fma2(aR, cf.p000, rl);
+            m00.rP = lr + rr;
+            if constexpr (kSepW) m00.rP = fma2(4.0f, cr, m00.rP);
+            else m00.rC = cr;
+        }
+        const F2 b10 = fma2(4.5f, cf.kxxy, cf.p010), b01 = fma2(4.5f, cf.kxxz, cf.p001);
+        XM m10 = stream_x(fma2(3.0f, cf.exy, b10), cf.p010, fma2(-3.0f, cf.exy, b10));
+        XM m01 = stream_x(fma2(3.0f, cf.exz, b01), cf.p001, fma2(-3.0f, cf.exz, b01));
+        // the remaining ones without their factors 3/2, 3/2, 3, 9/2, 9/2
+        XM m20 = stream_x(fma2(3.0f, cf.kxyy, cf.eyy), cf.eyy, fma2(-3.0f, cf.kxyy, cf.eyy));
+        XM m02 = stream_x(fma2(3.0f, cf.kxzz, cf.ezz), cf.ezz, fma2(-3.0f, cf.kxzz, cf.ezz));
+        XM m11 = stream_x(fma2(3.0f, cf.kxyz, cf.eyz), cf.eyz, fma2(-3.0f, cf.kxyz, cf.eyz));
+        XM m21 = stream_x(cf.kyyz, cf.kyyz, cf.kyyz);
+        XM m12 = stream_x(cf.kyzz, cf.kyzz, cf.kyzz);
+        const F2 eS = grid(aRl) + grid(aRr);
+        F2 red22 = pair(0.0f); // red sum of cy^2 cz^2, without the factor 3/2
+        if (any_iface) {
+            // Delta is odd in c: as a polynomial in (cy, cz) its coefficients at cx = +-1 and 0 are
+            // multiples of dF with d(1) = d, d(2) = d / sqrt 2, d(3) = d / sqrt 3
+            constexpr float i2 = 0.7071067811865475f;
+            [[maybe_unused]] constexpr float i3 = 0.5773502691896258f;
+            const F2 gx = shfl_up2(dFx) - shfl_down2(dFx);
+            const F2 gy = shfl_up2(dFy) + shfl_down2(dFy);
+            const F2 gz = shfl_up2(dFz) + shfl_down2(dFz);
+            m00.rP = m00.rP + gx;
+            m10.rP = fma2(i2, gy, m10.rP);
+            m01.rP = fma2(i2, gz, m01.rP);
+            m20.rP = fma2((i2 - 1.0f) / 1.5f, gx, m20.rP);
+            m02.rP = fma2((i2 - 1.0f) / 1.5f, gx, m02.rP);
+            if constexpr (kSepW) {
+                m10.rP = fma2(4.0f, dFy, m10.rP);
+                m01.rP = fma2(4.0f, dFz, m01.rP);
+                m12.rP = fma2(4.0f * (i2 - 1.0f) / 4.5f, dFy, m12.rP);
+                m21.rP = fma2(4.0f * (i2 - 1.0f) / 4.5f, dFz, m21.rP);
+                m12.rP = fma2((i3 - i2) / 4.5f, gy, m12.rP);
+                m21.rP = fma2((i3 - i2) / 4.5f, gz, m21.rP);
+                red22 = ((i3 - 2.0f * i2 + 1.0f) / 1.5f) * gx;
+            } else {
+                m10.rC = m10.rC + dFy;
+                m01.rC = m01.rC + dFz;
+                m12.rC = fma2((i2 - 1.0f) / 4.5f, dFy, m12.rC);
+                m21.rC = fma2((i2 - 1.0f) / 4.5f, dFz, m21.rC);
+            }
+        }
+
+        // ---- y streaming.  What leaves a row for the next row inwards (cy' = +1 of the mirrored
+        // frame) and outwards (cy' = -1) goes through shared memory; the row's own part waits in
+        // registers.  Weights: D3Q27 216 w = product over the axes of (4 if c_a = 0 else 1), the 4s
+        // applied when an axis is summed; D3Q19 36 w = 12, 2, 1 by |c|^2.
+        // The innermost pair is its own outer neighbour with the halves exchanged: it also writes its
+        // inward values, swapped, to the outward slot after the last warp's.
+        constexpr int kX = (H + 1) * 32; // one quantity's slots
+        float2* xw = xbuf + w * 32 + lane;
+        const bool innermost = w == H - 1;
+        constexpr int kDir = kSepW ? 12 : 8; // quantities each way
+        auto put = [&](int q, F2 in, F2 out) {
+            xw[q * kX] = in;
+            xw[(kDir + q) * kX] = out;
+            if (innermost) xw[(kDir + q) * kX + 32] = swap2(in);
+        };
+        auto put_both = [&](int q, F2 v) {
+            xw[q * kX] = v;
+            if (innermost) xw[q * kX + 32] = swap2(v);
+        };
+        // own part of the destination sums: [channel][power of cz] (D3Q27), or by class (D3Q19)
+        F2 own[4][3], ownE0;
+        if constexpr (kSepW) {
+            auto rows = [&](int ch, F2 a00, F2 a10, F2 a01, F2 a20, F2 a02, F2 a11, F2 a21, F2 a12) {
+                const F2 e0 = fma2(1.5f, a20, a00), e1 = fma2(4.5f, a21, a01);
+                put(3 * ch, e0 + a10, e0 - a10);
+                put(3 * ch + 1, fma2(3.0f, a11, e1), fma2(-3.0f, a11, e1));
+                put(3 * ch + 2, fma2(3.0f, a12, a02), fma2(-3.0f, a12, a02));
+                own[ch][0] = a00;
+                own[ch][1] = a01;
+                own[ch][2] = a02;
+            };
+            rows(0, m00.X, m10.X, m01.X, m20.X, m02.X, m11.X, m21.X, m12.X);
+            rows(1, m00.D, m10.D, m01.D, m20.D, m02.D, m11.D, m21.D, m12.D);
+            rows(2, m00.P, m10.P, m01.P, m20.P, m02.P, m11.P, m21.P, m12.P);
+            rows(3, m00.rP, m10.rP, m01.rP, m20.rP, m02.rP + red22, m11.rP, m21.rP, m12.rP);
+            own[3][2] = m02.rP;
+            ownE0 = fma2(4.0f, ec, eS);
+            put_both(24, ownE0);
+        } else {
+            // channels 0 (order 0), 1 (D), 2 (P), 3 (red); cz = 0 rows have |c|^2 - cx^2 = 1 beside,
+            // cz = +-1 rows beside this one only the centre (C)
+            auto axis = [&](int ch, F2 a00, F2 a10, F2 a20) { // cz = 0
+                const F2 e0 = fma2(1.5f, a20, a00);
+                put(ch, e0 + a10, e0 - a10);
+            };
+            auto corner = [&](int q, F2 c00, F2 c10, F2 c01, F2 c20, F2 c02, F2 c11, F2 c21, F2 c12) { // cz = +1, -1
+                const F2 e0 = fma2(1.5f, c02, fma2(1.5f, c20, c00));
+                const F2 oy = fma2(4.5f, c12, c10), oz = fma2(4.5f, c21, c01);
+                const F2 a = e0 + oy, b = fma2(3.0f, c11, oz), a2 = e0 - oy, b2 = fma2(-3.0f, c11, oz);
+                put(q, a + b, a2 + b2);
+                put(q + 1, a - b, a2 - b2);
+            };
+            auto a1 = [&](const XM& m) { return fma2(2.0f, m.X, m.P); };
+            auto r1 = [&](const XM& m) { return fma2(2.0f, m.rC, m.rP); };
+            auto a0 = [&](const XM& m) { return fma2(12.0f, m.X, 2.0f * m.P); };
+            auto r0 = [&](const XM& m) { return fma2(12.0f, m.rC, 2.0f * m.rP); };
+            axis(0, a1(m00), a1(m10), a1(m20));
+            axis(1, m00.D, m10.D, m20.D);
+            axis(2, m00.P, m10.P, m20.P);
+            axis(3, r1(m00), r1(m10), r1(m20));
+            corner(4, m00.X, m10.X, m01.X, m20.X, m02.X, m11.X, m21.X, m12.X);
+            corner(6, m00.rC, m10.rC, m01.rC, m20.rC, m02.rC, m11.rC, m21.rC, m12.rC);
+            // own row: cz = 0 (weights 12, 2), then cz = +1 and -1 (weights 2, 1)
+            auto zrow = [&](int ch, F2 b00, F2 b01, F2 b02) {
+                const F2 e0 = fma2(1.5f, b02, b00);
+                own[ch][1] = e0 + b01;
+                own[ch][2] = e0 - b01;
+            };
+            own[0][0] = a0(m00);
+            own[1][0] = 2.0f * m00.D;
+            own[2][0] = 2.0f * m00.P;
+            own[3][0] = r0(m00);
+            zrow(0, a1(m00), a1(m01), a1(m02));
+            zrow(1, m00.D, m01.D, m02.D);
+            zrow(2, m00.P, m01.P, m02.P);
+            zrow(3, r1(m00), r1(m01), r1(m02));
+            ownE0 = fma2(2.0f, ec, eS); // |c|^2 - cx^2 = 1; the row itself is 2 eS + 12 e
+            put_both(16, ownE0);
+            put_both(17, ec);
+        }
         __syncthreads();
 
-        // (4) y streaming into destination rows
-        auto gather = [&](auto czc, Acc& acc) {
-            constexpr int cz = decltype(czc)::value;
-            constexpr int cls = cz + 1;
-            constexpr int fi = (kSepW && cz == 0) ? 4 : 1;
-            constexpr float f = static_cast<float>(fi);
-            const float4 pv = xb_self[(cls * 2 + 0) * (W * 32) - 32]; // row w-1 exported cy = +1
-            const float4 mv = xb_self[(cls * 2 + 1) * (W * 32) + 32]; // row w+1 exported cy = -1
-            // slots (X0, XR, X1, X2)
-            const float2 s0r = __fadd2_rn(make_float2(pv.x, pv.y), make_float2(mv.x, mv.y)); // (s00, red)
-            const float2 s12 = __fadd2_rn(make_float2(pv.z, pv.w), make_float2(mv.z, mv.w)); // (s10, s20)
-            const float d00 = pv.x - mv.x;
-            acc.rr = acc2<fi>(acc.rr, s0r);
-            acc.jxx = acc2<fi>(acc.jxx, s12);
-            if constexpr (cz == 1) {
-                // first contributions to jy, xy, yy, yz of plane k+1 (f = 1)
-                acc.jy = d00;
-                acc.xy = pv.z - mv.z;
-                acc.yy = s0r.x;
-                acc.yz = d00;
-            } else {
-                acc.jy = fmaf(f, d00, acc.jy);
-                acc.xy = fmaf(f, pv.z - mv.z, acc.xy);
-                acc.yy = fmaf(f, s0r.x, acc.yy);
-                if (cz != 0) acc.yz += cz * d00;
-            }
-            if (cz != 0) {
-                acc.jz += cz * s0r.x;
-                acc.xz += cz * s12.x;
-                acc.zz += s0r.x;
-            }
-        };
-        const bool dest_row = (w >= 1 && w <= W - 2);
-        if (dest_row) gather(std::integral_constant<int, -1>{}, accP);
-
-        // (5) destination plane k-1 is complete: moments (lbm.cuh:239-261), store, boundary
+        // (4) y sums, z streaming; warp 0 holds the two halo rows and receives nothing: it refills the
+        // slot of plane k (whose fields everyone has read) and prepares the psi frame of plane k+2
         const int d = k - 1;
-        if (dest_thread && d >= zd0 && d < zd1) {
-            {
+        if (w == 0) {
+            if constexpr (kTMA)
+                if (k + kNSTAGE <= zd1 + 1) issue(k + kNSTAGE, sl);
+            const int sl2 = nxt(sl_next);
+            if (k + 2 <= zd1 + 1 && peek_slot(sl2)) fill_frame(mz2, inbox2, sl2);
+        } else {
+            // [moment][cz = -1, 0, +1], moments tot, jx, jy, xx, xy, yy, red
+            F2 Z0[7], Zp[7], Zm[7], Ep, E0;
+            auto in_ = [&](int q) { return xw[q * kX - 32]; };
+            auto ou_ = [&](int q) { return xw[(kDir + q) * kX + 32]; };
+            auto both = [&](int q) { return xw[q * kX - 32] + xw[q * kX + 32]; };
+            if constexpr (kSepW) {
+                // powers of cz -> cz = -1, 0, +1; the last coefficient carries the factor 3/2
+                auto zexp = [&](int i, const F2 (&c)[3]) {
+                    const F2 e = fma2(1.5f, c[2], c[0]);
+                    Zp[i] = e + c[1];
+                    Zm[i] = e - c[1];
+                    Z0[i] = c[0];
+                };
+                F2 y0[3], y1[3], y2[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const F2 i = in_(c), o = ou_(c);
+                    y2[c] = i + o;
+                    y1[c] = i - o;
+                    y0[c] = fma2(4.0f, own[0][c], y2[c]);
+                }
+                zexp(0, y0);
+                zexp(2, y1);
+                zexp(5, y2);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const F2 i = in_(3 + c), o = ou_(3 + c);
+                    y1[c] = i - o;
+                    y0[c] = fma2(4.0f, own[1][c], i + o);
+                }
+                zexp(1, y0);
+                zexp(4, y1);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    y0[c] = fma2(4.0f, own[2][c], in_(6 + c) + ou_(6 + c));
+                    y1[c] = fma2(4.0f, own[3][c], in_(9 + c) + ou_(9 + c));
+                }
+                zexp(3, y0);
+                zexp(6, y1);
+                Ep = fma2(4.0f, ownE0, both(24));
+                E0 = Ep;
+            } else {
+                // cz = 0: quantities 0 order 0, 1 D, 2 P, 3 red
+                {
+                    const F2 i = in_(0), o = ou_(0), s0 = i + o;
+                    Z0[0] = s0 + own[0][0];
+                    Z0[2] = i - o;
+                    Z0[5] = s0;
+                }
+                {
+                    const F2 i = in_(1), o = ou_(1);
+                    Z0[1] = (i + o) + own[1][0];
+                    Z0[4] = i - o;
+                }
+                Z0[3] = (in_(2) + ou_(2)) + own[2][0];
+                Z0[6] = (in_(3) + ou_(3)) + own[3][0];
+                // cz = +1 (quantities 4, 6) and -1 (5, 7): the neighbours send their centres
+                {
+                    const F2 i = in_(4), o = ou_(4), sp = i + o;
+                    Zp[0] = sp + own[0][1];
+                    Zp[2] = i - o;
+                    Zp[5] = sp;
+                }
+                {
+                    const F2 i = in_(5), o = ou_(5), sm = i + o;
+                    Zm[0] = sm + own[0][2];
+                    Zm[2] = i - o;
+                    Zm[5] = sm;
+                }
+                Zp[1] = own[1][1];
+                Zm[1] = own[1][2];
+                Zp[4] = Zm[4] = pair(0.0f);
+                Zp[3] = own[2][1];
+                Zm[3] = own[2][2];
+                Zp[6] = (in_(6) + ou_(6)) + own[3][1];
+                Zm[6] = (in_(7) + ou_(7)) + own[3][2];
+                E0 = both(16) + fma2(12.0f, ec, 2.0f * eS);
+                Ep = both(17) + ownE0;
+            }
+            // destination plane k-1 receives cz = -1, plane k cz = 0, plane k+1 cz = +1
+            accP.tot = accP.tot + Zm[0];
+            accP.zz = accP.zz + Zm[0];
+            accP.jz = accP.jz - Zm[0];
+            accP.jx = accP.jx + Zm[1];
+            accP.xz = accP.xz - Zm[1];
+            accP.jy = accP.jy + Zm[2];
+            accP.yz = accP.yz - Zm[2];
+            accP.xx = accP.xx + Zm[3];
+            accP.xy = accP.xy + Zm[4];
+            accP.yy = accP.yy + Zm[5];
+            accP.red = accP.red + Zm[6];
+            accP.E = accP.E + Ep;
+
+            // (5) destination plane k-1 is complete: moments (lbm.cuh:239-261), store, boundary
+            if (d >= zd0 && d < zd1) {
                 constexpr float kS = kSepW ? 216.0f : 36.0f;
                 constexpr float sc = 1.0f / kS;
                 // correctly rounded mass quotients (no systematic bias), plain scaling for the rest
-                const float2 q = __fmul2_rn(accP.rr, pair(sc));
-                const float2 e = __ffma2_rn(make_float2(-q.x, -q.y), pair(kS), accP.rr);
-                accP.rr = __ffma2_rn(e, pair(sc), q);
-                // xx stays a scalar here: xx sc - rho/3 below then contracts to one fma, which
-                // keeps Pi's bits through the cancellation
-                accP.jxx.x *= sc; accP.jxx.y *= sc;
-                accP.jy *= sc; accP.jz *= sc;
-                accP.xy *= sc; accP.yy *= sc; accP.yz *= sc; accP.zz *= sc; accP.xz *= sc;
-            }
-            const float rho = accP.rr.x;
-            const float rr = accP.rr.y;
-            const float rb = rho - rr;
-            const float inv = fast_rcp(rho);
-            float Fbx = 0.0f, Fby = 0.0f, Fbz = 0.0f;
-            constexpr bool kF = (kFB & F_FORCE) != 0;
-            if (kF && P.forced) {
-                Fbx = rho * P.g[0];
-                Fby = rho * P.g[1];
-                Fbz = rho * P.g[2];
-            }
-            const float ux = (accP.jxx.x + 0.5f * Fbx) * inv;
-            const float uy = (accP.jy + 0.5f * Fby) * inv;
-            const float uz = (accP.jz + 0.5f * Fbz) * inv;
-            const float ctr = cs2 * rho;
-            float pi[6];
-            pi[0] = (accP.jxx.y - ctr) - rho * ux * ux;
-            pi[1] = accP.xy - rho * ux * uy;
-            pi[2] = (accP.yy - ctr) - rho * uy * uy;
-            pi[3] = accP.yz - rho * uy * uz;
-            pi[4] = (accP.zz - ctr) - rho * uz * uz;
-            pi[5] = accP.xz - rho * ux * uz;
-            if (kF && P.forced) {
-                pi[0] += ux * Fbx;
-                pi[1] += 0.5f * (ux * Fby + uy * Fbx);
-                pi[2] += uy * Fby;
-                pi[3] += 0.5f * (uy * Fbz + uz * Fby);
-                pi[4] += uz * Fbz;
-                pi[5] += 0.5f * (ux * Fbz + uz * Fbx);
-            }
-            if (kF && P.ratio) {
-                const float Kc = (rr * P.kappa_r + rb * P.kappa_b) * cs2;
-                pi[0] -= Kc;
-                pi[2] -= Kc;
-                pi[4] -= Kc;
-            }
-            finalize_store<S>(P, xs, ys, d, rr, rb, ux, uy, uz, pi, img_x, img_y, key_base);
-
-            if ((kFB & F_INOUT) && (bc_xy || (bc_z && (d == 1 || d == nz - 2)))) {
-                // inlet / outlet functors fused into the first and last fluid layer
-                const int pa = ia == 0 ? xs : (ia == 1 ? ys : d);
-                {
-                    const bool inlet = pa == 1;
-                    const int gx = ia == 0 ? (inlet ? 0 : nx - 1) : xs;
-                    const int gy = ia == 1 ? (inlet ? 0 : ny - 1) : ys;
-                    const int gz = ia == 2 ? (inlet ? 0 : nz - 1) : d;
-                    const long long og = static_cast<long long>(gz) * P.plane + static_cast<long long>(gy) * P.pitch + gx;
-                    float orr, orb, oux, ouy, ouz;
-                    if (inlet) {
-                        // jet/boundary_conditions.cuh:16-39 (+ seeded per-node noise)
-                        const int t0 = ia == 0 ? ys : xs;
-                        const int t1 = ia == 2 ? ys : d;
-                        const float du = static_cast<float>(t0) - P.jet_c0;
-                        const float dv = static_cast<float>(t1) - P.jet_c1;
-                        const float m = (du * du + dv * dv) <= (P.jet_radius * P.jet_radius) ? 1.0f : 0.0f;
-                        orr = P.jet_blue ? (1.0f - m) * P.rho_r0 : m * P.rho_r0;
-                        orb = P.jet_blue ? m * P.rho_b0 : (1.0f - m) * P.rho_b0;
-                        float gu[3] = {0.0f, 0.0f, 0.0f};
-                        if (m != 0.0f) {
-                            if (P.noise_amp != 0.0f) {
-                                const unsigned long long node = static_cast<unsigned long long>(gx) +
-                                                                static_cast<unsigned long long>(gy) * nx +
-                                                                static_cast<unsigned long long>(gz) * nx * ny;
-                                gu[0] = m * P.noise_amp * noise_xi(P.seed, step, node, 0);
-                                gu[1] = m * P.noise_amp * noise_xi(P.seed, step, node, 1);
-                                gu[2] = m * P.noise_amp * noise_xi(P.seed, step, node, 2);
-                            }
-                        }
-                        oux = gu[0] + (ia == 0 ? m * P.jet_velocity : 0.0f);
-                        ouy = gu[1] + (ia == 1 ? m * P.jet_velocity : 0.0f);
-                        ouz = gu[2] + (ia == 2 ? m * P.jet_velocity : 0.0f);
-                    } else if (P.outlet == MBCG_OUTLET_ZERO_GRADIENT) {
-                        orr = rr; orb = rb; oux = ux; ouy = uy; ouz = uz;
-                    } else {
-                        // convective outlet (jet/boundary_conditions.cuh:45-109), old ghost from A
-                        float ov[NF];
-                        if (ia == 2) {
-                            ov[0] = Codec<S>::to_f(rb_box(st, 0)[bR]);
-                            ov[1] = Codec<S>::to_f(rb_box(st, 1)[bR]);
-#pragma unroll
-                            for (int f = 2; f < NF; ++f) ov[f] = Codec<S>::to_f(m_box(st, f)[bM]);
-                        } else {
-                            load_global<S>(P, og, ov);
-                        }
-                        Node<S> on{};
-                        decode<S>(P, ov, on);
-                        const float ua = ia == 0 ? ux : (ia == 1 ? uy : uz);
-                        const float uc = fminf(fmaxf(ua, 0.0f), 1.0f);
-                        if (on.rr + on.rb <= 1.0e-20f) {
-                            orr = rr; orb = rb; oux = ux; ouy = uy; ouz = uz;
-                        } else {
-                            orr = on.rr - uc * (on.rr - rr);
-                            orb = on.rb - uc * (on.rb - rb);
-                            oux = on.ux - uc * (on.ux - ux);
-                            ouy = on.uy - uc * (on.uy - uy);
-                            ouz = on.uz - uc * (on.uz - uz);
-                        }
-                    }
-                    const int gix = P.bc[0] == MBCG_BC_PERIODIC ? (gx == 1 ? nx - 1 : (gx == nx - 2 ? 0 : -1)) : -1;
-                    const int giy = P.bc[1] == MBCG_BC_PERIODIC ? (gy == 1 ? ny - 1 : (gy == ny - 2 ? 0 : -1)) : -1;
-                    finalize_store<S>(P, gx, gy, gz, orr, orb, oux, ouy, ouz, pi, gix, giy, key_base);
+                auto quot = [&](F2 a) {
+                    const F2 q = sc * a;
+                    return fma2(sc, fma2(-kS, q, a), q);
+                };
+                const F2 dev = quot(accP.tot);
+                const F2 rho_n = ref + dev;
+                // each colour: the grid part's quotient and its remainder, then the small part, one
+                // rounding at the density's own magnitude
+                const F2 devR = quot(accP.red);
+                auto colour = [&](F2 e, F2 low) {
+                    const F2 q = quot(e);
+                    return fma2(ref, q, fma2(pair(P.rho_ref * sc), fma2(-kS, q, e), low));
+                };
+                const F2 rr_n = colour(accP.E, devR);
+                const F2 rb_n = colour(pair(kS) - accP.E, dev - devR);
+                const F2 isc = sc * make_float2(fast_rcp(rho_n.x), fast_rcp(rho_n.y));
+                const F2 iscy = make_float2(isc.x, -isc.y); // back from the mirrored frame
+                const F2 scy = make_float2(sc, -sc);
+                F2 u_x = accP.jx * isc, u_y = accP.jy * iscy, u_z = accP.jz * isc;
+                constexpr bool kF = (kFeat & F_FORCE) != 0;
+                if (kF && P.forced) {
+                    // u = (j + F/2) / rho with F = rho g
+                    u_x = u_x + pair(0.5f * P.g[0]);
+                    u_y = u_y + pair(0.5f * P.g[1]);
+                    u_z = u_z + pair(0.5f * P.g[2]);
                 }
+                const F2 ctr = (-1.0f / 3.0f) * dev;
+                const F2 rho_m = fma2(-1.0f, dev, pair(-P.rho_ref)); // -rho
+                const F2 mx = rho_m * u_x, my = rho_m * u_y, mz = rho_m * u_z;
+                F2 pi[6];
+                pi[0] = fma2(mx, u_x, fma2(sc, accP.xx, ctr));
+                pi[1] = fma2(mx, u_y, scy * accP.xy);
+                pi[2] = fma2(my, u_y, fma2(sc, accP.yy, ctr));
+                pi[3] = fma2(my, u_z, scy * accP.yz);
+                pi[4] = fma2(mz, u_z, fma2(sc, accP.zz, ctr));
+                pi[5] = fma2(mx, u_z, sc * accP.xz);
+                if (kF && P.forced) {
+                    const float hx = -0.5f * P.g[0], hy = -0.5f * P.g[1], hz = -0.5f * P.g[2];
+                    pi[0] = fma2(2.0f * hx, mx, pi[0]);
+                    pi[1] = fma2(hy, mx, fma2(hx, my, pi[1]));
+                    pi[2] = fma2(2.0f * hy, my, pi[2]);
+                    pi[3] = fma2(hz, my, fma2(hy, mz, pi[3]));
+                    pi[4] = fma2(2.0f * hz, mz, pi[4]);
+                    pi[5] = fma2(hz, mx, fma2(hx, mz, pi[5]));
+                }
+                if (kF && P.ratio) {
+                    const F2 Kc = (-1.0f / 3.0f) * fma2(P.kappa_r, rr_n, P.kappa_b * rb_n);
+                    pi[0] = pi[0] + Kc;
+                    pi[2] = pi[2] + Kc;
+                    pi[4] = pi[4] + Kc;
+                }
+                const float pa[6] = {pi[0].x, pi[1].x, pi[2].x, pi[3].x, pi[4].x, pi[5].x};
+                const float pb[6] = {pi[0].y, pi[1].y, pi[2].y, pi[3].y, pi[4].y, pi[5].y};
+                S oa[NF], ob[NF];
+                {
+                    const float ua[3] = {u_x.x, u_y.x, u_z.x}, ub[3] = {u_x.y, u_y.y, u_z.y};
+                    encode<S>(P, rr_n.x, rb_n.x, ua, pa, oa, sizeof(S) == 4 ? 0U : node_round_key(P, key_base, xs, ysa, d));
+                    encode<S>(P, rr_n.y, rb_n.y, ub, pb, ob, sizeof(S) == 4 ? 0U : node_round_key(P, key_base, xs, ysb, d));
+                }
+                if constexpr (kStride) {
+                    unsigned char* base_a = static_cast<unsigned char*>(P.b[0]) + tile_base + off_a;
+                    unsigned char* base_b = static_cast<unsigned char*>(P.b[0]) + tile_base + off_b;
+#pragma unroll
+                    for (int f = 0; f < NF; ++f, base_a += P.b_stride, base_b += P.b_stride) {
+                        if (dest_a) *reinterpret_cast<S*>(base_a) = oa[f];
+                        if (dest_b) *reinterpret_cast<S*>(base_b) = ob[f];
+                    }
+                } else {
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) {
+                        unsigned char* base = static_cast<unsigned char*>(P.b[f]) + tile_base;
+                        if (dest_a) *reinterpret_cast<S*>(base + off_a) = oa[f];
+                        if (dest_b) *reinterpret_cast<S*>(base + off_b) = ob[f];
+                    }
+                }
+                if (images) { // the faces of a periodic x / y axis only
+                    const int ix = image_of(0, xs, nx);
+                    if (dest_a) store_images<S>(P, tile_base, off_a, xs, ysa, oa, ix, image_of(1, ysa, ny));
+                    if (dest_b) store_images<S>(P, tile_base, off_b, xs, ysb, ob, ix, image_of(1, ysb, ny));
+                }
+                if constexpr ((kFeat & F_INOUT) != 0) {
+                    if (dest_a) boundary(ysa, bRa, bMa, st, d, rr_n.x, rb_n.x, u_x.x, u_y.x, u_z.x, pa);
+                    if (dest_b) boundary(ysb, bRb, bMb, st, d, rr_n.y, rb_n.y, u_x.y, u_y.y, u_z.y, pb);
+                }
+                off_a += plane_bytes;
+                off_b += plane_bytes;
             }
-        }
-        if (dest_row) {
-            gather(std::integral_constant<int, 0>{}, accC);
-            gather(std::integral_constant<int, 1>{}, accN);
-        }
-        accP = accC;
-        accC = accN; // accN is assigned before it is added to again
-            return true;
-    };
-    auto run = [&](auto featc, int kend) -> bool {
-        for (; k <= kend; ++k, sl = nxt(sl))
-            if (!plane(featc)) return false;
-        return true;
-    };
-    if constexpr ((kFeat & (F_INOUT | F_WALL)) != 0 && kLeanZ) {
-        // The inlet/outlet or wall axis along z: planes 3 (walls: 2) .. nz-5 need none of its parts
-        // (fluid sources with identity mappings, no wall-adjacent source, no functor store).
-        const bool zin = ia == 2, zwall = P.bc[2] == MBCG_BC_WALL;
-        if (zin || zwall) {
-            const int k0 = max(zd0 - 1, zin ? 3 : 2), k1 = min(zd1, nz - 5);
-            if (k1 >= k0) {
-                if (!run(std::integral_constant<int, kFeat>{}, k0 - 1)) return false;
-                if (!run(std::integral_constant<int, kFeat & ~(F_INOUT | F_WALL)>{}, k1)) return false;
-            }
+            auto addz = [](F2 a, F2 b) { return kSepW ? fma2(4.0f, b, a) : a + b; };
+            accP.tot = fma2(kSepW ? 64.0f : 12.0f, rc0, addz(accC.tot, Z0[0]));
+            accP.red = fma2(kSepW ? 64.0f : 12.0f, aR * rc0, addz(accC.red, Z0[6]));
+            accP.E = addz(accC.E, E0);
+            accP.jx = addz(accC.jx, Z0[1]);
+            accP.jy = addz(accC.jy, Z0[2]);
+            accP.jz = accC.jz;
+            accP.xx = addz(accC.xx, Z0[3]);
+            accP.xy = addz(accC.xy, Z0[4]);
+            accP.yy = addz(accC.yy, Z0[5]);
+            accP.yz = accC.yz;
+            accP.zz = accC.zz;
+            accP.xz = accC.xz;
+            accC.tot = accC.jz = accC.zz = Zp[0];
+            accC.jx = accC.xz = Zp[1];
+            accC.jy = accC.yz = Zp[2];
+            accC.xx = Zp[3];
+            accC.xy = Zp[4];
+            accC.yy = Zp[5];
+            accC.red = Zp[6];
+            accC.E = Ep;
         }
     }
-    if (!run(std::integral_constant<int, kFeat>{}, zd1)) return false;
     // every load of this tile was waited for: carry the parities over to the next tile
     phase = par;
     return true;
 }
 
+// Whether a tile stays clear of the non-periodic axis: every node it reads is then a fluid node of that
+// axis (or a periodic image), and it needs none of the inlet/outlet or wall parts.  Both kinds of tile
+// do the same arithmetic on a fluid source, so which one a node falls into does not show in its bits.
+template <int W>
+__device__ __forceinline__ bool tile_is_interior(const StepParams& P, int bx, int by, int bz) {
+    int zd0, zd1;
+    z_range(P.nz, P.bc[2], P.zchunk, bz, zd0, zd1);
+    const int xb = kTX * bx, yb = (W - 2) * by;
+    const bool x = P.bc[0] == MBCG_BC_PERIODIC || (xb - 1 >= 1 && xb + 32 <= P.nx - 2);
+    const bool y = P.bc[1] == MBCG_BC_PERIODIC || (yb - 1 >= 1 && yb + W <= P.ny - 2);
+    const bool z = P.bc[2] == MBCG_BC_PERIODIC || (zd0 - 2 >= 1 && zd1 + 1 <= P.nz - 2);
+    return x && y && z;
+}
+
 // ------------------------------------------------------------------ plain step kernel
-// One tile per CTA over the grid ((nx-2)/30, (ny-2)/(W-2), (nz-2)/zchunk), rounded up.
+// One tile per CTA over the grid ((nx-2)/30, (ny-2)/(W-2), z_tiles), rounded up.
 template <int Q, typename S, int W, bool kTMA, int kFeat>
-__global__ void __launch_bounds__(32 * W, W <= 8 ? 2 : 1) step_kernel(const __grid_constant__ StepParams P,
+__global__ void __launch_bounds__(16 * W, W <= 8 ? 2 : 1) step_kernel(const __grid_constant__ StepParams P,
                                                                       const __grid_constant__ TensorMaps T) {
     unsigned char* smem = aligned_smem_base();
     if constexpr (kTMA) init_stage_barriers(smem);
     uint32_t phase = 0;
+    if constexpr (kTMA && (kFeat & (F_WALL | F_INOUT)) != 0) {
+        if (tile_is_interior<W>(P, blockIdx.x, blockIdx.y, blockIdx.z)) {
+            step_tile<Q, S, W, kTMA, kFeat & ~(F_WALL | F_INOUT)>(P, T.m, blockIdx.x, blockIdx.y, blockIdx.z, P.step, smem,
+                                                                  phase);
+            return;
+        }
+    }
     step_tile<Q, S, W, kTMA, kFeat>(P, T.m, blockIdx.x, blockIdx.y, blockIdx.z, P.step, smem, phase);
 }
 
@@ -1282,9 +1676,11 @@ cudaError_t launch_one(const StepParams& P, const TensorMaps& T, cudaStream_t s)
     auto kern = step_kernel<Q, S, W, kTMA, kFeat>;
     static std::atomic<unsigned long long> configured{0};
     if (cudaError_t e = configure_once(kern, G::smem, configured)) return e;
-    dim3 block(32, W, 1);
-    dim3 grid((P.nx - 2 + kTX - 1) / kTX, (P.ny - 2 + W - 3) / (W - 2), (P.nz - 2 + P.zchunk - 1) / P.zchunk);
-    kern<<<grid, block, G::smem, s>>>(P, T);
+    StepParams L = P;
+    L.zchunk = std::min(L.zchunk, max_zchunk(L.plane, static_cast<int>(sizeof(S))));
+    dim3 block(32, W / 2, 1);
+    dim3 grid((L.nx - 2 + kTX - 1) / kTX, (L.ny - 2 + W - 3) / (W - 2), z_tiles(L.nz, L.bc[2], L.zchunk));
+    kern<<<grid, block, G::smem, s>>>(L, T);
     return cudaGetLastError();
 }
 
@@ -1303,8 +1699,8 @@ cudaError_t launch_w(bool tma, const StepParams& P, const TensorMaps& T, cudaStr
 
 template <int Q, typename S>
 cudaError_t launch_qs(bool tma, int w, const StepParams& P, const TensorMaps& T, cudaStream_t s) {
-    if (w == 8) return launch_w<Q, S, 8>(tma, P, T, s);
-    return launch_w<Q, S, 16>(tma, P, T, s);
+    if (w == kStepWSmall) return launch_w<Q, S, step_rows(kStepWSmall)>(tma, P, T, s);
+    return launch_w<Q, S, step_rows(kStepW)>(tma, P, T, s);
 }
 
 } // namespace
