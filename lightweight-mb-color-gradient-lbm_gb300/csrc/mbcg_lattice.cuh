@@ -135,6 +135,24 @@ MBCG_HD void colour_split(float c, float rho, float& rr, float& rb) {
     rb = red_major ? minor : major;
 }
 
+// ------------------------------------------------------------------ sums
+// Sum of floats kept as an unevaluated pair: hi + lo is the exact sum but for the roundings of lo
+// (Knuth's two-sum), 2^-48 of it a term.
+struct PairSum {
+    float hi, lo;
+    __device__ __forceinline__ void add(float v, float err = 0.0f) {
+        const float t = hi + v, z = t - hi;
+        lo += ((hi - (t - z)) + (v - z)) + err;
+        hi = t;
+    }
+    // move the sum into d
+    __device__ __forceinline__ void flush(double& d) {
+        d += static_cast<double>(hi);
+        d += static_cast<double>(lo);
+        hi = lo = 0.0f;
+    }
+};
+
 // ------------------------------------------------------------------ parameter block
 struct StepParams {
     int nx, ny, nz;
