@@ -124,13 +124,20 @@ void fill_physics(const mbcg_params& p, StepParams& P) {
     P.ghost_images = 1;
 }
 
+// source rows of the CTAs that step this lattice in shape W
+int case_rows(const mbcg_params& p, int W) {
+    StepParams P;
+    fill_physics(p, P);
+    return uses_pop(p.precision != MBCG_FP32, features_of(P)) ? W : step_rows(W);
+}
+
 int choose_zchunk(const mbcg_params& p, int W) {
     if (const char* env = std::getenv("MBCG_ZCHUNK")) {
         const int v = std::atoi(env);
         if (v > 0) return v;
     }
     const long long gx = (p.nx - 2 + kStepTileX - 1) / kStepTileX;
-    const int rows = step_tile_rows(W);
+    const int rows = case_rows(p, W) - 2;
     const long long g = gx * ((p.ny - 2 + rows - 1) / rows); // tiles side by side
     int sms = 152;
     int dev = 0;
@@ -191,12 +198,12 @@ bool tma_capable(const mbcg_params& p, const void* const* f, long long pitch, in
     return get_encode() != nullptr;
 }
 
-// TMA descriptors of one state for step CTAs of shape W: rhor / rhob boxes kStepRBX x (rows+2),
+// TMA descriptors of one state for step CTAs of `rows` source rows: rhor / rhob boxes kStepRBX x (rows+2),
 // the other fields kStepMX x rows, one plane deep
-int encode_maps(const mbcg_params& p, const void* const* f, long long pitch, int precision, int W, TensorMaps& T) {
+int encode_maps(const mbcg_params& p, const void* const* f, long long pitch, int precision, int rows, TensorMaps& T) {
     EncodeFn enc = get_encode();
     if (!enc) return fail(MBCG_E_CUDA, "cuTensorMapEncodeTiled unavailable");
-    const int es = elem_bytes(precision), rows = step_rows(W);
+    const int es = elem_bytes(precision);
     for (int i = 0; i < NF; ++i) {
         const cuuint64_t dims[3] = {static_cast<cuuint64_t>(p.nx), static_cast<cuuint64_t>(p.ny),
                                     static_cast<cuuint64_t>(p.nz)};
@@ -249,8 +256,8 @@ void mbcg::fill_step_physics(const mbcg_params& p, StepParams& P) { fill_physics
 bool mbcg::state_tma_capable(const mbcg_params& p, const void* const* f, long long pitch) {
     return tma_capable(p, f, pitch, p.precision);
 }
-int mbcg::encode_state_maps(const mbcg_params& p, const void* const* f, long long pitch, int W, TensorMaps& T) {
-    return encode_maps(p, f, pitch, p.precision, W, T);
+int mbcg::encode_state_maps(const mbcg_params& p, const void* const* f, long long pitch, int rows, TensorMaps& T) {
+    return encode_maps(p, f, pitch, p.precision, rows, T);
 }
 
 struct mbcg_case {
@@ -462,7 +469,7 @@ int mbcg_create(const mbcg_params* p, mbcg_case** out) {
              tma_capable(*p, c->fields[1], c->pitch, p->precision);
     if (c->tma) {
         for (int s = 0; s < 2; ++s)
-            if (int rc = encode_maps(*p, c->fields[s], c->pitch, p->precision, c->w, c->tm[s])) {
+            if (int rc = encode_maps(*p, c->fields[s], c->pitch, p->precision, case_rows(*p, c->w), c->tm[s])) {
                 free_case(c);
                 return rc;
             }
@@ -770,7 +777,7 @@ int mbcg_rcs_moments(const mbcg_params* p, const mbcg_moments* a, const mbcg_mom
     std::memset(&T, 0, sizeof(T));
     const bool tma = tma_capable(*p, a->f, a->pitch, p->precision);
     if (tma)
-        if (int rc = encode_maps(*p, a->f, a->pitch, p->precision, kStepW, T)) return rc;
+        if (int rc = encode_maps(*p, a->f, a->pitch, p->precision, case_rows(*p, kStepW), T)) return rc;
     MBCG_TRY(launch_step(p->q, p->precision, tma, kStepW, P, T, reinterpret_cast<cudaStream_t>(s)), "RCS kernel");
     return MBCG_OK;
 }
@@ -808,7 +815,7 @@ int mbcg_set_shape(mbcg_case* c, int32_t block_rows, int32_t zchunk) {
     if (block_rows != c->w && c->tma) {
         TensorMaps t[2];
         for (int s = 0; s < 2; ++s)
-            if (int rc = encode_maps(c->p, c->fields[s], c->pitch, c->p.precision, block_rows, t[s])) return rc;
+            if (int rc = encode_maps(c->p, c->fields[s], c->pitch, c->p.precision, case_rows(c->p, block_rows), t[s])) return rc;
         c->tm[0] = t[0];
         c->tm[1] = t[1];
     }
@@ -842,7 +849,7 @@ int mbcg_autotune(mbcg_case* c, int32_t repeats, double* best_ms, mbcg_stream_t 
     for (const auto& cand : cands) {
         TensorMaps T;
         std::memset(&T, 0, sizeof(T));
-        if (c->tma && (rc = encode_maps(c->p, c->fields[c->cur], c->pitch, c->p.precision, cand.first, T))) break;
+        if (c->tma && (rc = encode_maps(c->p, c->fields[c->cur], c->pitch, c->p.precision, case_rows(c->p, cand.first), T))) break;
         StepParams P = make_params(c, c->cur, c->steps + 1);
         P.zchunk = cand.second;
         cudaError_t e = launch_step(c->p.q, c->p.precision, c->tma, cand.first, P, T, st);

@@ -20,6 +20,9 @@ namespace mbcg {
 constexpr int kStepW = 16;
 constexpr int kStepWSmall = 8;
 constexpr int step_rows(int w) { return w == kStepWSmall ? 8 : 24; }
+// Fully periodic, unforced lattices in 16-bit storage step by populations, one node a thread, w source
+// rows (the reason stands in mbcg_step_pop.cuh).
+constexpr bool uses_pop(bool storage16, int features) { return storage16 && features == 0; }
 constexpr int kStepTileX = 30; // destination columns per tile
 constexpr int kStepRBX = 48;   // staged width of the rhor / rhob boxes
 constexpr int kStepMX = 40;    // staged width of the other nine boxes
@@ -38,7 +41,7 @@ cudaError_t launch_step_q27_f32(bool tma, int w, const StepParams& P, const Tens
 cudaError_t launch_step_q27_f16(bool tma, int w, const StepParams& P, const TensorMaps& T, cudaStream_t s);
 cudaError_t launch_step_q27_bf16(bool tma, int w, const StepParams& P, const TensorMaps& T, cudaStream_t s);
 int step_smem_bytes(int precision, int w);
-inline int step_tile_rows(int w) { return step_rows(w) - 2; }
+inline int step_tile_rows(int w) { return step_rows(w) - 2; } // destination rows
 // The step addresses the planes of a tile by 32-bit byte offsets: the deepest tile it may be given.
 inline int max_zchunk(long long plane, int elem_bytes) {
     const long long bytes = plane * elem_bytes;
@@ -75,7 +78,7 @@ void case_set_steps(mbcg_case* c, long long steps);
 int validate_params(const mbcg_params* p);
 void fill_step_physics(const mbcg_params& p, StepParams& P);
 bool state_tma_capable(const mbcg_params& p, const void* const* f, long long pitch);
-int encode_state_maps(const mbcg_params& p, const void* const* f, long long pitch, int W, TensorMaps& T);
+int encode_state_maps(const mbcg_params& p, const void* const* f, long long pitch, int rows, TensorMaps& T);
 
 constexpr int kDiagSlots = 12; // mass_r, mass_b, mom x/y/z, p_in sum, n_in, p_out sum, n_out, nonfinite, nodes, spare
 

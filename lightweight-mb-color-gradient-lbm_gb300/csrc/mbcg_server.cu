@@ -329,7 +329,7 @@ cudaError_t admit(mbcg_server* s, Request& r, int slot) {
         C.P[par] = step_params(r, par, status_word);
         const void* f[NF];
         for (int i = 0; i < NF; ++i) f[i] = r.fields[par][i];
-        if (encode_state_maps(r.p, f, r.pitch, kBatchW, *reinterpret_cast<TensorMaps*>(C.maps[par])) != MBCG_OK)
+        if (encode_state_maps(r.p, f, r.pitch, step_rows(kBatchW), *reinterpret_cast<TensorMaps*>(C.maps[par])) != MBCG_OK)
             return cudaErrorInvalidValue;
     }
     C.kind = batch_kind(r.p.q, r.p.precision, r.features);

@@ -264,7 +264,9 @@ __device__ __forceinline__ void encode(const StepParams& P, float rr, float rb, 
     } else {
         const float rho = rr + rb;
         S unused;
-        Codec<S>::from_f_sr(colour_slot(rr, rb, rho), 0.0f, lowbias32(key), out[1], unused);
+        // a minority density a rounding error below zero is zero: its sign would turn the slot's, and
+        // with it the node's colour
+        Codec<S>::from_f_sr(colour_slot(fmaxf(rr, 0.0f), fmaxf(rb, 0.0f), rho), 0.0f, lowbias32(key), out[1], unused);
         const float phi = phi_of_slot(Codec<S>::to_f(out[1])); // the phi a reader decodes
         Codec<S>::from_f_sr((rho - (P.rho_mean + phi * P.rho_half_diff)) * P.inv_rho_scale, u[0] * P.inv_u_ref,
                             lowbias32(key + 1), out[0], out[2]);
@@ -1691,7 +1693,8 @@ cudaError_t launch_w(bool tma, const StepParams& P, const TensorMaps& T, cudaStr
     if (!tma) return launch_one<Q, S, W, false, F_ALL>(P, T, s);
     if (std::getenv("MBCG_ALL_FEATURES")) return launch_one<Q, S, W, true, F_ALL>(P, T, s); // (parity tests)
     const int f = features_of(P);
-    if (f == 0) return launch_one<Q, S, W, true, 0>(P, T, s);
+    if constexpr (sizeof(S) == 4) // (the 16-bit forms step such lattices by populations)
+        if (f == 0) return launch_one<Q, S, W, true, 0>(P, T, s);
     if (f == F_INOUT) return launch_one<Q, S, W, true, F_INOUT>(P, T, s);
     if ((f & F_INOUT) == 0) return launch_one<Q, S, W, true, F_WALL | F_FORCE>(P, T, s); // walls, force
     return launch_one<Q, S, W, true, F_ALL>(P, T, s);

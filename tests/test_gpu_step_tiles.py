@@ -88,3 +88,23 @@ def test_tile_edges(kind, axis, q):
             if first is None:
                 first = got
             np.testing.assert_array_equal(got[idx], first[idx], err_msg=f"{kind} {axis} q{q} {size}")
+
+
+@pytest.mark.parametrize("precision", [mbcg.FP16, mbcg.BF16])
+def test_pure_nodes_keep_their_colour_in_16_bits(precision):
+    """A minority density that rounds below zero must not turn the colour slot's sign: after a step of
+    the density-ratio case from the same state, phi of the 16-bit form stays within the form's
+    resolution of FP32's at every node (half of it stored, as much again read back: 2^-10 and 2^-7)."""
+    p = mbcg.rti_params(64, 192, q=27)
+    a = ol.oracle_init(p, np.float64).astype(np.float32)
+    z, y, x = np.meshgrid(*(np.arange(k) for k in p.shape), indexing="ij")
+    a[2] += 0.01 * np.sin(2 * np.pi * (y - 1) / (p.ny - 2)) * np.sin(np.pi * z / (p.nz - 1))
+    phi = []
+    for prec in (mbcg.FP32, precision):
+        p.precision = prec
+        with mbcg.Case(p) as c:
+            c.copy_in(a)
+            c.step(1)
+            s = c.copy_out()[:, 1:-1, 1:-1, 1:-1].astype(np.float64)
+        phi.append((s[0] - s[1]) / (s[0] + s[1]))
+    assert np.abs(phi[0] - phi[1]).max() < 2.0 * (2.0 ** -10 if precision == mbcg.FP16 else 2.0 ** -7)
