@@ -148,8 +148,11 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
 }
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(__cvta_generic_to_global(src)) : "memory");
+// (zeros, without reading src, if not `valid`)
+__device__ __forceinline__ void cp_async4(void* dst, const void* src, bool valid = true) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)),
+                 "l"(__cvta_generic_to_global(src)), "r"(valid ? 4 : 0)
+                 : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -608,25 +611,33 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
 #pragma unroll
                 for (int f = 2; f < NF; ++f) tma_load_3d(m_box(st, f), &maps[f], xm0, yb, kz, bar);
             }
-        } else {
-            // plain-load path for layouts TMA cannot describe (row pitch not 16-byte aligned)
+        } else if constexpr (sizeof(S) == 4) {
+            // layouts TMA cannot describe (row pitch not a multiple of 16 bytes): every thread copies its
+            // two nodes by 4-byte cp.async (no one else reads them, but for the elements beside a
+            // boundary); zeros outside the lattice, as TMA fills
             const long long zo = static_cast<long long>(kz) * P.plane;
-            for (int e = tid; e < 2 * G::RBY * kRBX; e += kThreads) {
-                const int f = e / (G::RBY * kRBX), r = (e / kRBX) % G::RBY, c = e % kRBX;
-                const int gx = xr0 + c, gy = yb - 1 + r;
-                S v = Codec<S>::from_f(0.0f);
-                if (gx >= 0 && gx < nx && gy >= 0 && gy < ny)
-                    v = static_cast<const S*>(P.a[f])[zo + gy * P.pitch + gx];
-                rb_box(st, f)[r * kRBX + c] = v;
-            }
-            for (int e = tid; e < 9 * G::MY * kMX; e += kThreads) {
-                const int f = 2 + e / (G::MY * kMX), r = (e / kMX) % G::MY, c = e % kMX;
-                const int gx = xm0 + c, gy = yb + r;
-                S v = Codec<S>::from_f(0.0f);
-                if (gx >= 0 && gx < nx && gy >= 0 && gy < ny)
-                    v = static_cast<const S*>(P.a[f])[zo + gy * P.pitch + gx];
-                m_box(st, f)[r * kMX + c] = v;
-            }
+            auto node = [&](int ys, int iR, int iM) {
+                const bool in = xs < nx && ys < ny;
+                const long long o = zo + (in ? static_cast<long long>(ys) * P.pitch + xs : 0);
+#pragma unroll
+                for (int f = 0; f < NF; ++f)
+                    cp_async4(f < 2 ? rb_box(st, f) + iR : m_box(st, f) + iM, static_cast<const S*>(P.a[f]) + o, in);
+            };
+            node(ysa, bRa, bMa);
+            node(ysb, bRb, bMb);
+        } else {
+            // 16-bit elements (a copy moves four bytes at least): plain loads and stores
+            const long long zo = static_cast<long long>(kz) * P.plane;
+            auto node = [&](int ys, int iR, int iM) {
+                const bool in = xs < nx && ys < ny;
+                const long long o = zo + static_cast<long long>(ys) * P.pitch + xs;
+#pragma unroll
+                for (int f = 0; f < NF; ++f)
+                    (f < 2 ? rb_box(st, f)[iR] : m_box(st, f)[iM]) =
+                        in ? static_cast<const S*>(P.a[f])[o] : Codec<S>::from_f(0.0f);
+            };
+            node(ysa, bRa, bMa);
+            node(ysb, bRb, bMb);
         }
     };
     constexpr long long kWaitLimit = 4000000000LL; // ~2 s at 2 GHz
@@ -707,7 +718,8 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
             const int dx = (px && gx >= 0 && gx <= nx - 1) ? gx : mx;
             const int dy = (py && gy >= 0 && gy <= ny - 1) ? gy : my;
             const int bc_ = dx - xr0, br_ = dy - (yb - 1);
-            const bool box = bc_ >= 0 && bc_ < kRBX && br_ >= 0 && br_ < G::RBY;
+            // (the plain copies stage the source nodes only)
+            const bool box = kTMA && bc_ >= 0 && bc_ < kRBX && br_ >= 0 && br_ < G::RBY;
             const int off = static_cast<int>(static_cast<long long>(my) * P.pitch + mx); // a plane is below 2^31 elements
             const int at = atomicAdd(&fcount[box ? 0 : 1], 1);
             ftab[box ? at : G::frame - 1 - at] = make_int2(((box ? br_ * kRBX + bc_ : 0) << 16) | (r * kPSX + c), off);
@@ -802,7 +814,10 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
     if (tid < 2) fcount[tid] = 0;
     __syncthreads();
     build_frame();
-    if constexpr (!kTMA) __syncthreads();
+    if constexpr (!kTMA) {
+        cp_async_wait_all();
+        __syncthreads();
+    }
     {
         // The first wait.  Testing only (wait_test_cycles > 0): it waits on the barrier nothing
         // completes, with that limit, so it runs out and the tile takes the bail path with all its
@@ -953,7 +968,8 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
             }
         }
         if (w == 0 && k + 2 <= zd1 + 1) fetch_far(mz2); // far psi elements of plane k+2, used in (4)
-        // (2) plain loads: plane k+kNSTAGE-1 into the slot plane k-1 used (TMA: at the end of (4))
+        // (2) plain copies: plane k+kNSTAGE-1 into the slot plane k-1 used, complete before the next
+        // barrier (TMA: at the end of (4))
         if constexpr (!kTMA)
             if (k + kNSTAGE - 1 <= zd1 + 1) issue(k + kNSTAGE - 1, sl_prev);
 
@@ -1402,6 +1418,7 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
             put_both(16, ownE0);
             put_both(17, ec);
         }
+        if constexpr (!kTMA) cp_async_wait_all();
         __syncthreads();
 
         // (4) y sums, z streaming; warp 0 holds the two halo rows and receives nothing: it refills the
@@ -1648,7 +1665,7 @@ __global__ void __launch_bounds__(16 * W, W <= 8 ? 2 : 1) step_kernel(const __gr
     unsigned char* smem = aligned_smem_base();
     if constexpr (kTMA) init_stage_barriers(smem);
     uint32_t phase = 0;
-    if constexpr (kTMA && (kFeat & (F_WALL | F_INOUT)) != 0) {
+    if constexpr ((kFeat & (F_WALL | F_INOUT)) != 0) {
         if (tile_is_interior<W>(P, blockIdx.x, blockIdx.y, blockIdx.z)) {
             step_tile<Q, S, W, kTMA, kFeat & ~(F_WALL | F_INOUT)>(P, T.m, blockIdx.x, blockIdx.y, blockIdx.z, P.step, smem,
                                                                   phase);
