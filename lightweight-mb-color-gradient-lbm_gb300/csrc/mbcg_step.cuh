@@ -75,6 +75,7 @@ constexpr int kRBX = kStepRBX;   // staged width of rhor/rhob rows (34 needed + 
 constexpr int kMX = kStepMX;     // staged width of the other 9 fields (32 needed + slack)
 constexpr int kPSX = 34;   // psi ring width (32 sources + 1 on each side)
 constexpr int kMaxStages = 4; // planes staged at most: k, k+1, and k+2, k+3 in flight
+constexpr int kPlaneBar = kMaxStages + 1; // the warps' barrier of a plane (after the stages' and the test's)
 constexpr unsigned kFull = 0xffffffffu;
 
 constexpr int align128(int b) { return (b + 127) / 128 * 128; }
@@ -120,6 +121,9 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
@@ -498,12 +502,14 @@ __device__ __forceinline__ unsigned char* aligned_smem_base() {
     return smem_raw + ((128U - (smem_u32(smem_raw) & 127U)) & 127U);
 }
 
-// Initialise the stage mbarriers (one elected thread) before the first tile of a CTA.  One more
-// barrier after them is never arrived at: the bounded-wait test hook waits on it.
+// Initialise the stage mbarriers (one elected thread) before the first tile of a CTA.  Of the two
+// barriers after them the first is never arrived at, the bounded-wait test hook waits on it, and the
+// second is the warps' (kPlaneBar).
 __device__ __forceinline__ void init_stage_barriers(unsigned char* smem) {
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
     if (threadIdx.x == 0 && threadIdx.y == 0) {
         for (int s = 0; s <= kMaxStages; ++s) mbar_init(&bars[s], 1);
+        mbar_init(&bars[kPlaneBar], blockDim.y); // one arrival per warp
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -943,8 +949,9 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
     int k = zd0 - 1;
     for (; k <= zd1; ++k, sl = nxt(sl)) {
         const int sl_next = nxt(sl), sl_prev = prv(sl);
-        // (1) psi of plane k+1; one barrier both publishes the ring and makes the bail decision
-        // uniform (a plane that never arrived leaves garbage in the ring, which nobody reads).
+        // (1) psi of plane k+1.  Each warp arrives at the plane's barrier when its part of the ring is
+        // written (and it has read the previous plane's y exchange) and waits for the others only where it
+        // needs theirs: before a colour gradient, and before it overwrites the exchange buffer.
         // Plane coordinates: every mapping (staging, colour-gradient rule, node role) is the
         // identity while planes k .. k+3 are fluid planes, which is almost every plane.
         const bool zid = k >= 1 && k + 3 <= nz - 2;
@@ -958,15 +965,13 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
             rz = axis_role<kFeat>(P, 2, k, nz);
         }
         const F2 s0 = c0, s1 = c1; // fields 0 and 1 at plane k
-        {
-            const bool ok = wait_slot(k + 1, sl_next);
-            load_colours(sl_next, c0, c1);
-            if (ok) fill_own(std::bool_constant<kMapXY>{}, mz1, inbox1, sl_next, c0, c1);
-            if (__syncthreads_or(!ok)) {
-                bail(min(zd1 + 1, k - 1 + kNSTAGE));
-                return false;
-            }
-        }
+        // a plane that never arrived leaves garbage in the ring; the tile ends at the next barrier
+        bool ok = wait_slot(k + 1, sl_next);
+        load_colours(sl_next, c0, c1);
+        if (ok) fill_own(std::bool_constant<kMapXY>{}, mz1, inbox1, sl_next, c0, c1);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[kPlaneBar]);
+        auto wait_plane = [&]() { return mbar_wait_bounded(&bars[kPlaneBar], (par >> kPlaneBar) & 1u, kWaitLimit); };
         if (w == 0 && k + 2 <= zd1 + 1) fetch_far(mz2); // far psi elements of plane k+2, used in (4)
         // (2) plain copies: plane k+kNSTAGE-1 into the slot plane k-1 used, complete before the next
         // barrier (TMA: at the end of (4))
@@ -1125,6 +1130,7 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
         const bool any_iface = __any_sync(kFull, if_a || if_b);
         F2 dFx = pair(0.0f), dFy = dFx, dFz = dFx;
         if (any_iface) {
+            ok = wait_plane() && ok;
             const float* rm = psi_ring + sl_prev * G::psi_plane;
             const float* r0p = psi_ring + sl * G::psi_plane;
             const float* rp = psi_ring + sl_next * G::psi_plane;
@@ -1338,6 +1344,9 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
             }
         }
 
+        ok = wait_plane() && ok;
+        par ^= 1u << kPlaneBar;
+
         // ---- y streaming.  What leaves a row for the next row inwards (cy' = +1 of the mirrored
         // frame) and outwards (cy' = -1) goes through shared memory; the row's own part waits in
         // registers.  Weights: D3Q27 216 w = product over the axes of (4 if c_a = 0 else 1), the 4s
@@ -1419,7 +1428,10 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
             put_both(17, ec);
         }
         if constexpr (!kTMA) cp_async_wait_all();
-        __syncthreads();
+        if (__syncthreads_or(!ok)) {
+            bail(min(zd1 + 1, k - 1 + kNSTAGE));
+            return false;
+        }
 
         // (4) y sums, z streaming; warp 0 holds the two halo rows and receives nothing: it refills the
         // slot of plane k (whose fields everyone has read) and prepares the psi frame of plane k+2
@@ -1663,7 +1675,7 @@ template <int Q, typename S, int W, bool kTMA, int kFeat>
 __global__ void __launch_bounds__(16 * W, W <= 8 ? 2 : 1) step_kernel(const __grid_constant__ StepParams P,
                                                                       const __grid_constant__ TensorMaps T) {
     unsigned char* smem = aligned_smem_base();
-    if constexpr (kTMA) init_stage_barriers(smem);
+    init_stage_barriers(smem);
     uint32_t phase = 0;
     if constexpr ((kFeat & (F_WALL | F_INOUT)) != 0) {
         if (tile_is_interior<W>(P, blockIdx.x, blockIdx.y, blockIdx.z)) {
