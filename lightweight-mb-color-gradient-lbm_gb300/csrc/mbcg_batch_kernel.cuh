@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(16 * W, 1)
     batch_kernel(const BatchCase* __restrict__ cases, const BatchTile* __restrict__ tiles, int ntiles,
                  const ChunkState* __restrict__ chunk, int* __restrict__ counter, int j) {
     __shared__ int s_tile;
-    init_stage_barriers(aligned_smem_base());
+    init_barriers<W / 2>(aligned_smem_base());
     uint32_t phase = 0;
     const int tid = threadIdx.y * 32 + threadIdx.x;
     for (;;) {

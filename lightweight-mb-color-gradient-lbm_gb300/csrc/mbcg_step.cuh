@@ -29,9 +29,9 @@
 // Two nodes a thread.  A warp holds two rows of the tile, w from below and w from above, one in each
 // half of f32x2 registers, the upper one in a frame with y mirrored: both halves take the same
 // operations throughout, and every arithmetic instruction does two nodes' work.  The kernel is bound by
-// instruction issue and latency, not by HBM (D3Q27 jet 256x256x1024, FP32, measured in ncu): 560 warp
-// instructions per 32 node updates and 12 warps per SM, against 971 and 16 for one node a thread with all
-// 27 populations formed and crossing lanes; 2.72 ms -> 2.02 ms a step (24.7 -> 33.2 GLUPS).
+// instruction issue and latency, not by HBM (D3Q27 jet 256x256x1024, FP32): 590 warp instructions per 32
+// node updates and 12 warps per SM, against 971 and 16 for one node a thread with all 27 populations
+// formed and crossing lanes; 2.72 ms -> 1.90 ms a step (24.7 -> 35.4 GLUPS).
 //
 // Tiling.  A CTA is 32 lanes (x) x W rows (y), W/2 warps.  Lanes 0 and 31 and rows 0 and W-1 are
 // halo sources; the CTA writes the 30 x (W-2) destination columns in between, for a chunk of
@@ -76,11 +76,12 @@ constexpr int kMX = kStepMX;     // staged width of the other 9 fields (32 neede
 constexpr int kPSX = 34;   // psi ring width (32 sources + 1 on each side)
 constexpr int kMaxStages = 4; // planes staged at most: k, k+1, and k+2, k+3 in flight
 constexpr int kPlaneBar = kMaxStages + 1; // the warps' barrier of a plane (after the stages' and the test's)
+constexpr int kYBar = kPlaneBar + 1;      // and one for each warp
 constexpr unsigned kFull = 0xffffffffu;
 
 constexpr int align128(int b) { return (b + 127) / 128 * 128; }
 
-// Shared-memory carve-up of one tile: the mbarriers in the first 128 bytes, then the staged
+// Shared-memory carve-up of one tile: the mbarriers in the first 256 bytes, then the staged
 // planes, the psi ring and the y-exchange buffer.  `smem` is the dynamic size to request (it
 // includes 128 bytes of slack for aligning the base).
 template <typename S, int W>
@@ -103,7 +104,7 @@ struct Geo {
     static constexpr int ftab = align128(frame * 8 + 8);   // int2 [element], then the two list lengths
     static constexpr int fbuf = align128(frame * 8);       // uint2 [far element]: words of fields 0 and 1
     static constexpr int off_bar = 0;
-    static constexpr int off_stage = 128;
+    static constexpr int off_stage = 256;
     static constexpr int off_psi = off_stage + NST * stage;
     static constexpr int off_xbuf = off_psi + psi;
     static constexpr int off_ftab = off_xbuf + xbuf;
@@ -457,13 +458,12 @@ __device__ __forceinline__ void build_coef(const StepParams& P, Coef& c, const N
     c.p000 = -0.5f * (c.exx + c.eyy + c.ezz);
 }
 
-// Sums of one destination pair over the directions received so far (weights scaled to integers):
-// tot (less the reference density), red (likewise less part E), the momentum and the second moments.
+// Sums of one destination pair over the directions received so far (weights scaled to integers): tot (less
+// the reference density), red (likewise less part E), momentum and second moments in the plane.  Those with
+// cz need none of their own while a plane is plane k: they are what came with cz = +1 (walls aside).
 struct Acc2 {
-    F2 tot, red, E, jx, jy, jz, xx, xy, yy, yz, zz, xz;
-    __device__ __forceinline__ void zero() {
-        tot = red = E = jx = jy = jz = xx = xy = yy = yz = zz = xz = make_float2(0.0f, 0.0f);
-    }
+    F2 tot, red, E, jx, jy, xx, xy, yy;
+    __device__ __forceinline__ void zero() { tot = red = E = jx = jy = xx = xy = yy = make_float2(0.0f, 0.0f); }
 };
 
 // ------------------------------------------------------------------ the kernel
@@ -502,14 +502,19 @@ __device__ __forceinline__ unsigned char* aligned_smem_base() {
     return smem_raw + ((128U - (smem_u32(smem_raw) & 127U)) & 127U);
 }
 
-// Initialise the stage mbarriers (one elected thread) before the first tile of a CTA.  Of the two
-// barriers after them the first is never arrived at, the bounded-wait test hook waits on it, and the
-// second is the warps' (kPlaneBar).
-__device__ __forceinline__ void init_stage_barriers(unsigned char* smem) {
+// Initialise the mbarriers (one elected thread) before the first tile of a CTA.  The one after the
+// stages' is never arrived at: the bounded-wait test hook waits on it.  kPlaneBar counts the H warps of a
+// CTA, kYBar + w the warps that warp w waits for in the y exchange: those of the rows beside its own (the
+// innermost is its own neighbour), or, warp 0, all others.
+template <int H>
+__device__ __forceinline__ void init_barriers(unsigned char* smem) {
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
     if (threadIdx.x == 0 && threadIdx.y == 0) {
         for (int s = 0; s <= kMaxStages; ++s) mbar_init(&bars[s], 1);
-        mbar_init(&bars[kPlaneBar], blockDim.y); // one arrival per warp
+        if constexpr (H > 0) {
+            mbar_init(&bars[kPlaneBar], H);
+            for (int w = 0; w < H; ++w) mbar_init(&bars[kYBar + w], w == 0 ? H - 1 : (w < H - 1 ? 2 : 1));
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -669,6 +674,22 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
         if constexpr (kTMA) return mbar_wait_bounded(&bars[sl], (par >> sl) & 1u, kWaitLimit);
         else return true;
     };
+    // ---- the warps' synchronisation within a plane: psi of plane k+1 in the ring and the y exchange of
+    // plane k-1 read (kPlaneBar, every warp for every warp), then the y exchange of plane k written and the
+    // plane's fields and psi read.  A warp needs the latter of warps w-1 and w+1 only, warp 0, which refills
+    // the ring, of all: kNearBar has each warp wait for just these, on a barrier of its own.  No warp arrives
+    // there twice before the waiting one has passed: kPlaneBar comes between.
+    // The slowest warp of a plane then does not hold the others: D3Q27 jet 256x256x1024 1.94 -> 1.90 ms, in
+    // FP16 2.46 -> 2.33 ms; periodic 192^3 507 -> 493 us; 128^3 RTI 665 -> 652 us, in FP16 794 -> 745 us.  One
+    // barrier of the CTA is the better where the warps are few (W = 8: periodic 64^3 493 against 515 us for
+    // 20 steps) and in bodies with an inlet (128^3 jet along y, 456 against 469 us for 4 steps).
+    constexpr bool kNearBar = kTMA && W > 8 && (kFeat & F_INOUT) == 0;
+    // this lane's kYBar to arrive at
+    int y_target = -1;
+    if (lane == 0) y_target = w == 0 ? 1 : 0;
+    if (lane == 1 && w >= 1 && w < H - 1) y_target = w + 1;
+    if (lane == 2 && w >= 2) y_target = w - 1;
+    auto plane_wait = [&](int bar) { return mbar_wait_bounded(&bars[bar], (par >> kPlaneBar) & 1u, kWaitLimit); };
     // On a failed wait: flag it, drain the copies still in flight (bounded) and leave.  If the drain
     // gives up too, copies may still land in this block's shared memory after it exits, which the
     // status cannot tell apart (a flag for it once cost the batch kernel 3-5 %): the host treats
@@ -676,7 +697,7 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
     auto bail = [&](int k_issued) {
         if (tid == 0 && P.status) atomicOr(P.status, 1);
         if constexpr (kTMA) {
-            for (int k = k_waited + 1; k <= k_issued; ++k) {
+            for (int k = k_waited + 1; w == 0 && k <= k_issued; ++k) {
                 const int sl = (k - kfirst) % kNSTAGE;
                 mbar_wait_bounded(&bars[sl], (par >> sl) & 1u, kWaitLimit / 4);
             }
@@ -845,8 +866,8 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
             return false;
         }
     }
-    F2 c0, c1; // stored slots 0 and 1 of this thread's nodes on the next plane to be a source
     {
+        F2 c0, c1;
         const int m0 = psi_coord(P, 2, kfirst, nz), m1 = psi_coord(P, 2, kfirst + 1, nz);
         load_colours(0, c0, c1);
         fill_own(std::bool_constant<kMapXY>{}, m0, m0 == zload(kfirst), 0, c0, c1);
@@ -873,9 +894,11 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
     unsigned off_b = (static_cast<unsigned>(ysb) * static_cast<unsigned>(P.pitch) + static_cast<unsigned>(xs)) *
                            static_cast<unsigned>(sizeof(S));
 
-    Acc2 accP, accC; // destination planes k-1 and k
+    Acc2 accP, accC; // destination planes k-1 and k (accC: what plane k-1 sent with cz = +1)
+    F2 jzP, yzP, zzP, xzP; // plane k-1's sums with cz, less what plane k sends it
     accP.zero();
     accC.zero();
+    jzP = yzP = zzP = xzP = make_float2(0.0f, 0.0f);
 
     // inlet / outlet functors fused into the store of the first and last fluid layer: the ghost node
     // behind node (xs, ys, d), whose new moments are given
@@ -945,13 +968,13 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
         finalize_store<S>(P, og * static_cast<int>(sizeof(S)), 0U, gx, gy, gz, orr, orb, oux, ouy, ouz, pi, gix, giy, key_base);
     };
 
+    bool ok = true; // kNearBar: this warp's (one that gave up arrives no more, and those that need it give up in turn)
     int sl = 1; // slot of plane k (k starts at kfirst + 1)
     int k = zd0 - 1;
     for (; k <= zd1; ++k, sl = nxt(sl)) {
         const int sl_next = nxt(sl), sl_prev = prv(sl);
-        // (1) psi of plane k+1.  Each warp arrives at the plane's barrier when its part of the ring is
-        // written (and it has read the previous plane's y exchange) and waits for the others only where it
-        // needs theirs: before a colour gradient, and before it overwrites the exchange buffer.
+        // (1) psi of plane k+1.  A warp waits for the others' part only where it needs it: before a colour
+        // gradient, and before it overwrites the exchange buffer.
         // Plane coordinates: every mapping (staging, colour-gradient rule, node role) is the
         // identity while planes k .. k+3 are fluid planes, which is almost every plane.
         const bool zid = k >= 1 && k + 3 <= nz - 2;
@@ -964,14 +987,15 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
             inbox2 = mz2 == zload(k + 2);
             rz = axis_role<kFeat>(P, 2, k, nz);
         }
-        const F2 s0 = c0, s1 = c1; // fields 0 and 1 at plane k
         // a plane that never arrived leaves garbage in the ring; the tile ends at the next barrier
-        bool ok = wait_slot(k + 1, sl_next);
+        ok = wait_slot(k + 1, sl_next);
+        if constexpr (kNearBar)
+            if (!(ok = __all_sync(kFull, ok))) break;
+        F2 c0, c1; // stored slots 0 and 1 of this thread's nodes
         load_colours(sl_next, c0, c1);
         if (ok) fill_own(std::bool_constant<kMapXY>{}, mz1, inbox1, sl_next, c0, c1);
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[kPlaneBar]);
-        auto wait_plane = [&]() { return mbar_wait_bounded(&bars[kPlaneBar], (par >> kPlaneBar) & 1u, kWaitLimit); };
         if (w == 0 && k + 2 <= zd1 + 1) fetch_far(mz2); // far psi elements of plane k+2, used in (4)
         // (2) plain copies: plane k+kNSTAGE-1 into the slot plane k-1 used, complete before the next
         // barrier (TMA: at the end of (4))
@@ -996,10 +1020,11 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
                 va[f] = Codec<S>::to_f(m_box(st, f)[bMa]);
                 vb[f] = Codec<S>::to_f(m_box(st, f)[bMb]);
             }
-            va[0] = s0.x;
-            vb[0] = s0.y;
-            va[1] = s1.x;
-            vb[1] = s1.y;
+            load_colours(sl, c0, c1); // (again: kept from the plane before, they spill others)
+            va[0] = c0.x;
+            vb[0] = c0.y;
+            va[1] = c1.x;
+            vb[1] = c1.y;
             decode2<S>(P, va, vb, nd);
             vx = nd.ux;
             vy = nd.uy;
@@ -1130,7 +1155,7 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
         const bool any_iface = __any_sync(kFull, if_a || if_b);
         F2 dFx = pair(0.0f), dFy = dFx, dFz = dFx;
         if (any_iface) {
-            ok = wait_plane() && ok;
+            ok = plane_wait(kPlaneBar) && ok;
             const float* rm = psi_ring + sl_prev * G::psi_plane;
             const float* r0p = psi_ring + sl * G::psi_plane;
             const float* rp = psi_ring + sl_next * G::psi_plane;
@@ -1212,7 +1237,10 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
         }
 
         // wall bounce-back of this thread's own populations (destination = source, plane k)
+        [[maybe_unused]] F2 wall[4]; // its part of jz, yz, zz, xz, less that of tot, jy, tot, jx
         if constexpr ((kFeat & F_WALL) != 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) wall[i] = pair(0.0f);
             auto reflect = [&](int half, int role, bool dest, int ysh) {
                 const bool wx0 = P.bc[0] == MBCG_BC_WALL && xs == 1, wx1 = P.bc[0] == MBCG_BC_WALL && xs == nx - 2;
                 const bool wy0 = P.bc[1] == MBCG_BC_WALL && ysh == 1, wy1 = P.bc[1] == MBCG_BC_WALL && ysh == ny - 2;
@@ -1255,8 +1283,12 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
                     sums[10] += cz * cz * g;
                     sums[11] += cx * cz * g;
                 }
-                F2* a[12] = {&accC.tot, &accC.red, &accC.E, &accC.jx, &accC.jy, &accC.jz,
-                             &accC.xx, &accC.xy, &accC.yy, &accC.yz, &accC.zz, &accC.xz};
+                F2* a[12] = {&accC.tot, &accC.red, &accC.E, &accC.jx, &accC.jy, &wall[0],
+                             &accC.xx, &accC.xy, &accC.yy, &wall[1], &wall[2], &wall[3]};
+                sums[5] -= sums[0];
+                sums[9] -= sums[4];
+                sums[10] -= sums[0];
+                sums[11] -= sums[3];
 #pragma unroll
                 for (int i = 0; i < 12; ++i) {
                     if (half) a[i]->y += sums[i];
@@ -1344,8 +1376,7 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
             }
         }
 
-        ok = wait_plane() && ok;
-        par ^= 1u << kPlaneBar;
+        ok = plane_wait(kPlaneBar) && ok;
 
         // ---- y streaming.  What leaves a row for the next row inwards (cy' = +1 of the mirrored
         // frame) and outwards (cy' = -1) goes through shared memory; the row's own part waits in
@@ -1428,10 +1459,15 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
             put_both(17, ec);
         }
         if constexpr (!kTMA) cp_async_wait_all();
-        if (__syncthreads_or(!ok)) {
-            bail(min(zd1 + 1, k - 1 + kNSTAGE));
-            return false;
+        if constexpr (kNearBar) {
+            if (!(ok = __all_sync(kFull, ok))) break;
+            __syncwarp();
+            if (y_target >= 0) mbar_arrive(&bars[kYBar + y_target]);
+            if (!(ok = __all_sync(kFull, plane_wait(kYBar + w)))) break;
+        } else {
+            if (!(ok = !__syncthreads_or(!ok))) break;
         }
+        par ^= 1u << kPlaneBar;
 
         // (4) y sums, z streaming; warp 0 holds the two halo rows and receives nothing: it refills the
         // slot of plane k (whose fields everyone has read) and prepares the psi frame of plane k+2
@@ -1522,21 +1558,17 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
                 Ep = both(17) + ownE0;
             }
             // destination plane k-1 receives cz = -1, plane k cz = 0, plane k+1 cz = +1
-            accP.tot = accP.tot + Zm[0];
-            accP.zz = accP.zz + Zm[0];
-            accP.jz = accP.jz - Zm[0];
-            accP.jx = accP.jx + Zm[1];
-            accP.xz = accP.xz - Zm[1];
-            accP.jy = accP.jy + Zm[2];
-            accP.yz = accP.yz - Zm[2];
-            accP.xx = accP.xx + Zm[3];
-            accP.xy = accP.xy + Zm[4];
-            accP.yy = accP.yy + Zm[5];
-            accP.red = accP.red + Zm[6];
-            accP.E = accP.E + Ep;
-
             // (5) destination plane k-1 is complete: moments (lbm.cuh:239-261), store, boundary
             if (d >= zd0 && d < zd1) {
+                accP.tot = accP.tot + Zm[0];
+                accP.jx = accP.jx + Zm[1];
+                accP.jy = accP.jy + Zm[2];
+                accP.xx = accP.xx + Zm[3];
+                accP.xy = accP.xy + Zm[4];
+                accP.yy = accP.yy + Zm[5];
+                accP.red = accP.red + Zm[6];
+                accP.E = accP.E + Ep;
+                const F2 jz = jzP - Zm[0], zz = zzP + Zm[0], xz = xzP - Zm[1], yz = yzP - Zm[2];
                 constexpr float kS = kSepW ? 216.0f : 36.0f;
                 constexpr float sc = 1.0f / kS;
                 // correctly rounded mass quotients (no systematic bias), plain scaling for the rest
@@ -1558,7 +1590,7 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
                 const F2 isc = sc * make_float2(fast_rcp(rho_n.x), fast_rcp(rho_n.y));
                 const F2 iscy = make_float2(isc.x, -isc.y); // back from the mirrored frame
                 const F2 scy = make_float2(sc, -sc);
-                F2 u_x = accP.jx * isc, u_y = accP.jy * iscy, u_z = accP.jz * isc;
+                F2 u_x = accP.jx * isc, u_y = accP.jy * iscy, u_z = jz * isc;
                 constexpr bool kF = (kFeat & F_FORCE) != 0;
                 if (kF && P.forced) {
                     // u = (j + F/2) / rho with F = rho g
@@ -1573,9 +1605,9 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
                 pi[0] = fma2(mx, u_x, fma2(sc, accP.xx, ctr));
                 pi[1] = fma2(mx, u_y, scy * accP.xy);
                 pi[2] = fma2(my, u_y, fma2(sc, accP.yy, ctr));
-                pi[3] = fma2(my, u_z, scy * accP.yz);
-                pi[4] = fma2(mz, u_z, fma2(sc, accP.zz, ctr));
-                pi[5] = fma2(mx, u_z, sc * accP.xz);
+                pi[3] = fma2(my, u_z, scy * yz);
+                pi[4] = fma2(mz, u_z, fma2(sc, zz, ctr));
+                pi[5] = fma2(mx, u_z, sc * xz);
                 if (kF && P.forced) {
                     const float hx = -0.5f * P.g[0], hy = -0.5f * P.g[1], hz = -0.5f * P.g[2];
                     pi[0] = fma2(2.0f * hx, mx, pi[0]);
@@ -1627,28 +1659,38 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
                 off_a += plane_bytes;
                 off_b += plane_bytes;
             }
+            jzP = zzP = accC.tot;
+            yzP = accC.jy;
+            xzP = accC.jx;
+            if constexpr ((kFeat & F_WALL) != 0) {
+                jzP = jzP + wall[0];
+                yzP = yzP + wall[1];
+                zzP = zzP + wall[2];
+                xzP = xzP + wall[3];
+            }
             auto addz = [](F2 a, F2 b) { return kSepW ? fma2(4.0f, b, a) : a + b; };
             accP.tot = fma2(kSepW ? 64.0f : 12.0f, rc0, addz(accC.tot, Z0[0]));
             accP.red = fma2(kSepW ? 64.0f : 12.0f, aR * rc0, addz(accC.red, Z0[6]));
             accP.E = addz(accC.E, E0);
             accP.jx = addz(accC.jx, Z0[1]);
             accP.jy = addz(accC.jy, Z0[2]);
-            accP.jz = accC.jz;
             accP.xx = addz(accC.xx, Z0[3]);
             accP.xy = addz(accC.xy, Z0[4]);
             accP.yy = addz(accC.yy, Z0[5]);
-            accP.yz = accC.yz;
-            accP.zz = accC.zz;
-            accP.xz = accC.xz;
-            accC.tot = accC.jz = accC.zz = Zp[0];
-            accC.jx = accC.xz = Zp[1];
-            accC.jy = accC.yz = Zp[2];
+            accC.tot = Zp[0];
+            accC.jx = Zp[1];
+            accC.jy = Zp[2];
             accC.xx = Zp[3];
             accC.xy = Zp[4];
             accC.yy = Zp[5];
             accC.red = Zp[6];
             accC.E = Ep;
         }
+    }
+    if constexpr (kNearBar) ok = !__syncthreads_or(!ok);
+    if (!ok) {
+        bail(min(zd1 + 1, k - 1 + kNSTAGE)); // (what warp 0 had issued)
+        return false;
     }
     // every load of this tile was waited for: carry the parities over to the next tile
     phase = par;
@@ -1675,7 +1717,7 @@ template <int Q, typename S, int W, bool kTMA, int kFeat>
 __global__ void __launch_bounds__(16 * W, W <= 8 ? 2 : 1) step_kernel(const __grid_constant__ StepParams P,
                                                                       const __grid_constant__ TensorMaps T) {
     unsigned char* smem = aligned_smem_base();
-    init_stage_barriers(smem);
+    init_barriers<W / 2>(smem);
     uint32_t phase = 0;
     if constexpr ((kFeat & (F_WALL | F_INOUT)) != 0) {
         if (tile_is_interior<W>(P, blockIdx.x, blockIdx.y, blockIdx.z)) {

@@ -685,7 +685,7 @@ template <int Q, typename S, int W>
 __global__ void __launch_bounds__(32 * W, W <= 8 ? 2 : 1) step_kernel(const __grid_constant__ StepParams P,
                                                                       const __grid_constant__ TensorMaps T) {
     unsigned char* smem = aligned_smem_base();
-    init_stage_barriers(smem);
+    init_barriers<0>(smem);
     uint32_t phase = 0;
     tile<Q, S, W>(P, T.m, blockIdx.x, blockIdx.y, blockIdx.z, P.step, smem, phase);
 }
