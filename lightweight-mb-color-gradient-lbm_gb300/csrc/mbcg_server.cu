@@ -111,6 +111,10 @@ struct Staging {
     bool pending = false;
 };
 
+constexpr int kResultDoubles = kDiagSlots + 2; // of one request's record: diagnostics, hash, status
+constexpr size_t kResultSlab = 512;             // records an allocation
+constexpr size_t kFetchKeep = size_t(64) << 20;
+
 struct Request {
     int64_t id = 0;
     mbcg_params p{};
@@ -186,6 +190,15 @@ struct mbcg_server {
     // statistics
     int64_t submitted = 0, completed = 0, failed = 0, node_updates = 0, compositions = 0, replays = 0;
     double first_admit = -1, last_done = -1;
+
+    // pinned result records of the requests, kResultSlab to an allocation (guarded by mu)
+    std::vector<double*> result_slabs;
+    size_t results_used = 0;
+
+    // device staging of fetched results, one fetch at a time; kept up to kFetchKeep bytes
+    std::mutex io_mu;
+    float* fetch_stage = nullptr;
+    size_t fetch_cap = 0;
 
     double now() const {
         return std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -720,8 +733,10 @@ void worker_main(mbcg_server* s) {
             fail_all(s, std::string("batch replay: ") + cudaGetErrorString(e));
             break;
         }
-        // at most two replays in flight
-        while (s->inflight.size() > 2) {
+        // At most two replays in flight, one running and one queued behind it: requests join at a replay's
+        // start.  With one more, the first of eight requests that came together ran all its 48 steps
+        // before the others joined.
+        while (s->inflight.size() > 1) {
             cudaEvent_t ev = s->inflight.front();
             lk.unlock();
             e = cudaEventSynchronize(ev);
@@ -882,8 +897,9 @@ void destroy_server(mbcg_server* s) {
     if (s->st) cudaStreamSynchronize(s->st);
     for (auto& kv : s->reqs) {
         if (kv.second->done_ev) cudaEventDestroy(kv.second->done_ev);
-        if (kv.second->h_result) cudaFreeHost(kv.second->h_result);
     }
+    for (double* slab : s->result_slabs) cudaFreeHost(slab);
+    if (s->fetch_stage) cudaFree(s->fetch_stage);
     if (s->exec) cudaGraphExecDestroy(s->exec);
     for (Staging* ring : {s->chunk_stage, s->tile_stage, s->case_stage})
         for (int i = 0; i < kRing; ++i) {
@@ -1033,15 +1049,17 @@ int mbcg_server_submit(mbcg_server* s, const mbcg_params* p, int64_t nsteps, int
     auto r = std::make_unique<Request>();
     r->p = *p;
     r->steps = nsteps;
-    if (cudaMallocHost(&r->h_result, sizeof(double) * (kDiagSlots + 2)) != cudaSuccess)
-        return fail(MBCG_E_NOMEM, "pinned result buffer");
-    std::memset(r->h_result, 0, sizeof(double) * (kDiagSlots + 2));
     {
         std::lock_guard<std::mutex> lk(s->mu);
-        if (!s->fatal.empty()) {
-            cudaFreeHost(r->h_result);
-            return fail(MBCG_E_CUDA, "server failed: " + s->fatal);
+        if (!s->fatal.empty()) return fail(MBCG_E_CUDA, "server failed: " + s->fatal);
+        if (s->results_used == s->result_slabs.size() * kResultSlab) {
+            double* slab = nullptr;
+            if (cudaMallocHost(&slab, sizeof(double) * kResultDoubles * kResultSlab) != cudaSuccess)
+                return fail(MBCG_E_NOMEM, "pinned result buffer");
+            std::memset(slab, 0, sizeof(double) * kResultDoubles * kResultSlab);
+            s->result_slabs.push_back(slab);
         }
+        r->h_result = s->result_slabs.back() + (s->results_used++ % kResultSlab) * kResultDoubles;
         r->id = s->next_id++;
         r->t_submit = s->now();
         *id = r->id;
@@ -1095,6 +1113,53 @@ int mbcg_server_drain(mbcg_server* s, double timeout_s) {
     return MBCG_OK;
 }
 
+// The 11 dense fields of a result into host memory: one kernel converts them all into a device staging
+// area, and one copy takes them where the caller's (pageable) fields lie end to end, one copy a field
+// elsewhere.  A field at a time through an area allocated and freed for the call took 200 us for a result of
+// 1 to 4 MB, and the free waited for the other requests' steps; 65 to 90 us now.  Results above kFetchKeep go
+// two fields at a time through an area of their own.
+static cudaError_t fetch_fields(mbcg_server* s, const mbcg_params& p, const StepParams& P, float* const host[NF]) {
+    const size_t n = static_cast<size_t>(p.nx) * p.ny * p.nz, bytes = n * sizeof(float);
+    if (NF * bytes > kFetchKeep) {
+        float* area = nullptr;
+        cudaError_t e = cudaMalloc(&area, 2 * bytes);
+        for (int i = 0; i < NF && e == cudaSuccess; ++i) {
+            float* buf = area + (i & 1) * n;
+            e = launch_to_dense(p.precision, P, i, buf, s->st_io);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(host[i], buf, bytes, cudaMemcpyDeviceToHost, s->st_io);
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s->st_io);
+        if (area) cudaFree(area);
+        return e;
+    }
+    bool joined = true;
+    for (int i = 0; i < NF && joined; ++i) {
+        cudaPointerAttributes a{};
+        joined = host[i] == host[0] + i * n && cudaPointerGetAttributes(&a, host[i]) == cudaSuccess &&
+                 a.type == cudaMemoryTypeUnregistered;
+    }
+    cudaGetLastError(); // (a failed query is no error of the fetch)
+    std::lock_guard<std::mutex> io(s->io_mu);
+    cudaError_t e = cudaSuccess;
+    if (s->fetch_cap < NF * bytes) {
+        if (s->fetch_stage) cudaFree(s->fetch_stage);
+        s->fetch_stage = nullptr;
+        s->fetch_cap = 0;
+        e = cudaMalloc(&s->fetch_stage, NF * bytes);
+        if (e != cudaSuccess) return e;
+        s->fetch_cap = NF * bytes;
+    }
+    float* dev[NF];
+    for (int i = 0; i < NF; ++i) dev[i] = s->fetch_stage + i * n;
+    e = launch_state_to_host(p.precision, P, dev, s->st_io);
+    const int copies = joined ? 1 : NF;
+    for (int i = 0; i < copies && e == cudaSuccess; ++i)
+        e = cudaMemcpyAsync(host[i], dev[i], joined ? NF * bytes : bytes, cudaMemcpyDeviceToHost, s->st_io);
+    // also after an error: the next fetch reuses the area
+    const cudaError_t done = cudaStreamSynchronize(s->st_io);
+    return e != cudaSuccess ? e : done;
+}
+
 int mbcg_server_fetch(mbcg_server* s, int64_t id, float* const host[MBCG_NFIELDS]) {
     if (!s || !host) return fail(MBCG_E_INVALID, "null argument");
     std::unique_lock<std::mutex> lk(s->mu);
@@ -1107,17 +1172,7 @@ int mbcg_server_fetch(mbcg_server* s, int64_t id, float* const host[MBCG_NFIELDS
     const mbcg_params p = r.p;
     r.fetching += 1; // release waits until this copy is done
     lk.unlock();
-    // one dense field per transfer through a dense device field (see mbcg_copy_out)
-    const size_t n = static_cast<size_t>(p.nx) * p.ny * p.nz;
-    float* staging = nullptr;
-    cudaError_t e = cudaMalloc(&staging, 2 * n * sizeof(float));
-    for (int i = 0; i < NF && e == cudaSuccess; ++i) {
-        float* buf = staging + (i & 1) * n;
-        e = launch_to_dense(p.precision, P, i, buf, s->st_io);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(host[i], buf, n * sizeof(float), cudaMemcpyDeviceToHost, s->st_io);
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s->st_io);
-    if (staging) cudaFree(staging);
+    const cudaError_t e = fetch_fields(s, p, P, host);
     lk.lock();
     r.fetching -= 1;
     s->cv_done.notify_all();
