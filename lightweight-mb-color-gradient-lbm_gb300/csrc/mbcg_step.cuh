@@ -162,6 +162,11 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src, bool valid
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// Programmatic dependent launch: lets the next kernel of the stream start its set-up once every CTA of
+// this one has begun, and waits for the kernel before this one to be complete.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ int floor8(int v) { return v & ~7; }
 
 // ------------------------------------------------------------------ coordinate roles
@@ -770,7 +775,8 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
     const bool has_col = col_n <= kPSX - 2, has_row = row_n <= W;
     const int nframe = 2 * kPSX + 2 * W + (has_col ? W + 2 : 0) + (has_row ? kPSX : 0);
     auto build_frame = [&]() {
-        for (int e = tid; e < nframe; e += kThreads) {
+        constexpr int kSkip = kTMA ? 32 : 0; // (warp 0 starts the copies)
+        for (int e = tid - kSkip; e < nframe; e += kThreads - kSkip) {
             int r, c, i = e;
             if (i < 2 * kPSX) {
                 r = i < kPSX ? 0 : W + 1;
@@ -886,10 +892,12 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
     // ---- set-up ------------------------------------------------------------------
     // every thread is done with the previous tile's shared memory before it is refilled
     __syncthreads();
-    for (int k = kfirst; k < kfirst + kNSTAGE; ++k) issue(k, k - kfirst);
     if (tid < 2) fcount[tid] = 0;
     __syncthreads();
-    build_frame();
+    // no state is read before the kernel that wrote it is complete
+    if (!kTMA || w != 0) build_frame();
+    wait_prior_grid();
+    for (int k = kfirst; k < kfirst + kNSTAGE; ++k) issue(k, k - kfirst);
     if constexpr (!kTMA) {
         cp_async_wait_all();
         __syncthreads();
@@ -1769,6 +1777,7 @@ template <int Q, typename S, int W, bool kTMA, int kFeat>
 __global__ void __launch_bounds__(16 * W, W <= 8 ? 2 : 1) step_kernel(const __grid_constant__ StepParams P,
                                                                       const __grid_constant__ TensorMaps T) {
     unsigned char* smem = aligned_smem_base();
+    launch_dependents();
     init_barriers<W / 2>(smem);
     uint32_t phase = 0;
     if constexpr ((kFeat & (F_WALL | F_INOUT)) != 0) {
@@ -1795,6 +1804,26 @@ cudaError_t configure_once(K kern, int smem, std::atomic<unsigned long long>& do
     return e;
 }
 
+// Launch as a programmatic dependent of the kernel before it in the stream: that one's last CTAs, the launch
+// itself and this kernel's set-up overlap.  Every CTA waits for the prior grid before it touches a state, so
+// a grid is complete only when all before it are.  Measured a step: 32^3 18.8 -> 16.4 us, 64^3 D3Q19 24.7 ->
+// 23.2 us, 128^3 jet 114 -> 111 us, 192^3 247 -> 245 us.  (The batch kernels gain nothing: their launches
+// run side by side, and a CTA that waits holds an SM another kind could use, 3.5 -> 3.7 ms for 8 requests.)
+template <typename... Par, typename... Arg>
+cudaError_t launch_pdl(void (*kern)(Par...), dim3 grid, dim3 block, int smem, cudaStream_t s, const Arg&... arg) {
+    cudaLaunchAttribute pdl{};
+    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &pdl;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, arg...);
+}
+
 template <int Q, typename S, int W, bool kTMA, int kFeat>
 cudaError_t launch_one(const StepParams& P, const TensorMaps& T, cudaStream_t s) {
     using G = Geo<S, W>;
@@ -1805,8 +1834,7 @@ cudaError_t launch_one(const StepParams& P, const TensorMaps& T, cudaStream_t s)
     L.zchunk = std::min(L.zchunk, max_zchunk(L.plane, static_cast<int>(sizeof(S))));
     dim3 block(32, W / 2, 1);
     dim3 grid((L.nx - 2 + kTX - 1) / kTX, (L.ny - 2 + W - 3) / (W - 2), z_tiles(L.nz, L.bc[2], L.zchunk));
-    kern<<<grid, block, G::smem, s>>>(L, T);
-    return cudaGetLastError();
+    return launch_pdl(kern, grid, block, G::smem, s, L, T);
 }
 
 // Feature set: the smallest instantiation covering the lattice (TMA path); the plain-load

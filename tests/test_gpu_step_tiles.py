@@ -108,3 +108,23 @@ def test_pure_nodes_keep_their_colour_in_16_bits(precision):
             s = c.copy_out()[:, 1:-1, 1:-1, 1:-1].astype(np.float64)
         phi.append((s[0] - s[1]) / (s[0] + s[1]))
     assert np.abs(phi[0] - phi[1]).max() < 2.0 * (2.0 ** -10 if precision == mbcg.FP16 else 2.0 ** -7)
+
+
+@pytest.mark.parametrize("precision", [mbcg.FP32, mbcg.FP16])
+@pytest.mark.parametrize("size", [(30, 22, 12), (125, 90, 40), (61, 45, 300)])  # one, some, many tiles at once
+def test_steps_in_a_row_are_the_steps_one_by_one(size, precision):
+    """Steps queued behind each other start their set-up before the one in front is complete: the state
+    has to be that of steps each waited for (bit for bit: the arithmetic is the same)."""
+    p = make("inout", 2, 27, size)
+    p.precision = precision
+    got = []
+    for alone in (False, True):
+        with mbcg.Case(p) as c:
+            c.init()
+            for n in [1] * 24 if alone else [24]:
+                c.step(n)
+                if alone:
+                    assert c.status() == 0  # (waits for the device)
+            assert c.status() == 0
+            got.append(c.copy_out())
+    assert np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))
