@@ -163,7 +163,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // Programmatic dependent launch: lets the next kernel of the stream start its set-up once every CTA of
-// this one has begun, and waits for the kernel before this one to be complete.
+// this one has said so or is done, and waits for the kernel before this one to be complete.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -1531,8 +1531,12 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
         // slot of plane k (whose fields everyone has read) and prepares the psi frame of plane k+2
         const int d = k - 1;
         if (w == 0) {
-            if constexpr (kTMA)
+            if constexpr (kTMA) {
+                // Nothing more to stage: the next step's CTAs may take the SMs that fall idle (from the start
+                // of the kernel they took them in another order: D3Q19 RTI 61^2x243, 8 steps, 493 against 510 us).
                 if (k + kNSTAGE <= zd1 + 1) issue(k + kNSTAGE, sl);
+                else launch_dependents();
+            }
             const int sl2 = nxt(sl_next);
             if (k + 2 <= zd1 + 1 && peek_slot(sl2)) fill_frame(mz2, inbox2, sl2);
         } else {
@@ -1777,7 +1781,6 @@ template <int Q, typename S, int W, bool kTMA, int kFeat>
 __global__ void __launch_bounds__(16 * W, W <= 8 ? 2 : 1) step_kernel(const __grid_constant__ StepParams P,
                                                                       const __grid_constant__ TensorMaps T) {
     unsigned char* smem = aligned_smem_base();
-    launch_dependents();
     init_barriers<W / 2>(smem);
     uint32_t phase = 0;
     if constexpr ((kFeat & (F_WALL | F_INOUT)) != 0) {
@@ -1806,8 +1809,8 @@ cudaError_t configure_once(K kern, int smem, std::atomic<unsigned long long>& do
 
 // Launch as a programmatic dependent of the kernel before it in the stream: that one's last CTAs, the launch
 // itself and this kernel's set-up overlap.  Every CTA waits for the prior grid before it touches a state, so
-// a grid is complete only when all before it are.  Measured a step: 32^3 18.8 -> 16.4 us, 64^3 D3Q19 24.7 ->
-// 23.2 us, 128^3 jet 114 -> 111 us, 192^3 247 -> 245 us.  (The batch kernels gain nothing: their launches
+// a grid is complete only when all before it are.  Measured a step: 32^3 18.8 -> 16.1 us, 64^3 D3Q19 24.7 ->
+// 22.9 us, 128^3 jet 114 -> 111 us, 192^3 247 -> 245 us.  (The batch kernels gain nothing: their launches
 // run side by side, and a CTA that waits holds an SM another kind could use, 3.5 -> 3.7 ms for 8 requests.)
 template <typename... Par, typename... Arg>
 cudaError_t launch_pdl(void (*kern)(Par...), dim3 grid, dim3 block, int smem, cudaStream_t s, const Arg&... arg) {
