@@ -266,8 +266,8 @@ int mbcg_checkpoint_load(const char *path, mbcg_case **out);
 
 /* ---- launch shape (no counterpart in the reference, whose block is the compile-time
  * 32x4x2 of compile.sh:34-36) --------------------------------------------------------- */
-/* Step CTA shape: block_rows warps (8 or 16) of 32 lanes; zchunk destination planes per CTA
- * along z.  mbcg_create picks a shape from a wave-filling model, or the shape an earlier
+/* Step CTA shape: block_rows names it (16: 24 source rows, 12 warps, one CTA per SM; 8: 8 rows,
+ * 4 warps, two per SM); zchunk destination planes per CTA along z.  mbcg_create picks a shape from a wave-filling model, or the shape an earlier
  * mbcg_autotune measured for the same lattice, precision, sizes and boundary features. */
 int mbcg_get_shape(const mbcg_case *c, int32_t *block_rows, int32_t *zchunk);
 int mbcg_set_shape(mbcg_case *c, int32_t block_rows, int32_t zchunk);

@@ -33,7 +33,7 @@ struct BatchCase {
     int pad[15];
 };
 
-// One unit of the flat tile queue: a (30 x 14 x zchunk) tile of the lattice in slot `slot`.
+// One unit of the flat tile queue: a (30 x 22 x zchunk) tile of the lattice in slot `slot`.
 struct BatchTile {
     uint16_t slot, bx, by, bz;
 };
@@ -48,7 +48,7 @@ struct ChunkState {
 
 constexpr int kBatchW = kStepW; // shape of the batch kernel's CTAs (step_rows)
 // Lattices resident at once: the batch kernel reads each one's step parameters (both parities)
-// from a constant-memory table of this many slots (2 x 64 x 392 bytes), as uniform loads the
+// from a constant-memory table of this many slots (2 x 64 x 408 bytes), as uniform loads the
 // instructions take as operands, where a copy in shared memory costs a load into a register per use.
 constexpr int kBatchParamSlots = 64;
 // Copies n slots' parameters (StepParams[n][2], host memory valid until the copy has executed)

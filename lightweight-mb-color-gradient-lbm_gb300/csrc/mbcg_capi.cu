@@ -124,12 +124,13 @@ void fill_physics(const mbcg_params& p, StepParams& P) {
     P.ghost_images = 1;
 }
 
-// source rows of the CTAs that step this lattice in shape W
-int case_rows(const mbcg_params& p, int W) {
+bool case_pop(const mbcg_params& p) {
     StepParams P;
     fill_physics(p, P);
-    return uses_pop(p.precision != MBCG_FP32, features_of(P)) ? W : step_rows(W);
+    return uses_pop(p.precision, features_of(P));
 }
+// source rows of the CTAs that step this lattice in shape W
+int case_rows(const mbcg_params& p, int W) { return case_pop(p) ? W : step_rows(W); }
 
 int choose_zchunk(const mbcg_params& p, int W) {
     if (const char* env = std::getenv("MBCG_ZCHUNK")) {
@@ -149,7 +150,7 @@ int choose_zchunk(const mbcg_params& p, int W) {
     // fill what the last wave leaves idle.  Small lattices get thin tiles this way (32^3: depth 1, 18.5 us
     // a step against 43 at depth 8).
     constexpr long long kExtra = 3;
-    const int nzf = p.nz - 2, cap = z_cap(p.nz, p.bc[2]), inner = nzf - 2 * cap;
+    const int nzf = p.nz - 2, cap = case_pop(p) ? 0 : z_cap(p.nz, p.bc[2]), inner = nzf - 2 * cap;
     const long long thin = cap ? 2 * g : 0, thin_cost = cap + kExtra;
     long long best = -1;
     int best_chunk = inner;

@@ -20,9 +20,11 @@ namespace mbcg {
 constexpr int kStepW = 16;
 constexpr int kStepWSmall = 8;
 constexpr int step_rows(int w) { return w == kStepWSmall ? 8 : 24; }
-// Fully periodic, unforced lattices in 16-bit storage step by populations, one node a thread, w source
-// rows (the reason stands in mbcg_step_pop.cuh).
-constexpr bool uses_pop(bool storage16, int features) { return storage16 && features == 0; }
+// Lattices in BF16 storage without an inlet, and in FP16 storage fully periodic and unforced ones, step by
+// populations, one node a thread, w source rows (the reason stands in mbcg_step_pop.cuh).
+constexpr bool uses_pop(int precision, int features) {
+    return precision == MBCG_BF16 ? (features & F_INOUT) == 0 : precision == MBCG_FP16 && features == 0;
+}
 constexpr int kStepTileX = 30; // destination columns per tile
 constexpr int kStepRBX = 48;   // staged width of the rhor / rhob boxes
 constexpr int kStepMX = 40;    // staged width of the other nine boxes

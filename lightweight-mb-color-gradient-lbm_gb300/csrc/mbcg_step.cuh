@@ -1847,10 +1847,11 @@ cudaError_t launch_w(bool tma, const StepParams& P, const TensorMaps& T, cudaStr
     if (!tma) return launch_one<Q, S, W, false, F_ALL>(P, T, s);
     if (std::getenv("MBCG_ALL_FEATURES")) return launch_one<Q, S, W, true, F_ALL>(P, T, s); // (parity tests)
     const int f = features_of(P);
-    if constexpr (sizeof(S) == 4) // (the 16-bit forms step such lattices by populations)
+    if constexpr (sizeof(S) == 4) // (for what the 16-bit forms step by populations, see uses_pop)
         if (f == 0) return launch_one<Q, S, W, true, 0>(P, T, s);
     if (f == F_INOUT) return launch_one<Q, S, W, true, F_INOUT>(P, T, s);
-    if ((f & F_INOUT) == 0) return launch_one<Q, S, W, true, F_WALL | F_FORCE>(P, T, s); // walls, force
+    if constexpr (!std::is_same<S, __nv_bfloat16>::value)
+        if ((f & F_INOUT) == 0) return launch_one<Q, S, W, true, F_WALL | F_FORCE>(P, T, s); // walls, force
     return launch_one<Q, S, W, true, F_ALL>(P, T, s);
 }
 

@@ -1,11 +1,13 @@
-// mbcg_step_pop.cuh -- the step of fully periodic, unforced lattices in the 16-bit storage forms, by
-// populations.
+// mbcg_step_pop.cuh -- the step by populations: of lattices in BF16 storage without an inlet, and of fully
+// periodic unforced ones in FP16 storage.
 //
-// step_tile() (mbcg_step.cuh) is faster (1.3x on a 192^3 drop) and nearer to the exact step.  These
-// lattices keep this kernel for what they store: the density slot of a drop in equal-density fluids holds
-// (rho - 1) / 0.01 with rho - 1 around 1e-6, so the FP32 rounding of the density sum, 1e-7, is 1 to 7 % of
-// the slot (64^3 to 200^3), and another order of summation changes stored states by that much.  With a
-// boundary, a force or a density ratio the slot is 10 to 1000 times larger and they agree to 1e-4.
+// step_tile() (mbcg_step.cuh) is faster (1.3x on a 192^3 drop, 1.07x on small walled ones) and nearer to the
+// exact step.  These lattices keep this kernel for what they store.  The density slot of a drop in
+// equal-density fluids holds (rho - 1) / 0.01 with rho - 1 around 1e-6, so the FP32 rounding of the density
+// sum, 1e-7, is 1 to 7 % of the slot (64^3 to 200^3), and another order of summation changes stored states by
+// that much.  With a density ratio a last bit of FP32 now and then rounds a colour slot the other way (three
+// nodes in 10^6); beside such a node the stress of the next step is up to 1.7 times the field's mean away
+// in BF16, 0.3 times in FP16 (RTI).  With an inlet states agree to 6e-4 (BF16) after two steps.
 //
 // Each source evaluates all Q populations of its coefficient tensor with a separable inverse transform (x, y,
 // then z); they stream to the neighbouring lanes by shuffles, to the neighbouring rows through shared memory and
@@ -46,14 +48,19 @@ struct Geo {
 struct Coef {
     float p000, p100, p010, p001, p200, p020, p002, p110, p101, p011;
     float p210, p201, p120, p102, p021, p012, p111;
+    float r0; // extra on the rest population (density ratio)
 };
 
-// Equilibrium (pdf.cuh:16-36) + oms * regularised non-equilibrium (pdf.cuh:38-79), as the coefficients
-// of a polynomial in c (w_i factored out).
-__device__ __forceinline__ void build_coef(const StepParams& P, Coef& c, float rho, float ux, float uy, float uz,
-                                           float pxx, float pxy, float pyy, float pyz, float pzz, float pxz) {
-    const float oms = P.oms;
+// Equilibrium (pdf.cuh:16-36) + oms * regularised non-equilibrium (pdf.cuh:38-79) + 1/2 Guo force
+// (pdf.cuh:94-136) + density-ratio rest term, as the coefficients of a polynomial in c (w_i factored out).
+template <int kFeat>
+__device__ __forceinline__ void build_coef(const StepParams& P, Coef& c, float rho, float rr, float rb, float ux,
+                                           float uy, float uz, float pxx, float pxy, float pyy, float pyz, float pzz,
+                                           float pxz) {
     const float vx = ux, vy = uy, vz = uz;
+    float oms = P.oms;
+    if constexpr ((kFeat & F_FORCE) != 0)
+        if (P.tau_var) oms = 1.0f - 1.0f / tau_eff_of(P, rr, rb);
     const float usq = ux * ux + uy * uy + uz * uz;
     const float rux = rho * ux, ruy = rho * uy, ruz = rho * uz;
     const float t1 = 3.0f - 4.5f * usq;
@@ -84,6 +91,40 @@ __device__ __forceinline__ void build_coef(const StepParams& P, Coef& c, float r
     c.p021 = 13.5f * ruy * uy * uz + o135 * a3yyz;
     c.p012 = 13.5f * ruy * uz * uz + o135 * a3yzz;
     c.p111 = 27.0f * rux * uy * uz + 2.0f * o135 * a3xyz;
+    c.r0 = 0.0f;
+    if constexpr ((kFeat & F_FORCE) == 0) return;
+    if (P.forced) {
+        const float Fx = rho * P.g[0], Fy = rho * P.g[1], Fz = rho * P.g[2];
+        const float Gxxy = Fx * ux * uy + 0.5f * Fy * ux * ux;
+        const float Gxxz = Fx * ux * uz + 0.5f * Fz * ux * ux;
+        const float Gxyy = Fy * ux * uy + 0.5f * Fx * uy * uy;
+        const float Gxzz = Fz * ux * uz + 0.5f * Fx * uz * uz;
+        const float Gyyz = Fy * uy * uz + 0.5f * Fz * uy * uy;
+        const float Gyzz = Fz * uy * uz + 0.5f * Fy * uz * uz;
+        const float Gxyz = Fx * uy * uz + Fy * ux * uz + Fz * ux * uy;
+        c.p000 -= 1.5f * (Fx * ux + Fy * uy + Fz * uz);
+        c.p100 += 1.5f * Fx - 4.5f * (Gxyy + Gxzz);
+        c.p010 += 1.5f * Fy - 4.5f * (Gxxy + Gyzz);
+        c.p001 += 1.5f * Fz - 4.5f * (Gxxz + Gyyz);
+        c.p200 += 4.5f * Fx * ux;
+        c.p020 += 4.5f * Fy * uy;
+        c.p002 += 4.5f * Fz * uz;
+        c.p110 += 4.5f * (Fx * uy + Fy * ux);
+        c.p101 += 4.5f * (Fx * uz + Fz * ux);
+        c.p011 += 4.5f * (Fy * uz + Fz * uy);
+        c.p210 += 13.5f * Gxxy;
+        c.p201 += 13.5f * Gxxz;
+        c.p120 += 13.5f * Gxyy;
+        c.p102 += 13.5f * Gxzz;
+        c.p021 += 13.5f * Gyyz;
+        c.p012 += 13.5f * Gyzz;
+        c.p111 += 13.5f * Gxyz;
+    }
+    if (P.ratio) {
+        const float K = rr * P.kappa_r + rb * P.kappa_b;
+        c.p000 += K;
+        c.r0 -= K;
+    }
 }
 
 // ------------------------------------------------------------------ accumulators
@@ -117,8 +158,20 @@ __device__ __forceinline__ Tri operator+(Tri a, Tri b) { return Tri{__fadd2_rn(a
 __device__ __forceinline__ Tri operator-(Tri a, Tri b) { return Tri{mbcg::operator-(a.o, b.o), a.c - b.c}; }
 __device__ __forceinline__ Tri operator+(Tri a, float s) { return Tri{__fadd2_rn(a.o, pair(s)), a.c + s}; }
 
+// add one population of velocity (ex, ey, ez) to a destination's moment sums
+__device__ __forceinline__ void add_pop(Acc& a, float g, float r, int ex, int ey, int ez) {
+    a.rr.x += g;
+    a.rr.y += r;
+    if (ex) { a.jxx.x += ex * g; a.jxx.y += g; }
+    if (ey) { a.jy += ey * g; a.yy += g; }
+    if (ez) { a.jz += ez * g; a.zz += g; }
+    if (ex && ey) a.xy += ex * ey * g;
+    if (ey && ez) a.yz += ey * ez * g;
+    if (ex && ez) a.xz += ex * ez * g;
+}
+
 // one tile (30 columns x (W-2) rows x zchunk planes), arguments as step_tile's
-template <int Q, typename S, int W>
+template <int Q, typename S, int W, int kFeat>
 __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* maps, int bx, int by, int bz, long long step,
                                      unsigned char* smem, uint32_t& phase) {
     using G = Geo<S, W>;
@@ -146,12 +199,21 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
     const int bM = w * kMX + lane + offM;         // this node in the other boxes
 
     const bool dest_thread = lane >= 1 && lane <= kTX && w >= 1 && w <= W - 2 && xs <= nx - 2 && ys <= ny - 2;
-    const bool in_xy = xs <= nx - 1 && ys <= ny - 1;
+    const int rx = axis_role<kFeat>(P, 0, xs, nx);
+    const int ry = axis_role<kFeat>(P, 1, ys, ny);
+    const bool in_xy = rx != R_OUT && ry != R_OUT;
+    // the node's role, given the role of its plane
+    auto role_of = [&](int rz) -> int {
+        if (rx == R_OUT || ry == R_OUT || rz == R_OUT) return R_OUT;
+        if ((kFeat & F_WALL) && (rx == R_WALL || ry == R_WALL || rz == R_WALL)) return R_WALL;
+        return R_FLUID;
+    };
+    const int role_xy = role_of(R_FLUID); // on fluid planes
     // stochastic rounding of the 16-bit stores: key base of this step
     const unsigned key_base = round_key_base(P.seed, step);
-    // periodic images of this column's store (x = 1 / nx-2, y = 1 / ny-2)
-    const int img_x = xs == 1 ? nx - 1 : (xs == nx - 2 ? 0 : -1);
-    const int img_y = ys == 1 ? ny - 1 : (ys == ny - 2 ? 0 : -1);
+    // periodic images of this column's store (x = 1 / nx-2, y = 1 / ny-2 on a periodic axis)
+    const int img_x = P.bc[0] == MBCG_BC_PERIODIC ? (xs == 1 ? nx - 1 : (xs == nx - 2 ? 0 : -1)) : -1;
+    const int img_y = P.bc[1] == MBCG_BC_PERIODIC ? (ys == 1 ? ny - 1 : (ys == ny - 2 ? 0 : -1)) : -1;
 
     // psi fill: each thread owns <= kPsiPer ring elements; their mapping never changes along z.
     // Each element reads the staged box at the node whose stored value equals psi there (the
@@ -177,9 +239,10 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
                 psi_box[j] = 0;
                 continue;
             }
-            const int mx = periodic_image(gx, nx), my = periodic_image(gy, ny);
-            const int dx = gx >= 0 && gx <= nx - 1 ? gx : mx;
-            const int dy = gy >= 0 && gy <= ny - 1 ? gy : my;
+            const int mx = psi_coord(P, 0, gx, nx), my = psi_coord(P, 1, gy, ny);
+            const bool px = P.bc[0] == MBCG_BC_PERIODIC, py = P.bc[1] == MBCG_BC_PERIODIC;
+            const int dx = (px && gx >= 0 && gx <= nx - 1) ? gx : mx;
+            const int dy = (py && gy >= 0 && gy <= ny - 1) ? gy : my;
             const int bc_ = dx - xr0, br_ = dy - (yb - 1);
             psi_box[j] = (bc_ >= 0 && bc_ < kRBX && br_ >= 0 && br_ < G::RBY) ? br_ * kRBX + bc_ : -1;
             psi_g[j] = static_cast<long long>(my) * P.pitch + mx;
@@ -201,7 +264,7 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
     auto m_box = [&](unsigned char* st, int f) -> S* {
         return reinterpret_cast<S*>(st + 2 * G::rb_field + (f - 2) * G::m_field);
     };
-    auto zload = [&](int k) -> int { return periodic_image(k, nz); };
+    auto zload = [&](int k) -> int { return data_coord(P, 2, k, nz); };
 
     // ---- stage loader -------------------------------------------------------------
     auto issue = [&](int k, int sl) {
@@ -250,10 +313,10 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
                 pf1[j] = Codec<S>::to_f(static_cast<const S*>(P.a[1])[zo + psi_g[j]]);
             }
     };
-    // mz: the staged plane
-    auto fill_psi = [&](int mz, int sl, bool prefetched) {
+    // mz: the plane the colour-gradient rule maps k to; plane_in_box: it is the staged plane
+    auto fill_psi = [&](int mz, bool plane_in_box, int sl, bool prefetched) {
         float* ring = psi_ring + sl * G::psi_plane;
-        if (!far_any) {
+        if (plane_in_box && !far_any) {
             // every element of this tile is in the staged box (the first one of each thread
             // always exists: the ring plane has at least 32 W elements)
             unsigned char* st = stage_at(sl);
@@ -273,7 +336,7 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
         for (int j = 0; j < kPsiPer; ++j) {
             if (psi_box[j] == -2) continue;
             float v;
-            if (psi_box[j] >= 0) {
+            if (plane_in_box && psi_box[j] >= 0) {
                 v = psi_of<S>(P, r0b[psi_box[j]], r1b[psi_box[j]]);
             } else if (prefetched && psi_box[j] == -1) {
                 v = psi_of_slots<S>(pf0[j], pf1[j]);
@@ -306,10 +369,11 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
         }
     }
     {
-        fill_psi(zload(kfirst), 0, false);
-        fill_psi(zload(kfirst + 1), 1, false);
+        const int m0 = psi_coord(P, 2, kfirst, nz), m1 = psi_coord(P, 2, kfirst + 1, nz);
+        fill_psi(m0, m0 == zload(kfirst), 0, false);
+        fill_psi(m1, m1 == zload(kfirst + 1), 1, false);
     }
-    if (far_any) prefetch_psi(zload(kfirst + 2));
+    if (far_any) prefetch_psi(psi_coord(P, 2, kfirst + 2, nz));
 
     Acc accP, accC, accN; // destination planes k-1, k, k+1
     accP.zero();
@@ -321,32 +385,51 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
 
     int sl = 1; // slot of plane k (k starts at kfirst + 1)
     int k = zd0 - 1;
-    for (; k <= zd1; ++k, sl = nxt(sl)) {
+    // One plane of the z-march with the feature set kFB: the tile's own, or, between the walls of a z
+    // axis, the same set without their part.  Returns false after a bail.
+    auto plane = [&](auto featc) -> bool {
+        constexpr int kFB = decltype(featc)::value;
         const int sl_next = nxt(sl), sl_prev = prv(sl);
         // (1) psi of plane k+1; one barrier both publishes the ring and makes the bail decision
         // uniform (a plane that never arrived leaves garbage in the ring, which nobody reads)
-        const bool zid = k >= 1 && k + kNSTAGE - 1 <= nz - 2; // planes k .. k+3 are fluid planes
+        // Plane coordinates: every mapping (staging, colour-gradient rule, node role) is the
+        // identity while planes k .. k+3 are fluid planes, which is almost every plane.
+        const bool zid = k >= 1 && k + kNSTAGE - 1 <= nz - 2;
+        int mz1 = k + 1, mz2 = k + 2, rz = R_FLUID;
+        bool inbox1 = true;
+        if (!zid) {
+            mz1 = psi_coord(P, 2, k + 1, nz);
+            inbox1 = mz1 == zload(k + 1);
+            mz2 = psi_coord(P, 2, k + 2, nz);
+            rz = axis_role<kFB>(P, 2, k, nz);
+        }
         {
             const bool ok = wait_slot(k + 1, sl_next);
-            if (ok) fill_psi(zid ? k + 1 : zload(k + 1), sl_next, true);
+            if (ok) fill_psi(mz1, inbox1, sl_next, true);
             if (__syncthreads_or(!ok)) {
                 bail(k_issued);
                 return false;
             }
         }
-        if (far_any && k + 2 <= zd1 + 1) prefetch_psi(zid ? k + 2 : zload(k + 2));
+        if (far_any && k + 2 <= zd1 + 1) prefetch_psi(mz2);
         // (2) prefetch plane k+3 into the slot plane k-1 used
         if (k + kNSTAGE - 1 <= zd1 + 1 && k + kNSTAGE - 1 > k_issued) {
             issue(k + kNSTAGE - 1, sl_prev);
             k_issued = k + kNSTAGE - 1;
+        } else {
+            launch_dependents(); // nothing more to stage
         }
 
         // (3) this thread's source node at plane k
-        // (sources outside the lattice only ever stream into nodes that are not destinations of this
-        // tile, so every source is processed branch-free)
+        const int role = zid ? role_xy : role_of(rz);
+        // Sources outside the lattice (lanes / rows past the last ghost layer) only ever stream
+        // into nodes that are not destinations of this tile, so without walls every source is
+        // processed branch-free; wall ghost layers hold data and must not emit.
+        const bool active = ((kFB & F_WALL) == 0) || role == R_FLUID;
+
         unsigned char* st = stage_at(sl);
         Node<S> nd{};
-        {
+        if (active) {
             float v[NF];
             v[0] = Codec<S>::to_f(rb_box(st, 0)[bR]);
             v[1] = Codec<S>::to_f(rb_box(st, 1)[bR]);
@@ -354,17 +437,25 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
             for (int f = 2; f < NF; ++f) v[f] = Codec<S>::to_f(m_box(st, f)[bM]);
             decode<S>(P, v, nd);
         }
+
+        // coefficient tensor and colour split; inactive sources keep all-zero coefficients
         Coef cf{};
-        float dcoef = 0.0f, Fx = 0.0f, Fy = 0.0f, Fz = 0.0f, omega2_rest = 0.0f;
-        const float rho_src = nd.rr + nd.rb, rr_src = nd.rr;
-        const float inv = fast_rcp(rho_src);
-        // colour fraction as a correctly rounded quotient (see step_tile)
-        const float q0 = nd.rr * inv;
-        const float q1 = fmaf(fmaf(-q0, rho_src, nd.rr), inv, q0);
-        const float aR = nd.rb == 0.0f ? 1.0f : (nd.rr == 0.0f ? 0.0f : q1);
-        // (zero-filled staging outside the lattice decodes to a mixed node: off the interface path)
-        const bool iface = (4.0f * nd.rr * nd.rb * inv * inv) > 1.0e-4f && in_xy; // lbm.cuh:181,187
-        build_coef(P, cf, rho_src, nd.ux, nd.uy, nd.uz, nd.pxx, nd.pxy, nd.pyy, nd.pyz, nd.pzz, nd.pxz);
+        float aR = 0.0f, dcoef = 0.0f, Fx = 0.0f, Fy = 0.0f, Fz = 0.0f, omega2_rest = 0.0f;
+        bool iface = false;
+        if (active) {
+            const float rho = nd.rr + nd.rb;
+            const float inv = fast_rcp(rho);
+            // colour fraction as a correctly rounded quotient (one residual correction): a
+            // product with a rounded reciprocal is biased (aR rho - rr averages +2.5e-10 per
+            // mixed node), which would move colour mass the same way every step
+            const float q0 = nd.rr * inv;
+            const float q1 = fmaf(fmaf(-q0, rho, nd.rr), inv, q0);
+            aR = nd.rb == 0.0f ? 1.0f : (nd.rr == 0.0f ? 0.0f : q1);
+            iface = (4.0f * nd.rr * nd.rb * inv * inv) > 1.0e-4f; // lbm.cuh:181,187
+            // zero-filled staging outside the lattice decodes to a mixed node: off the interface path
+            iface = iface && in_xy;
+            build_coef<kFB>(P, cf, rho, nd.rr, nd.rb, nd.ux, nd.uy, nd.uz, nd.pxx, nd.pxy, nd.pyy, nd.pyz, nd.pzz, nd.pxz);
+        }
         const bool any_iface = __any_sync(kFull, iface);
         if (any_iface && iface) {
             // colour gradient at the source (forces.cuh:20-60) from the psi ring
@@ -394,7 +485,9 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
             Fz = 3.0f * sz;
             const float absF = sqrtf(Fx * Fx + Fy * Fy + Fz * Fz);
             // Omega2 (collisionOperators.cuh:16-25) folded into the coefficients
-            const float Aeff = P.A; // A_calculation (forces.cuh:114-117)
+            float Aeff = P.A; // A_calculation (forces.cuh:114-117) at the node's relaxation time
+            if constexpr ((kFB & F_FORCE) != 0)
+                if (P.tau_var) Aeff = P.s4 / tau_eff_of(P, nd.rr, nd.rb);
             float hA = (P.omega2_conservative && !(absF > 1.0e-4f)) ? 0.0f : 0.5f * Aeff * absF;
             if (absF > 1.0e-4f) {
                 const float ia_ = fast_rcp(absF);
@@ -408,12 +501,18 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
                 cf.p110 += 2.0f * qf * Fx * Fy;
                 cf.p101 += 2.0f * qf * Fx * Fz;
                 cf.p011 += 2.0f * qf * Fy * Fz;
-                // recolouring (collisionOperators.cuh:60-80): beta rr rb / (rho^2 |F|) * rho
-                dcoef = P.beta * (nd.rr * nd.rb) * inv * inv * ia_ * rho_src;
+                // recolouring (collisionOperators.cuh:60-80): beta rr rb / (rho^2 |F|) * feq0, where
+                // the rest equilibrium of moving directions is w rho (w (rho + K) with a density ratio)
+                const float rho = nd.rr + nd.rb;
+                const float feq0 = ((kFB & F_FORCE) && P.ratio) ? rho + nd.rr * P.kappa_r + nd.rb * P.kappa_b : rho;
+                const float irho = fast_rcp(rho);
+                dcoef = P.beta * (nd.rr * nd.rb) * irho * irho * ia_ * feq0;
             }
             cf.p000 -= hA;
             omega2_rest = hA; // rest-population part, -hA (B0 - w0) = +2/3 hA, added below in exact units
         }
+        const float rho_src = active ? nd.rr + nd.rb : 0.0f;
+        const float rr_src = active ? nd.rr : 0.0f;
         // colour fractions of the x neighbours (lane -1 and lane +1)
         float2 aRlr;
         aRlr.x = __shfl_up_sync(kFull, aR, 1);
@@ -438,9 +537,19 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
         const float dk1 = kSepW ? dcoef : 2.0f * dcoef;
         const float dk2 = dcoef * 0.7071067811865475f;
         const float dk3 = kSepW ? dcoef * 0.5773502691896258f : 0.0f;
-        // rest-population part of Omega2, -hA (B0 - w0) = +2/3 hA, in value units of the rest weight (64 of
-        // 216, or 12 of 36), so that Omega2 sums to zero over the directions
-        const float rc0 = (kSepW ? 2.25f : 2.0f) * omega2_rest;
+        // rest-population correction (density-ratio K and the Omega2 rest term), with the Omega2
+        // part in exact units so that Omega2 sums to zero over the directions (B0 - w0 = -2/3
+        // for both lattices)
+        // in value units before the rest weight (64 of 216, or 12 of 36): S r0 / W_0 and
+        // S (w0 - B0) hA / W_0 = (2/3) S hA / W_0, i.e. 3.375 r0 + 2.25 hA or 3 r0 + 2 hA
+        const float rc0 = kSepW ? fmaf(cf.r0, 3.375f, 2.25f * omega2_rest) : fmaf(cf.r0, 3.0f, 2.0f * omega2_rest);
+
+        // wall bounce-back of this node's own populations (destination = this node, plane k)
+        const bool wx0 = P.bc[0] == MBCG_BC_WALL && xs == 1, wx1 = P.bc[0] == MBCG_BC_WALL && xs == nx - 2;
+        const bool wy0 = P.bc[1] == MBCG_BC_WALL && ys == 1, wy1 = P.bc[1] == MBCG_BC_WALL && ys == ny - 2;
+        const bool wz0 = P.bc[2] == MBCG_BC_WALL && k == 1, wz1 = P.bc[2] == MBCG_BC_WALL && k == nz - 2;
+        const bool reflect = (kFB & F_WALL) && role == R_FLUID && dest_thread && (wx0 | wx1 | wy0 | wy1 | wz0 | wz1);
+        const bool any_reflect = (kFB & F_WALL) ? __any_sync(kFull, reflect) : false;
 
         // ---- emit: populations of the rows this warp exports, x streaming, own-row moments,
         // y exchange.  Halo rows export one population row (cy = +1 for warp 0, -1 for warp W-1).
@@ -520,6 +629,27 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
                     if (shc == 1) return fmaf(2.0f, b, dl);
                     return fmaf(12.0f, b, dl);
                 };
+                if constexpr (ROWS == 7 && (kFB & F_WALL) != 0) {
+                    if (any_reflect && reflect) {
+#pragma unroll
+                        for (int i = 0; i < 3; ++i)
+#pragma unroll
+                            for (int j = 0; j < 3; ++j) {
+                                const int cx = i - 1, cy = j - 1;
+                                if (!Stencil<Q>::has(cx, cy, cz)) continue;
+                                const bool into = (wx0 && cx < 0) || (wx1 && cx > 0) || (wy0 && cy < 0) ||
+                                                  (wy1 && cy > 0) || (wz0 && cz < 0) || (wz1 && cz > 0);
+                                if (!into) continue;
+                                const float f = kSepW ? static_cast<float>((cx == 0 ? 4 : 1) * (cy == 0 ? 4 : 1) *
+                                                                           (cz == 0 ? 4 : 1))
+                                                      : 1.0f;
+                                const float gv = i == 0 ? g[j].o.x : (i == 2 ? g[j].o.y : g[j].c);
+                                const float smv = i == 0 ? sm[j].o.x : (i == 2 ? sm[j].o.y : sm[j].c);
+                                const float rr_ = red_pop(rr_src, smv, gv, any_iface ? delta(i, j) : 0.0f, i, j, any_iface);
+                                add_pop(accC, f * gv, f * rr_, -cx, -cy, -cz);
+                            }
+                    }
+                }
                 // x streaming: destination x receives cx=+1 from lane-1 and cx=-1 from lane+1.
                 // The populations cross lanes; on interface warps the source forms its red
                 // populations (red_pop) and they cross too, elsewhere the destination forms them
@@ -656,7 +786,16 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
             const float rr = accP.rr.y;
             const float rb = rho - rr;
             const float inv = fast_rcp(rho);
-            const float ux = accP.jxx.x * inv, uy = accP.jy * inv, uz = accP.jz * inv;
+            float Fbx = 0.0f, Fby = 0.0f, Fbz = 0.0f;
+            constexpr bool kF = (kFB & F_FORCE) != 0;
+            if (kF && P.forced) {
+                Fbx = rho * P.g[0];
+                Fby = rho * P.g[1];
+                Fbz = rho * P.g[2];
+            }
+            const float ux = (accP.jxx.x + 0.5f * Fbx) * inv;
+            const float uy = (accP.jy + 0.5f * Fby) * inv;
+            const float uz = (accP.jz + 0.5f * Fbz) * inv;
             const float ctr = cs2 * rho;
             float pi[6];
             pi[0] = (accP.jxx.y - ctr) - rho * ux * ux;
@@ -665,6 +804,20 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
             pi[3] = accP.yz - rho * uy * uz;
             pi[4] = (accP.zz - ctr) - rho * uz * uz;
             pi[5] = accP.xz - rho * ux * uz;
+            if (kF && P.forced) {
+                pi[0] += ux * Fbx;
+                pi[1] += 0.5f * (ux * Fby + uy * Fbx);
+                pi[2] += uy * Fby;
+                pi[3] += 0.5f * (uy * Fbz + uz * Fby);
+                pi[4] += uz * Fbz;
+                pi[5] += 0.5f * (ux * Fbz + uz * Fbx);
+            }
+            if (kF && P.ratio) {
+                const float Kc = (rr * P.kappa_r + rb * P.kappa_b) * cs2;
+                pi[0] -= Kc;
+                pi[2] -= Kc;
+                pi[4] -= Kc;
+            }
             const long long at = static_cast<long long>(d) * P.plane + static_cast<long long>(ys) * P.pitch + xs;
             finalize_store<S>(P, at * static_cast<int>(sizeof(S)), 0U, xs, ys, d, rr, rb, ux, uy, uz, pi, img_x, img_y,
                               key_base);
@@ -675,29 +828,58 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
         }
         accP = accC;
         accC = accN; // accN is assigned before it is added to again
+            return true;
+    };
+    auto run = [&](auto featc, int kend) -> bool {
+        for (; k <= kend; ++k, sl = nxt(sl))
+            if (!plane(featc)) return false;
+        return true;
+    };
+    if constexpr ((kFeat & F_WALL) != 0) {
+        // walls on the z axis: planes 2 .. nz-5 need none of their part (fluid sources with identity
+        // mappings, no wall-adjacent source)
+        if (P.bc[2] == MBCG_BC_WALL) {
+            const int k0 = max(zd0 - 1, 2), k1 = min(zd1, nz - 5);
+            if (k1 >= k0) {
+                if (!run(std::integral_constant<int, kFeat>{}, k0 - 1)) return false;
+                if (!run(std::integral_constant<int, kFeat & ~F_WALL>{}, k1)) return false;
+            }
+        }
     }
+    if (!run(std::integral_constant<int, kFeat>{}, zd1)) return false;
     // every load of this tile was waited for: carry the parities over to the next tile
     phase = par;
     return true;
 }
 
-template <int Q, typename S, int W>
+template <int Q, typename S, int W, int kFeat>
 __global__ void __launch_bounds__(32 * W, W <= 8 ? 2 : 1) step_kernel(const __grid_constant__ StepParams P,
                                                                       const __grid_constant__ TensorMaps T) {
     unsigned char* smem = aligned_smem_base();
     init_barriers<0>(smem);
+    wait_prior_grid();
     uint32_t phase = 0;
-    tile<Q, S, W>(P, T.m, blockIdx.x, blockIdx.y, blockIdx.z, P.step, smem, phase);
+    tile<Q, S, W, kFeat>(P, T.m, blockIdx.x, blockIdx.y, blockIdx.z, P.step, smem, phase);
 }
 
-template <int Q, typename S, int W>
-cudaError_t launch(const StepParams& P, const TensorMaps& T, cudaStream_t s) {
-    auto kern = step_kernel<Q, S, W>;
+template <int Q, typename S, int W, int kFeat>
+cudaError_t launch_one(const StepParams& P, const TensorMaps& T, cudaStream_t s) {
+    auto kern = step_kernel<Q, S, W, kFeat>;
     static std::atomic<unsigned long long> configured{0};
     if (cudaError_t e = configure_once(kern, Geo<S, W>::smem, configured)) return e;
     const dim3 grid((P.nx - 2 + kTX - 1) / kTX, (P.ny - 2 + W - 3) / (W - 2), (P.nz - 2 + P.zchunk - 1) / P.zchunk);
-    kern<<<grid, dim3(32, W, 1), Geo<S, W>::smem, s>>>(P, T);
-    return cudaGetLastError();
+    return launch_pdl(kern, grid, dim3(32, W, 1), Geo<S, W>::smem, s, P, T);
+}
+
+template <int Q, typename S, int kFeat>
+cudaError_t launch_w(int w, const StepParams& P, const TensorMaps& T, cudaStream_t s) {
+    return w == kStepWSmall ? launch_one<Q, S, kStepWSmall, kFeat>(P, T, s) : launch_one<Q, S, kStepW, kFeat>(P, T, s);
+}
+template <int Q, typename S>
+cudaError_t launch(int w, const StepParams& P, const TensorMaps& T, cudaStream_t s) {
+    if constexpr (std::is_same<S, __nv_bfloat16>::value)
+        if (features_of(P) != 0) return launch_w<Q, S, F_WALL | F_FORCE>(w, P, T, s);
+    return launch_w<Q, S, 0>(w, P, T, s);
 }
 
 } // namespace pop

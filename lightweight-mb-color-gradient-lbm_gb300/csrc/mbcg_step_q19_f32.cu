@@ -1,5 +1,5 @@
-// Plain step kernels for D3Q19 with float storage: block shapes W = 8 and 16, feature sets
-// {none, inlet/outlet, all} on the TMA path and all features on the plain-load path.
+// Plain step kernels for D3Q19 with float storage: block shapes 8 and 16, feature sets
+// {none, inlet/outlet, walls + force, all} on the TMA path and all features on the plain-load path.
 #include "mbcg_step.cuh"
 
 namespace mbcg {

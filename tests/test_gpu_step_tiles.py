@@ -128,3 +128,25 @@ def test_steps_in_a_row_are_the_steps_one_by_one(size, precision):
             assert c.status() == 0
             got.append(c.copy_out())
     assert np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))
+
+
+@pytest.mark.parametrize("kind,axis", [("periodic", 0), ("wall", 0), ("wall", 1), ("wall", 2)])
+def test_tiling_does_not_show_in_bf16(kind, axis):
+    """Lattices without an inlet in BF16 storage step by populations; tile shape and depth change no bit."""
+    for size in SIZES:
+        p = make(kind, axis, 27, size)
+        p.precision = mbcg.BF16
+        a = state_of(p).astype(np.float32)
+        idx = written_nodes(p)
+        first = None
+        for shape in ((16, 5), (8, 2), (16, 64)):
+            with mbcg.Case(p) as c:
+                c.set_shape(*shape)
+                c.copy_in(a)
+                c.step(STEPS)
+                got = c.copy_out()
+                assert c.status() == 0
+            assert np.isfinite(got[idx]).all()
+            if first is None:
+                first = got
+            np.testing.assert_array_equal(got[idx], first[idx], err_msg=f"{kind} {axis} {size} {shape}")
