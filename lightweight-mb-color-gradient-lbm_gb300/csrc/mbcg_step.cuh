@@ -29,7 +29,7 @@
 // Two nodes a thread.  A warp holds two rows of the tile, w from below and w from above, one in each
 // half of f32x2 registers, the upper one in a frame with y mirrored: both halves take the same
 // operations throughout, and every arithmetic instruction does two nodes' work.  The kernel is bound by
-// instruction issue and latency, not by HBM (D3Q27 jet 256x256x1024, FP32): 590 warp instructions per 32
+// instruction issue and latency, not by HBM (D3Q27 jet 256x256x1024, FP32): 663 warp instructions per 32
 // node updates and 12 warps per SM, against 971 and 16 for one node a thread with all 27 populations
 // formed and crossing lanes; 2.72 ms -> 1.90 ms a step (24.7 -> 35.4 GLUPS).
 //
