@@ -145,10 +145,10 @@ int choose_zchunk(const mbcg_params& p, int W) {
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long units = static_cast<long long>(sms) * (W == kStepWSmall ? 2 : 1); // CTAs at a time
     // The depth with the shortest launch: tiles of a chunk take its planes and about three more (the two
-    // source planes outside it, and the start: 18.5 us at depth 1, 43 at 8, 127 at 32 on one tile per
-    // SM, 3.5 us a plane), run in waves, and the two-plane tiles at the ends of a non-periodic z axis
-    // fill what the last wave leaves idle.  Small lattices get thin tiles this way (32^3: depth 1, 18.5 us
-    // a step against 43 at depth 8).
+    // source planes outside it, and the start: 32^3, 15.5 us a step at depth 1, 39 at 8, 120 at 32, 3.4 us
+    // a plane), run in waves, and the two-plane tiles at the ends of a non-periodic z axis fill what the
+    // last wave leaves idle.  (8-row tiles, two to an SM, are no faster at any depth from 64^3 on: 28.5
+    // against 23.1 us a step there, 88 against 62 on 61^2x243.)
     constexpr long long kExtra = 3;
     const int nzf = p.nz - 2, cap = case_pop(p) ? 0 : z_cap(p.nz, p.bc[2]), inner = nzf - 2 * cap;
     const long long thin = cap ? 2 * g : 0, thin_cost = cap + kExtra;
