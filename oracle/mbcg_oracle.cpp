@@ -475,9 +475,9 @@ struct Oracle {
             for (int64_t o = 0; o < n_all; ++o) psi_c[o] = psi(A[0][o], A[1][o]);
             psi_ready = true;
 #pragma omp parallel for schedule(static) num_threads(threads) if (threads > 1)
-            for (int z = 0; z < N[2]; ++z)
-                for (int y = 0; y < N[1]; ++y)
-                    for (int x = 0; x < N[0]; ++x) {
+            for (int z = 1; z < N[2] - 1; ++z) // (bulk sources are fluid nodes; a ghost node's stencil leaves the arrays)
+                for (int y = 1; y < N[1] - 1; ++y)
+                    for (int x = 1; x < N[0] - 1; ++x) {
                         const int64_t o = id(x, y, z);
                         if (!interface_node(o)) continue;
                         const int n[3] = {x, y, z};
