@@ -4,8 +4,8 @@
 // The work is a flat queue of tiles (BatchTile) over the live lattices of one kind (Q, storage, feature
 // set), sorted by the host, largest tiles first.  Each CTA of a grid of at most one CTA per SM takes the
 // next tile with an atomic counter and runs the same step_tile() as the plain kernel on that lattice's
-// step parameters in a constant-memory table indexed by slot.  The stage mbarriers are initialised once
-// per CTA; their phase carries from tile to tile.  The kinds' launches of one step are branches of the
+// step parameters in a constant-memory table indexed by slot.  The mbarriers are initialised once
+// per CTA; their parities carry from tile to tile.  The kinds' launches of one step are branches of the
 // server's graph and overlap: a kind's next step waits for its own tiles only.
 //
 // One kernel per kind, not one with every body: side by side in one kernel the bodies spilled 280 bytes
