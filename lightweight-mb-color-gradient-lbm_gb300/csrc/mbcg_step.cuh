@@ -945,10 +945,11 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
             }
         }
     }
-    if constexpr (kTMA) {
-        __syncthreads(); // plane kfirst is a source of nothing: its slot is free
+    // Plane kfirst is a source of nothing: once every warp has its psi, which beside an x or y boundary comes
+    // from a neighbour's node, its slot is free (plain copies: refilled by the first plane's step (2)).
+    __syncthreads();
+    if constexpr (kTMA)
         if (kfirst + kNSTAGE <= zd1 + 1) issue(kfirst + kNSTAGE, 0);
-    }
 
     // store addresses: bytes from the tile's first destination plane, advanced plane by plane
     const long long tile_base = static_cast<long long>(zd0) * P.plane * static_cast<int>(sizeof(S));
