@@ -262,15 +262,20 @@ __global__ void merge_kernel(const PhaseArgs A) {
 }
 
 // Region sizes.  Most lanes of a warp share a root: one atomic per distinct root and warp (one per node
-// on the few roots took 174 us for 1.2 M tracked nodes of 192x192x512).
+// on the few roots took 174 us for 1.2 M tracked nodes of 192x192x512).  Every lane of a warp goes through
+// the loop as often as the others and takes part in the match, with a root of -1 where it has no node.
 __global__ void region_kernel(const PhaseArgs A, int* volume, unsigned char* touches) {
     const long long total = static_cast<long long>(A.nf[0]) * A.nf[1] * A.nf[2];
-    for (long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; e < total;
-         e += static_cast<long long>(gridDim.x) * blockDim.x) {
-        if (A.labels[e] < 0) continue;
-        const int r = find_root(A.labels, static_cast<int>(e), A.status);
-        const unsigned peers = __match_any_sync(__activemask(), r);
-        if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&volume[r], __popc(peers));
+    const int lane = threadIdx.x & 31;
+    for (long long e0 = blockIdx.x * static_cast<long long>(blockDim.x) + (threadIdx.x - lane); e0 < total;
+         e0 += static_cast<long long>(gridDim.x) * blockDim.x) {
+        const long long e = e0 + lane;
+        int r = -1;
+        if (e < total && A.labels[e] >= 0) r = find_root(A.labels, static_cast<int>(e), A.status);
+        if (!__any_sync(0xffffffffu, r >= 0)) continue;
+        const unsigned peers = __match_any_sync(0xffffffffu, r);
+        if (r < 0) continue;
+        if (lane == __ffs(peers) - 1) atomicAdd(&volume[r], __popc(peers));
         if (A.ia >= 0) {
             const int c[3] = {static_cast<int>(e % A.nf[0]), static_cast<int>((e / A.nf[0]) % A.nf[1]),
                               static_cast<int>(e / (static_cast<long long>(A.nf[0]) * A.nf[1]))};
