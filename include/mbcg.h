@@ -365,7 +365,8 @@ typedef struct mbcg_server_stats {
     int32_t reserved;
     double plane_ns[10];    /* cost model: ns per tile plane of each batch-kernel body, in the
                                order Q19 FP32/FP16/BF16, Q27 FP32/FP16/BF16 (every feature),
-                               Q19 FP32/FP16, Q27 FP32/FP16 (fully periodic, unforced)          */
+                               Q19 FP32/FP16, Q27 FP32/FP16 (fully periodic, unforced); the
+                               bodies of BF16 lattices without an inlet are not listed         */
     double tile_overhead_planes; /* cost model: fixed cost of a tile, in planes                */
     double busy_s;          /* first admission to the last completion                          */
 } mbcg_server_stats;

@@ -11,17 +11,26 @@ namespace mbcg {
 enum BatchKind : int {
     BK_Q19_F32 = 0, BK_Q19_F16, BK_Q19_BF16, BK_Q27_F32, BK_Q27_F16, BK_Q27_BF16, // every feature
     BK_Q19_F32_P, BK_Q19_F16_P, BK_Q27_F32_P, BK_Q27_F16_P,                      // fully periodic, unforced
+    BK_Q19_BF16_N, BK_Q27_BF16_N,                                                // without an inlet
     BK_COUNT
 };
 
 inline int batch_kind(int q, int precision, int features) {
+    if (precision == MBCG_BF16 && uses_pop(precision, features)) return q == 27 ? BK_Q27_BF16_N : BK_Q19_BF16_N;
     const bool lean = features == 0 && precision != MBCG_BF16;
     if (lean) return (q == 27 ? BK_Q27_F32_P : BK_Q19_F32_P) + (precision == MBCG_FP16 ? 1 : 0);
     return (q == 27 ? BK_Q27_F32 : BK_Q19_F32) + precision;
 }
 
 inline int batch_q(int kind) {
-    return (kind >= BK_Q27_F32 && kind <= BK_Q27_BF16) || kind >= BK_Q27_F32_P ? 27 : 19;
+    return (kind >= BK_Q27_F32 && kind <= BK_Q27_BF16) || kind == BK_Q27_F32_P || kind == BK_Q27_F16_P ||
+                   kind == BK_Q27_BF16_N
+               ? 27
+               : 19;
+}
+// the kinds that step by populations (uses_pop)
+inline bool batch_pop(int kind) {
+    return kind == BK_Q19_F16_P || kind == BK_Q27_F16_P || kind == BK_Q19_BF16_N || kind == BK_Q27_BF16_N;
 }
 
 // One resident lattice: TMA descriptors and step parameters for both directions
@@ -33,7 +42,8 @@ struct BatchCase {
     int pad[15];
 };
 
-// One unit of the flat tile queue: a (30 x 22 x zchunk) tile of the lattice in slot `slot`.
+// One unit of a kind's tile queue: a tile of the lattice in slot `slot`, 30 columns x (batch_rows - 2) rows x
+// a chunk of planes.
 struct BatchTile {
     uint16_t slot, bx, by, bz;
 };
@@ -46,7 +56,11 @@ struct ChunkState {
     int nsteps;
 };
 
-constexpr int kBatchW = kStepW; // shape of the batch kernel's CTAs (step_rows)
+constexpr int kBatchW = kStepW; // shape of the batch kernels' CTAs (step_rows)
+// source rows of a kind's CTAs
+inline int batch_rows(int kind) { return batch_pop(kind) ? kBatchW : step_rows(kBatchW); }
+// Z boundary as the cut of a kind's z axis (z_tiles, z_range) takes it: the step by populations has no end tiles.
+inline int batch_bcz(int kind, int bcz) { return batch_pop(kind) ? MBCG_BC_PERIODIC : bcz; }
 // Lattices resident at once: the batch kernel reads each one's step parameters (both parities)
 // from a constant-memory table of this many slots (2 x 64 x 408 bytes), as uniform loads the
 // instructions take as operands, where a copy in shared memory costs a load into a register per use.

@@ -21,7 +21,8 @@ constexpr int kStepW = 16;
 constexpr int kStepWSmall = 8;
 constexpr int step_rows(int w) { return w == kStepWSmall ? 8 : 24; }
 // Lattices in BF16 storage without an inlet, and in FP16 storage fully periodic and unforced ones, step by
-// populations, one node a thread, w source rows (the reason stands in mbcg_step_pop.cuh).
+// populations, one node a thread, w source rows, on every path: cases, the server, plain loads (the reason
+// stands in mbcg_step_pop.cuh).
 constexpr bool uses_pop(int precision, int features) {
     return precision == MBCG_BF16 ? (features & F_INOUT) == 0 : precision == MBCG_FP16 && features == 0;
 }

@@ -130,7 +130,7 @@ struct Request {
     size_t off = 0, bytes = 0;
     long long pitch = 0, plane = 0, fstride = 0;
     int es = 4;
-    int features = 0;
+    int kind = -1;           // its batch kernel (BatchKind)
     int zchunk = 32;
     void* fields[2][NF] = {};
     int cur = 0;             // parity of the state holding step steps_done
@@ -174,7 +174,7 @@ struct mbcg_server {
     cudaEvent_t t0_ev = nullptr;
     std::chrono::steady_clock::time_point t0;
     // cost model of a tile: (planes + tile_ovh) x plane_ns[kind]; measured by calibrate()
-    double plane_ns[BK_COUNT] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
+    double plane_ns[BK_COUNT] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
     double tile_ovh = 3.0;
     int last_z = 0; // tile depth the planner chose for the current composition
 
@@ -221,6 +221,12 @@ size_t footprint(const mbcg_params& p, long long* pitch, long long* fstride, int
     const size_t states = 2ull * NF * static_cast<size_t>(*fstride) * *es;
     const size_t diag = align_up(sizeof(double) * kDiagSlots * (*nparts + 1) + 16, kAlign);
     return states + diag;
+}
+
+int kind_of(const mbcg_params& p) {
+    StepParams P;
+    fill_step_physics(p, P);
+    return batch_kind(p.q, p.precision, features_of(P));
 }
 
 StepParams step_params(const Request& r, int from, int* status_word) {
@@ -328,11 +334,7 @@ cudaError_t admit(mbcg_server* s, Request& r, int slot) {
     r.slot = slot;
     r.cur = 0;
     r.resident = true;
-    {
-        StepParams P0;
-        fill_step_physics(r.p, P0);
-        r.features = features_of(P0);
-    }
+    if (r.kind < 0) r.kind = kind_of(r.p); // (calibrate() chooses its own)
     r.zchunk = r.p.nz - 2; // set per composition by the planner (rebuild)
 
     // lattice table entry (host side; rebuild() uploads the table of the composition)
@@ -342,10 +344,10 @@ cudaError_t admit(mbcg_server* s, Request& r, int slot) {
         C.P[par] = step_params(r, par, status_word);
         const void* f[NF];
         for (int i = 0; i < NF; ++i) f[i] = r.fields[par][i];
-        if (encode_state_maps(r.p, f, r.pitch, step_rows(kBatchW), *reinterpret_cast<TensorMaps*>(C.maps[par])) != MBCG_OK)
+        if (encode_state_maps(r.p, f, r.pitch, batch_rows(r.kind), *reinterpret_cast<TensorMaps*>(C.maps[par])) != MBCG_OK)
             return cudaErrorInvalidValue;
     }
-    C.kind = batch_kind(r.p.q, r.p.precision, r.features);
+    C.kind = r.kind;
     // a clean state (every byte the case can read is its own) and its initial condition
     cudaError_t e = cudaMemsetAsync(base, 0, r.bytes, s->st);
     if (e == cudaSuccess) {
@@ -364,7 +366,8 @@ cudaError_t admit(mbcg_server* s, Request& r, int slot) {
 // tiles of a lattice at the reference depth of 16 planes (the admission measure of load)
 long long load_tiles(const mbcg_params& p) {
     const long long gx = (p.nx - 2 + kStepTileX - 1) / kStepTileX;
-    const long long gy = (p.ny - 2 + step_tile_rows(kBatchW) - 1) / step_tile_rows(kBatchW);
+    const int rows = batch_rows(kind_of(p)) - 2;
+    const long long gy = (p.ny - 2 + rows - 1) / rows;
     return gx * gy * ((p.nz - 2 + 15) / 16);
 }
 
@@ -439,17 +442,17 @@ void make_tiles(const mbcg_server* s, int z, std::vector<TileItem>& items, std::
         if (!id) continue;
         const Request& r = *s->reqs.at(id);
         const int gx = (r.p.nx - 2 + kStepTileX - 1) / kStepTileX;
-        const int gy = (r.p.ny - 2 + step_tile_rows(kBatchW) - 1) / step_tile_rows(kBatchW);
-        const int nzf = r.p.nz - 2 - 2 * z_cap(r.p.nz, r.p.bc[2]);
+        const int kind = r.kind, rows = batch_rows(kind) - 2, bcz = batch_bcz(kind, r.p.bc[2]);
+        const int gy = (r.p.ny - 2 + rows - 1) / rows;
+        const int nzf = r.p.nz - 2 - 2 * z_cap(r.p.nz, bcz);
         const int zmax = std::min(z, max_zchunk(r.plane, r.es));
         const int nch = std::max(1, (nzf + zmax - 1) / zmax);
         const int depth = (nzf + nch - 1) / nch;
-        const int gz = z_tiles(r.p.nz, r.p.bc[2], depth);
+        const int gz = z_tiles(r.p.nz, bcz, depth);
         zc[slot] = depth;
-        const int kind = batch_kind(r.p.q, r.p.precision, r.features);
         for (int bz = 0; bz < gz; ++bz) {
             int zd0, zd1;
-            z_range(r.p.nz, r.p.bc[2], depth, bz, zd0, zd1);
+            z_range(r.p.nz, bcz, depth, bz, zd0, zd1);
             const double planes = zd1 - zd0 + 2 + s->tile_ovh;
             for (int by = 0; by < gy; ++by)
                 for (int bx = 0; bx < gx; ++bx)
@@ -798,21 +801,15 @@ int calibrate(mbcg_server* s) {
     double ovh_sum = 0.0;
     int ovh_n = 0;
     for (int kind = 0; kind < BK_COUNT; ++kind) {
-        const bool lean = kind >= BK_Q19_F32_P;
-        int q, prec;
-        if (!lean) {
-            q = kind >= BK_Q27_F32 ? 27 : 19;
-            prec = kind % 3;
-        } else {
-            q = kind >= BK_Q27_F32_P ? 27 : 19;
-            prec = (kind - BK_Q19_F32_P) % 2;
-        }
+        const bool lean = kind >= BK_Q19_F32_P && kind <= BK_Q27_F16_P;
+        const int q = batch_q(kind), rows = batch_rows(kind) - 2;
+        const int prec = kind >= BK_Q19_BF16_N ? MBCG_BF16 : lean ? (kind - BK_Q19_F32_P) % 2 : kind % 3;
         mbcg_params p;
         mbcg_params_default(&p);
         p.q = q;
         p.precision = prec;
         p.nx = 2 + gx * kStepTileX;
-        p.ny = 2 + gy * step_tile_rows(kBatchW);
+        p.ny = 2 + gy * rows;
         p.nz = 2 + kDeep;
         p.bc[0] = p.bc[1] = p.bc[2] = MBCG_BC_PERIODIC;
         p.ic = MBCG_IC_BUBBLE;
@@ -829,6 +826,7 @@ int calibrate(mbcg_server* s) {
         Request r;
         r.p = p;
         r.id = -1;
+        r.kind = kind; // (BF16: the body with an inlet steps it as well)
         long long pitch, fstride;
         int es, nparts;
         r.bytes = footprint(p, &pitch, &fstride, &es, &nparts);
@@ -836,7 +834,6 @@ int calibrate(mbcg_server* s) {
         const int64_t saved = s->slot_req[0];
         cudaError_t e = admit(s, r, 0);
         s->slot_req[0] = saved;
-        if (e == cudaSuccess && batch_kind(q, prec, r.features) != kind) e = cudaErrorInvalidValue;
         float t[2] = {0, 0};
         for (int d = 0; d < 2 && e == cudaSuccess; ++d) {
             const int depth = d == 0 ? kDeep : kShallow;
@@ -1040,7 +1037,7 @@ int mbcg_server_submit(mbcg_server* s, const mbcg_params* p, int64_t nsteps, int
     if (int rc = validate_params(p)) return rc;
     if (nsteps < 0) return fail(MBCG_E_INVALID, "negative step count");
     if (p->ic == MBCG_IC_NONE) return fail(MBCG_E_INVALID, "a served case needs an initial condition");
-    if (p->nx - 2 > 0xffff * kStepTileX || p->ny - 2 > 0xffff * step_tile_rows(kBatchW) || p->nz - 2 > 0xffff * 8)
+    if (p->nx - 2 > 0xffff * kStepTileX || p->ny - 2 > 0xffff * (batch_rows(kind_of(*p)) - 2) || p->nz - 2 > 0xffff * 8)
         return fail(MBCG_E_UNSUPPORTED, "lattice too large for the tile queue");
     long long pitch, fstride;
     int es, nparts;
@@ -1214,7 +1211,7 @@ int mbcg_server_get_stats(mbcg_server* s, mbcg_server_stats* out) {
     out->arena_bytes = static_cast<int64_t>(s->arena.size());
     out->arena_peak_bytes = static_cast<int64_t>(s->arena.peak());
     out->zchunk = s->last_z;
-    for (int k = 0; k < BK_COUNT; ++k) out->plane_ns[k] = s->plane_ns[k];
+    for (int k = 0; k < BK_Q19_BF16_N; ++k) out->plane_ns[k] = s->plane_ns[k];
     out->tile_overhead_planes = s->tile_ovh;
     out->busy_s = (s->first_admit >= 0 && s->last_done >= 0) ? s->last_done - s->first_admit : 0.0;
     return MBCG_OK;

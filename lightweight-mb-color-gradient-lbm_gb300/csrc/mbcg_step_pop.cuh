@@ -8,6 +8,9 @@
 // that much.  With a density ratio a last bit of FP32 now and then rounds a colour slot the other way (three
 // nodes in 10^6); beside such a node the stress of the next step is up to 1.7 times the field's mean away
 // in BF16, 0.3 times in FP16 (RTI).  With an inlet states agree to 6e-4 (BF16) after two steps.
+// For the same reason the server and the plain-load path step them by populations too: served by step_tile
+// their states differed from a case's by up to a unit of the form after the first step (served alone, D3Q27 drop
+// 61^3 in FP16 41 us a step against 31 by step_tile, in BF16 46 against 31; RTI 31^2x64 in BF16 26 against 41).
 //
 // Each source evaluates all Q populations of its coefficient tensor with a separable inverse transform (x, y,
 // then z); they stream to the neighbouring lanes by shuffles, to the neighbouring rows through shared memory and
@@ -171,7 +174,7 @@ __device__ __forceinline__ void add_pop(Acc& a, float g, float r, int ex, int ey
 }
 
 // one tile (30 columns x (W-2) rows x zchunk planes), arguments as step_tile's
-template <int Q, typename S, int W, int kFeat>
+template <int Q, typename S, int W, bool kTMA, int kFeat>
 __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* maps, int bx, int by, int bz, long long step,
                                      unsigned char* smem, uint32_t& phase) {
     using G = Geo<S, W>;
@@ -270,14 +273,28 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
     auto issue = [&](int k, int sl) {
         unsigned char* st = stage_at(sl);
         const int kz = zload(k);
-        if (tid == 0) {
-            uint64_t* bar = &bars[sl];
-            fence_proxy_async();
-            mbar_expect_tx(bar, G::tx);
-            tma_load_3d(rb_box(st, 0), &maps[0], xr0, yb - 1, kz, bar);
-            tma_load_3d(rb_box(st, 1), &maps[1], xr0, yb - 1, kz, bar);
+        if constexpr (kTMA) {
+            if (tid == 0) {
+                uint64_t* bar = &bars[sl];
+                fence_proxy_async();
+                mbar_expect_tx(bar, G::tx);
+                tma_load_3d(rb_box(st, 0), &maps[0], xr0, yb - 1, kz, bar);
+                tma_load_3d(rb_box(st, 1), &maps[1], xr0, yb - 1, kz, bar);
 #pragma unroll
-            for (int f = 2; f < NF; ++f) tma_load_3d(m_box(st, f), &maps[f], xm0, yb, kz, bar);
+                for (int f = 2; f < NF; ++f) tma_load_3d(m_box(st, f), &maps[f], xm0, yb, kz, bar);
+            }
+        } else {
+            // plain loads, for layouts TMA cannot describe: whole boxes, zeros outside the lattice
+            const long long zo = static_cast<long long>(kz) * P.plane;
+            auto box = [&](int f, S* dst, int x0, int y0, int width, int rows) {
+                for (int e = tid; e < rows * width; e += 32 * W) {
+                    const int gx = x0 + e % width, gy = y0 + e / width;
+                    const bool in = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
+                    dst[e] = in ? static_cast<const S*>(P.a[f])[zo + gy * P.pitch + gx] : Codec<S>::from_f(0.0f);
+                }
+            };
+            for (int f = 0; f < 2; ++f) box(f, rb_box(st, f), xr0, yb - 1, kRBX, G::RBY);
+            for (int f = 2; f < NF; ++f) box(f, m_box(st, f), xm0, yb, kMX, G::MY);
         }
     };
     constexpr long long kWaitLimit = 4000000000LL; // ~2 s at 2 GHz
@@ -286,7 +303,8 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
     uint32_t par = phase;
     int k_waited = kfirst - 1; // last plane whose load was waited for
     auto wait_slot = [&](int k, int sl) -> bool {
-        const bool ok = mbar_wait_bounded(&bars[sl], (par >> sl) & 1u, kWaitLimit);
+        bool ok = true;
+        if constexpr (kTMA) ok = mbar_wait_bounded(&bars[sl], (par >> sl) & 1u, kWaitLimit);
         if (ok) {
             par ^= 1u << sl;
             k_waited = k;
@@ -296,7 +314,7 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
     // on a failed wait (see step_tile)
     auto bail = [&](int k_issued) {
         if (tid == 0 && P.status) atomicOr(P.status, 1);
-        for (int k = k_waited + 1; k <= k_issued; ++k) {
+        for (int k = k_waited + 1; kTMA && k <= k_issued; ++k) {
             const int sl = (k - kfirst) % kNSTAGE;
             mbar_wait_bounded(&bars[sl], (par >> sl) & 1u, kWaitLimit / 4);
         }
@@ -353,14 +371,18 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
     __syncthreads();
     int k_issued = kfirst + kNSTAGE - 1;
     for (int k = kfirst; k <= k_issued; ++k) issue(k, k - kfirst);
+    if constexpr (!kTMA) __syncthreads();
     {
         // the first wait (wait_test_cycles: see step_tile)
-        const bool test = P.wait_test_cycles > 0;
-        bool ok = mbar_wait_bounded(test ? &bars[kMaxStages] : &bars[0], test ? 0u : (par & 1u),
-                                    test ? static_cast<long long>(P.wait_test_cycles) : kWaitLimit);
-        if (ok) {
-            par ^= 1u;
-            k_waited = kfirst;
+        bool ok = true;
+        if constexpr (kTMA) {
+            const bool test = P.wait_test_cycles > 0;
+            ok = mbar_wait_bounded(test ? &bars[kMaxStages] : &bars[0], test ? 0u : (par & 1u),
+                                   test ? static_cast<long long>(P.wait_test_cycles) : kWaitLimit);
+            if (ok) {
+                par ^= 1u;
+                k_waited = kfirst;
+            }
         }
         ok = ok && wait_slot(kfirst + 1, 1);
         if (__syncthreads_or(!ok)) {
@@ -852,34 +874,42 @@ __device__ __forceinline__ bool tile(const StepParams& P, const CUtensorMap* map
     return true;
 }
 
-template <int Q, typename S, int W, int kFeat>
+// the features of the lattices that step by populations in this storage (uses_pop)
+template <typename S>
+constexpr int pop_features() {
+    return std::is_same<S, __nv_bfloat16>::value ? F_WALL | F_FORCE : 0;
+}
+
+template <int Q, typename S, int W, bool kTMA, int kFeat>
 __global__ void __launch_bounds__(32 * W, W <= 8 ? 2 : 1) step_kernel(const __grid_constant__ StepParams P,
                                                                       const __grid_constant__ TensorMaps T) {
     unsigned char* smem = aligned_smem_base();
     init_barriers<0>(smem);
     wait_prior_grid();
     uint32_t phase = 0;
-    tile<Q, S, W, kFeat>(P, T.m, blockIdx.x, blockIdx.y, blockIdx.z, P.step, smem, phase);
+    tile<Q, S, W, kTMA, kFeat>(P, T.m, blockIdx.x, blockIdx.y, blockIdx.z, P.step, smem, phase);
 }
 
-template <int Q, typename S, int W, int kFeat>
+template <int Q, typename S, int W, bool kTMA, int kFeat>
 cudaError_t launch_one(const StepParams& P, const TensorMaps& T, cudaStream_t s) {
-    auto kern = step_kernel<Q, S, W, kFeat>;
+    auto kern = step_kernel<Q, S, W, kTMA, kFeat>;
     static std::atomic<unsigned long long> configured{0};
     if (cudaError_t e = configure_once(kern, Geo<S, W>::smem, configured)) return e;
     const dim3 grid((P.nx - 2 + kTX - 1) / kTX, (P.ny - 2 + W - 3) / (W - 2), (P.nz - 2 + P.zchunk - 1) / P.zchunk);
     return launch_pdl(kern, grid, dim3(32, W, 1), Geo<S, W>::smem, s, P, T);
 }
 
-template <int Q, typename S, int kFeat>
-cudaError_t launch_w(int w, const StepParams& P, const TensorMaps& T, cudaStream_t s) {
-    return w == kStepWSmall ? launch_one<Q, S, kStepWSmall, kFeat>(P, T, s) : launch_one<Q, S, kStepW, kFeat>(P, T, s);
+template <int Q, typename S, int W>
+cudaError_t launch_w(bool tma, const StepParams& P, const TensorMaps& T, cudaStream_t s) {
+    constexpr int kAll = pop_features<S>();
+    if (!tma) return launch_one<Q, S, W, false, kAll>(P, T, s);
+    if constexpr (kAll != 0)
+        if (features_of(P) != 0) return launch_one<Q, S, W, true, kAll>(P, T, s);
+    return launch_one<Q, S, W, true, 0>(P, T, s);
 }
 template <int Q, typename S>
-cudaError_t launch(int w, const StepParams& P, const TensorMaps& T, cudaStream_t s) {
-    if constexpr (std::is_same<S, __nv_bfloat16>::value)
-        if (features_of(P) != 0) return launch_w<Q, S, F_WALL | F_FORCE>(w, P, T, s);
-    return launch_w<Q, S, 0>(w, P, T, s);
+cudaError_t launch(bool tma, int w, const StepParams& P, const TensorMaps& T, cudaStream_t s) {
+    return w == kStepWSmall ? launch_w<Q, S, kStepWSmall>(tma, P, T, s) : launch_w<Q, S, kStepW>(tma, P, T, s);
 }
 
 } // namespace pop

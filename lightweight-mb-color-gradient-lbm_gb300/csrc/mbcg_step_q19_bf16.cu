@@ -5,8 +5,7 @@
 namespace mbcg {
 
 cudaError_t launch_step_q19_bf16(bool tma, int w, const StepParams& P, const TensorMaps& T, cudaStream_t s) {
-    if (tma && uses_pop(MBCG_BF16, features_of(P)))
-        return pop::launch<19, __nv_bfloat16>(w, P, T, s);
+    if (uses_pop(MBCG_BF16, features_of(P))) return pop::launch<19, __nv_bfloat16>(tma, w, P, T, s);
     return launch_qs<19, __nv_bfloat16>(tma, w, P, T, s);
 }
 

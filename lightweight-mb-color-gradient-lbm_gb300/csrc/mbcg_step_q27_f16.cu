@@ -6,8 +6,7 @@
 namespace mbcg {
 
 cudaError_t launch_step_q27_f16(bool tma, int w, const StepParams& P, const TensorMaps& T, cudaStream_t s) {
-    if (tma && uses_pop(MBCG_FP16, features_of(P)))
-        return pop::launch<27, __half>(w, P, T, s);
+    if (uses_pop(MBCG_FP16, features_of(P))) return pop::launch<27, __half>(tma, w, P, T, s);
     return launch_qs<27, __half>(tma, w, P, T, s);
 }
 
