@@ -340,7 +340,7 @@ def serve_batched(reqs, policy=mbcg.POLICY_FIFO) -> dict:
     work = sum(r["p"].active_nodes() * r["steps"] for r in reqs)
     return {"cases_per_s": len(reqs) / span, "p50_s": _pct(ttc, 50), "p99_s": _pct(ttc, 99), "makespan_s": span,
             "mlups": work / span / 1e6, "failed": sum(i.state != mbcg.REQ_DONE for i in infos),
-            "compositions": st["compositions"], "replays": st["replays"], "zchunk_last": st["zchunk"],
+            "compositions": st["compositions"], "replays": st["replays"], "zchunk_last": st["zchunk"], "zsplit_last": st["zsplit"],
             "cost_model_ns_per_plane": st["plane_ns"], "tile_overhead_planes": st["tile_overhead_planes"],
             "arena_peak_gb": st["arena_peak_bytes"] / 1e9,
             "mass": [(i.diag.mass_r, i.diag.mass_b) for i in infos],

@@ -360,9 +360,9 @@ typedef struct mbcg_server_stats {
     int64_t compositions;   /* distinct batch compositions (graph captures)                    */
     int64_t replays;        /* graph replays                                                   */
     int64_t arena_bytes, arena_peak_bytes;
-    int32_t zchunk;         /* tile z depth the planner chose for the current composition (8
-                               stands for every thinner depth too)                             */
-    int32_t reserved;
+    int32_t zchunk;         /* tile z depth the planner chose for the current composition, */
+    int32_t zsplit;         /* and the parts it cuts such tiles into where they would leave SMs
+                               idle (else 1): a tile is at most ceil(zchunk / zsplit) planes   */
     double plane_ns[10];    /* cost model: ns per tile plane of each batch-kernel body, in the
                                order Q19 FP32/FP16/BF16, Q27 FP32/FP16/BF16 (every feature),
                                Q19 FP32/FP16, Q27 FP32/FP16 (fully periodic, unforced); the

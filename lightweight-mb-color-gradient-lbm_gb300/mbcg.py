@@ -288,7 +288,7 @@ class ServerStats(ctypes.Structure):
     _fields_ = [("submitted", ctypes.c_int64), ("completed", ctypes.c_int64), ("failed", ctypes.c_int64),
                 ("live", ctypes.c_int64), ("queued", ctypes.c_int64), ("node_updates", ctypes.c_int64),
                 ("compositions", ctypes.c_int64), ("replays", ctypes.c_int64), ("arena_bytes", ctypes.c_int64),
-                ("arena_peak_bytes", ctypes.c_int64), ("zchunk", ctypes.c_int32), ("reserved", ctypes.c_int32),
+                ("arena_peak_bytes", ctypes.c_int64), ("zchunk", ctypes.c_int32), ("zsplit", ctypes.c_int32),
                 ("plane_ns", ctypes.c_double * 10), ("tile_overhead_planes", ctypes.c_double),
                 ("busy_s", ctypes.c_double)]
 
@@ -296,7 +296,7 @@ class ServerStats(ctypes.Structure):
               "q19_f32_periodic", "q19_f16_periodic", "q27_f32_periodic", "q27_f16_periodic")
 
     def as_dict(self) -> dict:
-        d = {n: getattr(self, n) for n, _ in self._fields_ if n not in ("plane_ns", "reserved")}
+        d = {n: getattr(self, n) for n, _ in self._fields_ if n != "plane_ns"}
         d["plane_ns"] = dict(zip(self.BODIES, list(self.plane_ns)))
         return d
 
