@@ -34,6 +34,7 @@
 
 #include "mbcg_batch.h"
 #include "mbcg_internal.h"
+#include "mbcg_plan.h"
 
 using namespace mbcg;
 
@@ -425,112 +426,45 @@ cudaError_t admit_pending(mbcg_server* s) {
 }
 
 // ---------------------------------------------------------------- composition and graph
-struct TileItem {
-    BatchTile t;
-    int kind;
-    double cost; // predicted ns
-};
-
-// Tiles of every live lattice for a target depth z: each lattice's z axis is cut into equal
-// chunks of at most z planes; a tile costs (planes + 2 warm-up planes + overhead) x the
-// calibrated time of one plane of its kernel body.
-void make_tiles(const mbcg_server* s, int z, std::vector<TileItem>& items, std::vector<int>& zc) {
-    items.clear();
-    zc.assign(s->cfg.max_live, 0);
-    for (int slot = 0; slot < s->cfg.max_live; ++slot) {
-        const int64_t id = s->slot_req[slot];
-        if (!id) continue;
-        const Request& r = *s->reqs.at(id);
-        const int gx = (r.p.nx - 2 + kStepTileX - 1) / kStepTileX;
-        const int kind = r.kind, rows = batch_rows(kind) - 2, bcz = batch_bcz(kind, r.p.bc[2]);
-        const int gy = (r.p.ny - 2 + rows - 1) / rows;
-        const int nzf = r.p.nz - 2 - 2 * z_cap(r.p.nz, bcz);
-        const int zmax = std::min(z, max_zchunk(r.plane, r.es));
-        const int nch = std::max(1, (nzf + zmax - 1) / zmax);
-        const int depth = (nzf + nch - 1) / nch;
-        const int gz = z_tiles(r.p.nz, bcz, depth);
-        zc[slot] = depth;
-        for (int bz = 0; bz < gz; ++bz) {
-            int zd0, zd1;
-            z_range(r.p.nz, bcz, depth, bz, zd0, zd1);
-            const double planes = zd1 - zd0 + 2 + s->tile_ovh;
-            for (int by = 0; by < gy; ++by)
-                for (int bx = 0; bx < gx; ++bx)
-                    items.push_back({BatchTile{static_cast<uint16_t>(slot), static_cast<uint16_t>(bx),
-                                               static_cast<uint16_t>(by), static_cast<uint16_t>(bz)},
-                                     kind, planes * s->plane_ns[kind]});
-        }
-    }
-    // longest tiles first: the atomic queues then run a greedy longest-processing-time schedule
-    std::stable_sort(items.begin(), items.end(), [](const TileItem& a, const TileItem& b) {
-        if (a.cost != b.cost) return a.cost > b.cost;
-        return a.kind < b.kind;
-    });
-}
-
-// Predicted duration of one launch: the greedy schedule of the sorted tiles on nsm CTAs.
-double predict_ns(const std::vector<TileItem>& items, int nsm) {
-    std::vector<double> load(std::max(1, nsm), 0.0);
-    std::make_heap(load.begin(), load.end(), std::greater<double>());
-    for (const TileItem& it : items) {
-        std::pop_heap(load.begin(), load.end(), std::greater<double>());
-        load.back() += it.cost;
-        std::push_heap(load.begin(), load.end(), std::greater<double>());
-    }
-    return *std::max_element(load.begin(), load.end());
-}
-
-// The planner's cuts: tiles z planes deep (8 or more), or such tiles in `split` parts, which compositions too
-// small to fill the SMs take (8 requests of 16 to 48 nodes across: 4.6 ms, 5.5 without the parts).
-struct Cut {
-    int z, split;
-    int depth() const { return (z + split - 1) / split; }
-};
-constexpr Cut kCuts[] = {{8, 8}, {8, 4}, {8, 3}, {8, 2}, {12, 2}, {8, 1}, {12, 1}, {16, 1}, {24, 1},
-                         {32, 1}, {48, 1}, {64, 1}, {96, 1}, {128, 1}, {192, 1}, {256, 1}, {512, 1}};
-
-cudaError_t rebuild(mbcg_server* s) {
-    // planner: the cut with the shortest predicted launch (fixed if configured)
-    std::vector<TileItem> items, best_items;
-    std::vector<int> zc, best_zc;
-    Cut best_cut{s->cfg.zchunk, 1};
-    if (best_cut.z > 0) {
-        make_tiles(s, best_cut.z, best_items, best_zc);
-    } else {
-        double best = 1e300;
-        for (const Cut& cut : kCuts) {
-            make_tiles(s, cut.depth(), items, zc);
-            const double t = predict_ns(items, s->nsm);
-            if (t < best * 0.999) {
-                best = t;
-                best_cut = cut;
-                best_items.swap(items);
-                best_zc.swap(zc);
-            }
-        }
-    }
-    s->last_z = best_cut.z;
-    s->last_split = best_cut.split;
-    // lattice table with this composition's depths
+// the live lattices as the planner takes them
+std::vector<PlanLattice> plan_lattices(const mbcg_server* s) {
+    std::vector<PlanLattice> out;
     for (int slot = 0; slot < s->cfg.max_live; ++slot) {
         if (!s->slot_req[slot]) continue;
-        Request& r = *s->reqs.at(s->slot_req[slot]);
-        r.zchunk = best_zc[slot];
-        s->h_cases[slot].P[0].zchunk = r.zchunk;
-        s->h_cases[slot].P[1].zchunk = r.zchunk;
+        const Request& r = *s->reqs.at(s->slot_req[slot]);
+        out.push_back({slot, r.kind, r.p.nx, r.p.ny, r.p.nz, r.p.bc[2], max_zchunk(r.plane, r.es)});
+    }
+    return out;
+}
+
+cudaError_t rebuild(mbcg_server* s) {
+    // the cut with the shortest predicted launch (fixed if configured)
+    const std::vector<PlanLattice> lattices = plan_lattices(s);
+    std::vector<TileItem> items;
+    Cut cut{s->cfg.zchunk, 1};
+    if (cut.z > 0) plan_tiles(lattices, cut.z, s->plane_ns, s->tile_ovh, items);
+    else cut = plan_cut(lattices, s->plane_ns, s->tile_ovh, s->nsm, items);
+    s->last_z = cut.z;
+    s->last_split = cut.split;
+    // lattice table with this composition's depths
+    for (const PlanLattice& l : lattices) {
+        Request& r = *s->reqs.at(s->slot_req[l.slot]);
+        r.zchunk = plan_depth(l, cut.depth());
+        s->h_cases[l.slot].P[0].zchunk = r.zchunk;
+        s->h_cases[l.slot].P[1].zchunk = r.zchunk;
     }
     cudaError_t e = upload(s, s->case_stage, &s->case_ring, s->d_cases, s->h_cases,
                            sizeof(BatchCase) * s->cfg.max_live);
     if (e == cudaSuccess) e = upload_params(s);
     if (e != cudaSuccess) return e;
     // one queue per kind, in one array
-    std::stable_sort(best_items.begin(), best_items.end(),
+    std::stable_sort(items.begin(), items.end(),
                      [](const TileItem& a, const TileItem& b) { return a.kind < b.kind; });
-    std::vector<BatchTile> tiles(best_items.size());
+    std::vector<BatchTile> tiles(items.size());
     int kind_tiles[BK_COUNT] = {}, kind_first[BK_COUNT] = {};
-    for (size_t i = 0; i < best_items.size(); ++i) {
-        tiles[i] = best_items[i].t;
-        kind_tiles[best_items[i].kind] += 1;
+    for (size_t i = 0; i < items.size(); ++i) {
+        tiles[i] = items[i].t;
+        kind_tiles[items[i].kind] += 1;
     }
     for (int kind = 1; kind < BK_COUNT; ++kind) kind_first[kind] = kind_first[kind - 1] + kind_tiles[kind - 1];
     const int ntiles = static_cast<int>(tiles.size());
