@@ -31,10 +31,12 @@ constexpr Cut kCuts[] = {{8, 8}, {8, 4}, {8, 3}, {8, 2}, {12, 2}, {8, 1}, {12, 1
                          {32, 1}, {48, 1}, {64, 1}, {96, 1}, {128, 1}, {192, 1}, {256, 1}, {512, 1}};
 
 inline int plan_bcz(const PlanLattice& l) { return batch_bcz(l.kind, l.bcz); }
-// Depth of a lattice's tiles for a target z: equal chunks of at most z planes.
+// Depth of a lattice's tiles for a target z: equal chunks of at most z planes, or more where the chunks and two
+// end tiles would outgrow a tile's 16-bit index.
 inline int plan_depth(const PlanLattice& l, int z) {
     const int nzf = l.nz - 2 - 2 * z_cap(l.nz, plan_bcz(l));
-    const int zmax = std::min(z, l.max_depth);
+    constexpr int kMaxChunks = 0xffff - 2;
+    const int zmax = std::max(std::min(z, l.max_depth), (nzf + kMaxChunks - 1) / kMaxChunks);
     const int nch = std::max(1, (nzf + zmax - 1) / zmax);
     return (nzf + nch - 1) / nch;
 }

@@ -1,15 +1,39 @@
 // The server's planner (csrc/mbcg_plan.h) against building every cut: the same choice, and how many tiles it
-// built for it.  argv: seed, compositions.  Prints one line a composition: chosen index, exhaustive index, their
+// built for it.  argv: seed, compositions; or "cover": every fluid plane of long lattices in exactly one tile, at
+// any depth.  Prints one line a composition: chosen index, exhaustive index, their
 // predicted times, tiles built, tiles of the chosen cut, tiles of all cuts.
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <random>
 
 #include "mbcg_plan.h"
 
 using namespace mbcg;
 
+int cover() {
+    double ns[BK_COUNT];
+    for (double& v : ns) v = 1.0;
+    for (int nz : {66000, 70003, 524282})
+        for (int bcz : {MBCG_BC_PERIODIC, MBCG_BC_WALL})
+            for (int z : {1, 5, 8, 12}) {
+                const PlanLattice l{0, BK_Q27_F32, 6, 6, nz, bcz, 1 << 20};
+                std::vector<TileItem> items;
+                plan_tiles({l}, z, ns, 3.0, items);
+                std::vector<char> seen(nz, 0);
+                for (const TileItem& it : items) {
+                    int zd0, zd1;
+                    z_range(nz, bcz, plan_depth(l, z), it.t.bz, zd0, zd1);
+                    for (int k = zd0; k < zd1; ++k) seen[k] += 1;
+                }
+                for (int k = 1; k < nz - 1; ++k)
+                    if (seen[k] != 1) return std::printf("nz %d bcz %d z %d: plane %d in %d tiles\n", nz, bcz, z, k, seen[k]), 1;
+            }
+    return 0;
+}
+
 int main(int argc, char** argv) {
+    if (argc > 1 && !std::strcmp(argv[1], "cover")) return cover();
     std::mt19937 rng(argc > 1 ? std::atoi(argv[1]) : 1);
     const int count = argc > 2 ? std::atoi(argv[2]) : 100;
     constexpr int n = sizeof(kCuts) / sizeof(kCuts[0]);

@@ -32,3 +32,13 @@ def test_reported_cut():
     # 63 tiles side by side, 192 planes: deep tiles fill the SMs, and a part more only adds its two planes
     depth, st, _ = planned(mbcg.bubble_params(192, q=27), calibrate=1)
     assert depth in DEPTHS and st["zsplit"] == 1 and st["zchunk"] == depth >= 8, st
+
+
+def test_long_lattice_at_depth_one():
+    """More planes than a tile's 16-bit index counts."""
+    p = mbcg.bubble_params(8, q=19, radius=3.0)
+    p.nx, p.ny, p.nz = 4, 4, 66005
+    p.bubble_center[2] = 65990.0
+    got = [planned(p, steps=3, calibrate=0, zchunk=z)[2] for z in (1, 64)]
+    assert np.ptp(got[1][0]) > 0.1
+    np.testing.assert_array_equal(got[0], got[1])

@@ -11,10 +11,15 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 
 @pytest.fixture(scope="module")
-def plans(tmp_path_factory):
+def exe(tmp_path_factory):
     exe = str(tmp_path_factory.mktemp("plan") / "plan_check")
     subprocess.run([NVCC, "-O2", "-std=c++17", "-x", "cu", f"-I{CSRC}", f"-I{ROOT}/include",
                     os.path.join(ROOT, "tests", "cpp", "plan_check.cpp"), "-o", exe], check=True)
+    return exe
+
+
+@pytest.fixture(scope="module")
+def plans(exe):
     r = subprocess.run([exe, "7", "150"], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout[-500:]
     return [[float(v) for v in line.split()] for line in r.stdout.split("\n") if line]
@@ -33,3 +38,9 @@ def test_tiles_built(plans):
     assert built <= 6 * ntiles and built <= 0.05 * all_
     # and never more than every cut's and the chosen one's again
     assert all(p[4] <= p[6] + p[5] for p in plans)
+
+
+def test_long_lattices_are_covered(exe):
+    """A tile's index along z has 16 bits: lattices of up to 524,280 fluid planes are accepted."""
+    r = subprocess.run([exe, "cover"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
