@@ -1058,25 +1058,29 @@ int mbcg_server_drain(mbcg_server* s, double timeout_s) {
     return MBCG_OK;
 }
 
-// The 11 dense fields of a result into host memory: one kernel converts them all into a device staging
-// area, and one copy takes them where the caller's (pageable) fields lie end to end, one copy a field
-// elsewhere.  A field at a time through an area allocated and freed for the call took 200 us for a result of
-// 1 to 4 MB, and the free waited for the other requests' steps; 65 to 90 us now.  Results above kFetchKeep go
-// two fields at a time through an area of their own.
+// The 11 dense fields of a result into host memory, two at a time through an area of the call's own: results
+// above kFetchKeep, and any where the device has no memory left for more.
+static cudaError_t fetch_by_field(mbcg_server* s, const mbcg_params& p, const StepParams& P, float* const host[NF]) {
+    const size_t n = static_cast<size_t>(p.nx) * p.ny * p.nz, bytes = n * sizeof(float);
+    float* area = nullptr;
+    cudaError_t e = cudaMalloc(&area, 2 * bytes);
+    for (int i = 0; i < NF && e == cudaSuccess; ++i) {
+        float* buf = area + (i & 1) * n;
+        e = launch_to_dense(p.precision, P, i, buf, s->st_io);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(host[i], buf, bytes, cudaMemcpyDeviceToHost, s->st_io);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->st_io);
+    if (area) cudaFree(area);
+    return e;
+}
+
+// All of them at once: one kernel converts them into a device staging area, and one copy takes them where the
+// caller's (pageable) fields lie end to end, one copy a field elsewhere.  A field at a time through an area
+// allocated and freed for the call took 200 us for a result of 1 to 4 MB, and the free waited for the other
+// requests' steps; 65 to 90 us now.
 static cudaError_t fetch_fields(mbcg_server* s, const mbcg_params& p, const StepParams& P, float* const host[NF]) {
     const size_t n = static_cast<size_t>(p.nx) * p.ny * p.nz, bytes = n * sizeof(float);
-    if (NF * bytes > kFetchKeep) {
-        float* area = nullptr;
-        cudaError_t e = cudaMalloc(&area, 2 * bytes);
-        for (int i = 0; i < NF && e == cudaSuccess; ++i) {
-            float* buf = area + (i & 1) * n;
-            e = launch_to_dense(p.precision, P, i, buf, s->st_io);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(host[i], buf, bytes, cudaMemcpyDeviceToHost, s->st_io);
-        }
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s->st_io);
-        if (area) cudaFree(area);
-        return e;
-    }
+    if (NF * bytes > kFetchKeep) return fetch_by_field(s, p, P, host);
     bool joined = true;
     for (int i = 0; i < NF && joined; ++i) {
         cudaPointerAttributes a{};
@@ -1091,7 +1095,11 @@ static cudaError_t fetch_fields(mbcg_server* s, const mbcg_params& p, const Step
         s->fetch_stage = nullptr;
         s->fetch_cap = 0;
         e = cudaMalloc(&s->fetch_stage, NF * bytes);
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess) {
+            s->fetch_stage = nullptr;
+            cudaGetLastError();
+            return fetch_by_field(s, p, P, host);
+        }
         s->fetch_cap = NF * bytes;
     }
     float* dev[NF];
