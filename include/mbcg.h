@@ -308,22 +308,24 @@ int mbcg_diagnostics_static(const mbcg_params *p, const mbcg_moments *a, mbcg_di
  * device arena and a worker thread.  Requests (a case and a step count) queue on submit and are
  * admitted while a slot and arena space are free, in the order the policy gives (with backfill
  * a later request that fits may pass one that does not yet).  All resident lattices advance
- * together: one persistent batch-kernel launch per time step runs every live lattice's tiles
- * from one flat queue, and each batch composition (the set of live lattices) is captured once
- * as a CUDA graph of chunk_steps launches that is replayed until the composition changes.  A
- * lattice computes the same arithmetic alone or in any mix (its tiles never read another
- * lattice's data), so its result is identical, bit for bit, whatever else runs beside it. */
+ * together: for each kind of step body (lattice, storage, features) one persistent batch-kernel
+ * launch per time step runs the tiles of every live lattice of that kind from one queue, and each
+ * batch composition (the set of live lattices) is captured once as a CUDA graph, with a branch of
+ * chunk_steps launches for each kind, that is replayed until the composition changes.  A lattice
+ * computes the same arithmetic alone or in any mix (its tiles never read another lattice's data), so
+ * its result is identical, bit for bit, whatever else runs beside it. */
 typedef struct mbcg_server mbcg_server;
 
 typedef struct mbcg_server_config {
     int64_t arena_bytes;    /* device memory for resident states (0: 70% of the free memory)  */
     int32_t max_live;       /* lattices resident at once (0: 64; at most 64)                   */
-    int32_t chunk_steps;    /* launches per graph replay, the admission granularity (0: 16)    */
+    int32_t chunk_steps;    /* steps per graph replay, the admission granularity (0: 16)    */
     int32_t keep_results;   /* 1: finished states stay resident until fetched or released      */
     int32_t backfill;       /* 1: admit later requests that fit while an earlier one waits     */
     int32_t zchunk;         /* z depth of the tiles (0: the planner picks one per composition:
                                the depth whose greedy schedule of all live tiles on the SMs,
-                               under the cost model, gives the shortest launch)                */
+                               under the cost model, is the shortest).  Lattices with more than
+                               65,533 planes take the depth that a tile's 16-bit index needs   */
     int32_t calibrate;      /* 1: measure the cost model (time of one tile plane per kernel body
                                and lattice, fixed cost per tile) at start-up; 0: defaults      */
     int32_t policy;         /* MBCG_POLICY_*: admission order (default FIFO: highest throughput;

@@ -274,7 +274,9 @@ struct DiagParams {
 // FP64 sums over the fluid nodes.  GB300 has two FP64 lanes per SM and clock: one FP64 add per quantity
 // and node took 561 us for 192x192x512 nodes (830 MB, 123 us of HBM time).  So each thread sums 16 nodes
 // at a time in FP32 pairs, products with their rounding errors, and adds the pairs in FP64: 10 FP64
-// additions per 16 nodes instead of 10 a node, and fewer FP64 roundings.  A node with values so large that
+// additions per 16 nodes instead of 10 a node, and fewer FP64 roundings (against the exact sums of drops, RTI and
+// jets of 14 thousand to 3 million nodes: masses and momenta within 2e-16 of the sum of magnitudes, 4e-15 with one
+// FP64 add a node).  A node with values so large that
 // the pair could overflow (or not finite) is added in FP64 directly.
 template <typename S, bool kBubble>
 __global__ void __launch_bounds__(256) diag_kernel(const StepParams P, const DiagParams D, double* partials) {

@@ -71,7 +71,9 @@ __device__ __forceinline__ int nb_coord(const StepParams& P, int a, int c, int n
 // through shared memory, with the tile's edge columns added by its first threads.  Volumes, interface
 // nodes, centroid and penetration are whole numbers, counted as such; the area's terms are formed in FP32
 // pairs and summed in FP64 (GB300 has two FP64 lanes per SM and clock: with FP64 roots at the nodes where
-// phi varies, 223 us).  192x192x512 FP32: 3,100 us before.
+// phi varies, 223 us).  192x192x512 FP32: 3,100 us before.  The area is within 6e-16 of the exact sum of the terms
+// of the FP32 phi (drops 24^3 to 150^3, RTI, jet, 16-bit forms; 3e-15 with FP64 terms), and as far as before, 2e-10
+// to 7e-8, from that of phi in 64 bits.
 constexpr int kTileX = 32, kTileY = 8;
 
 template <typename S>

@@ -1541,7 +1541,7 @@ __device__ __forceinline__ bool step_tile(const StepParams& P, const CUtensorMap
         if (w == 0) {
             if constexpr (kTMA) {
                 // Nothing more to stage: the next step's CTAs may take the SMs that fall idle (from the start
-                // of the kernel they took them in another order: D3Q19 RTI 61^2x243, 8 steps, 493 against 510 us).
+                // of the kernel they took them in another order: D3Q19 RTI 61^2x243, 8 steps, 494 against 512 us).
                 if (k + kNSTAGE <= zd1 + 1) issue(k + kNSTAGE, sl);
                 else launch_dependents();
             }

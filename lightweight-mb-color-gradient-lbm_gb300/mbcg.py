@@ -612,7 +612,7 @@ def server_config(**kw) -> ServerConfig:
 
 class Server:
     """Continuous-batching server (mbcg_server*): many cases resident on one GPU, advanced
-    together by the persistent batch kernel."""
+    together by persistent batch kernels, one for each kind of step body."""
 
     def __init__(self, config: Optional[ServerConfig] = None, lib: Optional[Library] = None, **kw):
         self.lib = lib or Library.get()
